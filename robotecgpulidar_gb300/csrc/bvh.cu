@@ -578,20 +578,36 @@ __global__ void __launch_bounds__(256) kCollapseSmall(CollapseInputs gin, WideNo
 // refit kernel.
 namespace {
 
+void freeSmallScratch(TlasBuild& t)
+{
+	void* ptrs[] = {t.lo, t.hi, t.sahScratch, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds};
+	for (void* p : ptrs) {
+		cudaFree(p);
+	}
+	t.lo = t.hi = nullptr;
+	t.sahScratch = nullptr;
+	t.bin = nullptr;
+	t.rangeFirst = t.rangeLast = nullptr;
+	t.sortedIds = nullptr;
+	t.smallCapacity = 0;
+}
+
 void allocTlas(TlasBuild& t, int n)
 {
-	if (n <= t.capacity) {
-		return;
+	if (n > t.capacity) {
+		freeTlas(t);
+		t.capacity = n;
+		RGL_CUDA_OK(cudaMalloc(&t.nodes, sizeof(WideNode) * (size_t) n));
+		RGL_CUDA_OK(cudaMalloc(&t.leaves, sizeof(TriRecord) * (size_t) n));
+		RGL_CUDA_OK(cudaMalloc(&t.boxes, sizeof(Box) * (size_t) n));
+		t.levelCapacity = n + 2;
+		RGL_CUDA_OK(cudaMalloc(&t.levelStarts, sizeof(int32_t) * (size_t) t.levelCapacity));
+		RGL_CUDA_OK(cudaMalloc(&t.nLevels, sizeof(int32_t)));
 	}
-	freeTlas(t);
-	t.capacity = n;
-	RGL_CUDA_OK(cudaMalloc(&t.nodes, sizeof(WideNode) * (size_t) n));
-	RGL_CUDA_OK(cudaMalloc(&t.leaves, sizeof(TriRecord) * (size_t) n));
-	RGL_CUDA_OK(cudaMalloc(&t.boxes, sizeof(Box) * (size_t) n));
-	t.levelCapacity = n + 2;
-	RGL_CUDA_OK(cudaMalloc(&t.levelStarts, sizeof(int32_t) * (size_t) t.levelCapacity));
-	RGL_CUDA_OK(cudaMalloc(&t.nLevels, sizeof(int32_t)));
-	if (n <= kSahSmallMax) {
+	// The one-block rebuild's scratch has a size of its own: a scene that shrinks from above
+	// kSahSmallMax instances keeps its node storage but has no scratch yet.
+	if (n <= kSahSmallMax && n > t.smallCapacity) {
+		freeSmallScratch(t);
 		RGL_CUDA_OK(cudaMalloc(&t.lo, sizeof(float4) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.hi, sizeof(float4) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.sahScratch, sahSmallScratchBytes(n)));
@@ -599,8 +615,10 @@ void allocTlas(TlasBuild& t, int n)
 		RGL_CUDA_OK(cudaMalloc(&t.rangeFirst, sizeof(int32_t) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.rangeLast, sizeof(int32_t) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.sortedIds, sizeof(uint32_t) * (size_t) n));
-		// Shared memory of the one-block collapse for up to n instances (set outside any capture).
-		RGL_CUDA_OK(cudaFuncSetAttribute(kCollapseSmall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smallCollapseLayout(n).bytes));
+		// Shared memory of the one-block collapse, set outside any capture and for the largest scene: the limit
+		// is the kernel's, so a small scene must not lower it under a large one.
+		RGL_CUDA_OK(cudaFuncSetAttribute(kCollapseSmall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smallCollapseLayout(kSahSmallMax).bytes));
+		t.smallCapacity = n;
 	}
 }
 
@@ -686,8 +704,8 @@ void refitTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 
 void freeTlas(TlasBuild& t)
 {
-	void* ptrs[] = {t.nodes, t.leaves, t.boxes, t.levelStarts, t.nLevels, t.lo, t.hi, t.sahScratch, t.bin, t.rangeFirst,
-	                t.rangeLast, t.sortedIds};
+	freeSmallScratch(t);
+	void* ptrs[] = {t.nodes, t.leaves, t.boxes, t.levelStarts, t.nLevels};
 	for (void* p : ptrs) {
 		cudaFree(p);
 	}

@@ -63,7 +63,8 @@ struct TlasBuild
 	int32_t capacity = 0;
 	int32_t nInstances = 0;
 	uint32_t nodeCount = 0;          // node count of the last host-synchronous build (statistics)
-	// Scratch of the graph-capturable rebuild (instances up to kSahSmallMax), sized with `capacity`.
+	// Scratch of the graph-capturable rebuild (up to kSahSmallMax instances), for smallCapacity of them.
+	int32_t smallCapacity = 0;
 	float4* lo = nullptr;
 	float4* hi = nullptr;
 	void* sahScratch = nullptr;
