@@ -3,6 +3,7 @@
 //
 // Replaces the OptiX acceleration-structure builds of reference src/scene/GASBuilder.hpp:31-100 and
 // src/scene/Scene.cpp:131-190 (where any pose change triggers a full IAS rebuild plus a stream sync).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -11,6 +12,7 @@
 #include <vector>
 
 #include "bvh_core.hpp"
+#include "collapse.cuh"
 #include "kernels.hpp"
 #include "sah_build.hpp"
 
@@ -163,13 +165,67 @@ __global__ void kBottomUp(int n, const uint32_t* __restrict__ ids, const float4*
 	}
 }
 
-__global__ void kCollapse(const int2* __restrict__ qIn, const uint32_t* __restrict__ qInCount, CollapseInputs in,
-                          CollapseOutputs out)
+// Counters of one collapse: three depth counters used in turn (see kCollapse), then its results.
+struct CollapseState
 {
-	uint32_t cnt = *qInCount;
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-		int2 it = qIn[i];
-		collapseItem(it.x, (uint32_t) it.y, in, out);
+	collapsedev::DepthCounter depth[3];
+	uint32_t nodes, leaves;
+};
+
+// The whole collapse of a binary tree over n primitives in one cooperative launch, depth by depth with
+// a grid barrier between (one launch per depth, sixteen between host checks of the queue, before). A
+// depth adds to its own counter; the counter after next is cleared meanwhile, when nobody reads it.
+// `st` is zero at the start. levelStarts (optional) receives the first node of every depth and the node
+// count, up to levelCap entries. 131,072 triangles: 516 us for sixteen launches before, see
+// collapse.cuh for what a depth cost and why.
+constexpr int kCollapseThreads = 128;
+__global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* st,
+                                                              int32_t* levelStarts, int32_t* nLevels, int levelCap)
+{
+	cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+	const uint32_t warp = (blockIdx.x * kCollapseThreads + threadIdx.x) >> 5, warps = gridDim.x * (kCollapseThreads / 32);
+	const uint32_t group = (threadIdx.x & 31u) >> 3;
+	const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+	uint32_t start = 0, end = 1, leaves = 0;
+	int level = 0;
+	for (; start < end; ++level) {
+		collapsedev::DepthCounter* ctr = &st->depth[level % 3];
+		if (first) {
+			st->depth[(level + 1) % 3] = 0;
+			if (levelStarts != nullptr && level < levelCap) {
+				levelStarts[level] = (int32_t) start;
+			}
+		}
+		for (uint32_t at = start + 4 * warp; at < end; at += 4 * warps) {
+			const uint32_t idx = at + group;
+			const bool valid = idx < end;
+			collapsedev::CollapseTask task{0, 0};
+			if (valid) {
+				task = level == 0 ? collapsedev::rootTask(in.bin, n) : out.queue[idx];
+			}
+			if (in.vertices != nullptr) {
+				collapsedev::collapseGroups<true>(valid, idx, task, in, out, ctr, end, leaves, (uint32_t) n);
+			} else {
+				collapsedev::collapseGroups<false>(valid, idx, task, in, out, ctr, end, leaves, (uint32_t) n);
+			}
+		}
+		grid.sync();
+		// Stable until the depth after next clears it, so every block takes the same decision.
+		const collapsedev::DepthCounter got = *(volatile collapsedev::DepthCounter*) ctr;
+		start = end;
+		end += (uint32_t) got;
+		leaves += (uint32_t) (got >> 32);
+		if (end > (uint32_t) n || leaves > (uint32_t) n) {
+			break; // not a proper tree; the host sees the counts
+		}
+	}
+	if (first) {
+		st->nodes = end;
+		st->leaves = leaves;
+		if (levelStarts != nullptr && level < levelCap) {
+			levelStarts[level] = (int32_t) end;
+			*nLevels = level;
+		}
 	}
 }
 
@@ -193,16 +249,39 @@ struct WideBuildResult
 	Box bounds;
 };
 
+// Where a collapse records the first node of every depth (device): levelCap entries and the depths.
+struct LevelRecord
+{
+	int32_t* starts = nullptr;
+	int32_t* count = nullptr;
+	int capacity = 0;
+};
+
+void launchCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* state, LevelRecord levels, cudaStream_t s)
+{
+	static const int most = [] { // blocks that fit the device at once, as the grid barrier needs
+		int dev = 0, sms = 0, perSm = 0;
+		RGL_CUDA_OK(cudaGetDevice(&dev));
+		RGL_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+		RGL_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kCollapse, kCollapseThreads, 0));
+		return sms * std::min(perSm, 4);
+	}();
+	// The widest depths hold about n / 6 nodes, 16 at a time per block; a small tree takes fewer blocks,
+	// whose barrier is cheaper.
+	int grid = std::max(1, std::min(most, n / 256));
+	void* args[] = {&in, &out, &n, &state, &levels.starts, &levels.count, &levels.capacity};
+	RGL_CUDA_OK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&kCollapse), dim3(grid), dim3(kCollapseThreads), args, 0, s));
+	countLaunch();
+}
+
 // Wide BVH over n primitive boxes lo/hi (device) whose centroid bounds are in cb (6 ordered uints),
 // all written on stream s: the binary topology (binned SAH when `sah`, else Morton codes, onesweep
-// sort, LBVH and bottom-up bounds), then the collapse into 8-wide nodes, one launch per depth. Leaf
-// records are triangles (dV/dI given) or primitive indices (dV null). With levelStarts, it receives the
-// first node index of every depth and the node count (the collapse allocates the nodes of depth L + 1
-// while it writes depth L, so the counter before each launch starts the next depth). Frees lo, hi, cb
-// and its temporaries and synchronises s (a one-off build).
+// sort, LBVH and bottom-up bounds), then the collapse into 8-wide nodes (one launch). Leaf records are
+// triangles (dV/dI given) or primitive indices (dV null). `levels` optionally receives the first node
+// index of every depth and the node count. Frees lo, hi, cb and its temporaries and synchronises s (a
+// one-off build).
 WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const float* dV, const int32_t* dI, int leafMax,
-                          WideNode* outNodes, TriRecord* outLeaves, Box* outBoxes, cudaStream_t s, bool sah,
-                          std::vector<int32_t>* levelStarts = nullptr)
+                          WideNode* outNodes, TriRecord* outLeaves, Box* outBoxes, cudaStream_t s, bool sah, LevelRecord levels = {})
 {
 	uint32_t* codes = mallocAsync<uint32_t>(n, s);
 	uint32_t* ids = mallocAsync<uint32_t>(n, s);
@@ -213,13 +292,12 @@ WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const flo
 	int32_t* pi = mallocAsync<int32_t>(n, s);
 	int32_t* pl = mallocAsync<int32_t>(n, s);
 	uint32_t* visits = mallocAsync<uint32_t>(n, s);
-	int2* q0 = mallocAsync<int2>(n, s);
-	int2* q1 = mallocAsync<int2>(n, s);
-	// counters: [0] wide, [1] leaf records, [2] q0 count, [3] q1 count, [4] error
-	uint32_t* ctr = mallocAsync<uint32_t>(8, s);
+	collapsedev::CollapseTask* queue = mallocAsync<collapsedev::CollapseTask>(n, s);
+	CollapseState* state = mallocAsync<CollapseState>(1, s);
+	int32_t* err = mallocAsync<int32_t>(1, s);
 	RGL_CUDA_OK(cudaMemsetAsync(visits, 0, sizeof(uint32_t) * n, s));
-	RGL_CUDA_OK(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 8, s));
-	int32_t* err = reinterpret_cast<int32_t*>(ctr + 4);
+	RGL_CUDA_OK(cudaMemsetAsync(state, 0, sizeof(CollapseState), s));
+	RGL_CUDA_OK(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
 
 	if (sah) {
 		buildSahTopologyDevice(lo, hi, n, bin, rf, rl, ids, s);
@@ -234,56 +312,12 @@ WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const flo
 			countLaunch();
 		}
 	}
-	int2 root = make_int2(n == 1 ? ~0 : 0, 0);
-	uint32_t one[2] = {1u, 0u};
-	RGL_CUDA_OK(cudaMemcpyAsync(q0, &root, sizeof(int2), cudaMemcpyHostToDevice, s));
-	RGL_CUDA_OK(cudaMemcpyAsync(ctr, one, sizeof(uint32_t), cudaMemcpyHostToDevice, s));     // wide counter = 1 (root)
-	RGL_CUDA_OK(cudaMemcpyAsync(ctr + 2, one, sizeof(uint32_t), cudaMemcpyHostToDevice, s)); // q0 count = 1
 	CollapseInputs ci{bin, rf, rl, reinterpret_cast<const int32_t*>(ids), lo, hi, dV, dI, leafMax};
-	int2* qa = q0;
-	int2* qb = q1;
-	uint32_t* ca = ctr + 2;
-	uint32_t* cbn = ctr + 3;
-	// A wide level descends at least one binary level. The LBVH's binary depth is below 64 (30-bit keys
-	// with index tie-break); an SAH tree may be deeper, so the queue is checked after every 16 levels
-	// (empty launches exit immediately).
-	const int grid = 152 * 4;
-	uint32_t pending = 1;
-	uint32_t* snap = levelStarts ? mallocAsync<uint32_t>(16, s) : nullptr; // node counter before each launch of a round
-	uint32_t hostSnap[16];
-	if (levelStarts) {
-		levelStarts->assign(1, 0);
-	}
-	for (int round = 0; pending != 0; ++round) {
-		for (int level = 0; level < 16; ++level) {
-			if (snap) {
-				RGL_CUDA_OK(cudaMemcpyAsync(snap + level, ctr, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-			}
-			RGL_CUDA_OK(cudaMemsetAsync(cbn, 0, sizeof(uint32_t), s));
-			CollapseOutputs co{outNodes, outLeaves, ctr, ctr + 1, qb, cbn, outBoxes};
-			kCollapse<<<grid, 128, 0, s>>>(qa, ca, ci, co);
-			countLaunch();
-			int2* tq = qa;
-			qa = qb;
-			qb = tq;
-			uint32_t* tc = ca;
-			ca = cbn;
-			cbn = tc;
-		}
-		RGL_CUDA_OK(cudaMemcpyAsync(&pending, ca, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-		if (snap) {
-			RGL_CUDA_OK(cudaMemcpyAsync(hostSnap, snap, sizeof(hostSnap), cudaMemcpyDeviceToHost, s));
-		}
-		RGL_CUDA_OK(cudaStreamSynchronize(s));
-		if (levelStarts) {
-			levelStarts->insert(levelStarts->end(), hostSnap, hostSnap + 16);
-		}
-		if (round > (n >> 4) + 4) {
-			throw std::runtime_error("BVH build: wide collapse does not terminate");
-		}
-	}
-	uint32_t hostCtr[8];
-	RGL_CUDA_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(hostCtr), cudaMemcpyDeviceToHost, s));
+	launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, s);
+	CollapseState result{};
+	int32_t sortFailed = 0;
+	RGL_CUDA_OK(cudaMemcpyAsync(&result, state, sizeof(result), cudaMemcpyDeviceToHost, s));
+	RGL_CUDA_OK(cudaMemcpyAsync(&sortFailed, err, sizeof(sortFailed), cudaMemcpyDeviceToHost, s));
 	BinNode rootBox{};
 	float4 leafLo{}, leafHi{};
 	if (n > 1) {
@@ -292,23 +326,20 @@ WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const flo
 		RGL_CUDA_OK(cudaMemcpyAsync(&leafLo, lo, sizeof(float4), cudaMemcpyDeviceToHost, s));
 		RGL_CUDA_OK(cudaMemcpyAsync(&leafHi, hi, sizeof(float4), cudaMemcpyDeviceToHost, s));
 	}
-	void* temps[] = {lo, hi, cb, codes, ids, sortScratch, bin, rf, rl, pi, pl, visits, q0, q1, ctr};
+	void* temps[] = {lo, hi, cb, codes, ids, sortScratch, bin, rf, rl, pi, pl, visits, queue, state, err};
 	for (void* p : temps) {
 		RGL_CUDA_OK(cudaFreeAsync(p, s));
 	}
-	if (snap) {
-		RGL_CUDA_OK(cudaFreeAsync(snap, s));
-	}
 	RGL_CUDA_OK(cudaStreamSynchronize(s));
-	if (hostCtr[4] != 0) {
+	if (sortFailed != 0) {
 		throw std::runtime_error("BVH build: radix sort look-back did not complete");
 	}
-	if (hostCtr[1] != (uint32_t) n || hostCtr[0] > (uint32_t) n || hostCtr[ca - ctr] != 0) {
-		throw std::runtime_error("BVH build: collapse produced an inconsistent tree (leaf records " + std::to_string(hostCtr[1]) +
-		                         ", nodes " + std::to_string(hostCtr[0]) + ")");
+	if (result.leaves != (uint32_t) n || result.nodes > (uint32_t) n) {
+		throw std::runtime_error("BVH build: collapse produced an inconsistent tree (leaf records " + std::to_string(result.leaves) +
+		                         ", nodes " + std::to_string(result.nodes) + ")");
 	}
 	WideBuildResult r;
-	r.nodeCount = hostCtr[0];
+	r.nodeCount = result.nodes;
 	r.bounds = n > 1 ? Box{rootBox.lox, rootBox.loy, rootBox.loz, rootBox.hix, rootBox.hiy, rootBox.hiz}
 	                 : Box{leafLo.x, leafLo.y, leafLo.z, leafHi.x, leafHi.y, leafHi.z};
 	return r;
@@ -477,11 +508,11 @@ __global__ void kTlasBoxes(const InstanceRec* __restrict__ inst, int n, float4* 
 }
 
 // Shared-memory layout of the one-block collapse over n primitives (16-byte aligned parts): primitive
-// boxes lo[n] | hi[n] | binary nodes[n - 1] | two queues[n] | sorted ids[n] | ranges first[n - 1],
-// last[n - 1] | counters[4].
+// boxes lo[n] | hi[n] | binary nodes[n - 1] | queue[n] | sorted ids[n] | ranges first[n - 1],
+// last[n - 1] | depth counters[3].
 struct SmallCollapseLayout
 {
-	size_t lo, hi, bin, q0, q1, ids, rf, rl, ctr, bytes;
+	size_t lo, hi, bin, queue, ids, rf, rl, ctr, bytes;
 };
 __host__ __device__ SmallCollapseLayout smallCollapseLayout(int n)
 {
@@ -491,34 +522,33 @@ __host__ __device__ SmallCollapseLayout smallCollapseLayout(int n)
 	L.lo = 0;
 	L.hi = L.lo + up(sizeof(float4) * (size_t) n);
 	L.bin = L.hi + up(sizeof(float4) * (size_t) n);
-	L.q0 = L.bin + up(sizeof(BinNode) * m);
-	L.q1 = L.q0 + up(sizeof(int2) * (size_t) n);
-	L.ids = L.q1 + up(sizeof(int2) * (size_t) n);
+	L.queue = L.bin + up(sizeof(BinNode) * m);
+	L.ids = L.queue + up(sizeof(collapsedev::CollapseTask) * (size_t) n);
 	L.rf = L.ids + up(sizeof(int32_t) * (size_t) n);
 	L.rl = L.rf + up(sizeof(int32_t) * m);
 	L.ctr = L.rl + up(sizeof(int32_t) * m);
-	L.bytes = L.ctr + 16;
+	L.bytes = L.ctr + up(3 * sizeof(collapsedev::DepthCounter));
 	return L;
 }
 
-// The wide collapse of a small binary tree by one block, depth by depth until its queue is empty. The
-// tree, the primitive boxes, the queues and the counters live in shared memory, so each depth costs
-// shared-memory latency, not a chain of global loads. Records the first node of every depth and the
-// number of depths (the collapse allocates depth L + 1 while it writes depth L).
-__global__ void __launch_bounds__(256) kCollapseSmall(CollapseInputs gin, WideNode* wide, TriRecord* leaves, Box* boxes,
-                                                      int32_t* levelStarts, int32_t* nLevels, int n)
+// The wide collapse of a small binary tree by one block, depth by depth (as kCollapse, with block
+// barriers). The tree, the primitive boxes, the queue and the counters live in shared memory, so each
+// depth costs shared-memory latency, not a chain of global loads. Records the first node of every depth
+// and the number of depths. 94 instances: 172 us with one thread per node.
+constexpr int kSmallThreads = 256;
+__global__ void __launch_bounds__(kSmallThreads) kCollapseSmall(CollapseInputs gin, WideNode* wide, TriRecord* leaves, Box* boxes,
+                                                                int32_t* levelStarts, int32_t* nLevels, int n)
 {
 	extern __shared__ __align__(16) uint8_t smem[];
 	const SmallCollapseLayout L = smallCollapseLayout(n);
 	float4* lo = reinterpret_cast<float4*>(smem + L.lo);
 	float4* hi = reinterpret_cast<float4*>(smem + L.hi);
 	BinNode* bin = reinterpret_cast<BinNode*>(smem + L.bin);
-	int2* qa = reinterpret_cast<int2*>(smem + L.q0);
-	int2* qb = reinterpret_cast<int2*>(smem + L.q1);
+	collapsedev::CollapseTask* queue = reinterpret_cast<collapsedev::CollapseTask*>(smem + L.queue);
 	int32_t* ids = reinterpret_cast<int32_t*>(smem + L.ids);
 	int32_t* rf = reinterpret_cast<int32_t*>(smem + L.rf);
 	int32_t* rl = reinterpret_cast<int32_t*>(smem + L.rl);
-	uint32_t* counters = reinterpret_cast<uint32_t*>(smem + L.ctr);
+	collapsedev::DepthCounter* depth = reinterpret_cast<collapsedev::DepthCounter*>(smem + L.ctr);
 	for (int i = threadIdx.x; i < n; i += blockDim.x) {
 		lo[i] = gin.triLo[i];
 		hi[i] = gin.triHi[i];
@@ -529,43 +559,41 @@ __global__ void __launch_bounds__(256) kCollapseSmall(CollapseInputs gin, WideNo
 		rf[i] = gin.rangeFirst[i];
 		rl[i] = gin.rangeLast[i];
 	}
-	if (threadIdx.x == 0) {
-		counters[0] = 1u; // wide nodes (the root)
-		counters[1] = 0u; // leaf records
-		counters[2] = 1u; // items in qa
-		counters[3] = 0u;
-		qa[0] = make_int2(n == 1 ? ~0 : 0, 0);
-		levelStarts[0] = 0;
+	if (threadIdx.x < 3) {
+		depth[threadIdx.x] = 0;
 	}
+	__syncthreads();
 	const CollapseInputs in{bin, rf, rl, ids, lo, hi, nullptr, nullptr, gin.leafMax};
-	uint32_t* ca = counters + 2;
-	uint32_t* cb = counters + 3;
+	const collapsedev::CollapseTarget out{wide, leaves, boxes, queue};
+	const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, group = (threadIdx.x & 31u) >> 3;
+	uint32_t start = 0, end = 1, done = 0;
 	int level = 0;
-	for (;; ++level) {
-		__syncthreads();
-		const uint32_t cnt = *(volatile uint32_t*) ca;
-		__syncthreads();
+	for (; start < end; ++level) {
+		collapsedev::DepthCounter* ctr = &depth[level % 3];
 		if (threadIdx.x == 0) {
-			levelStarts[level + 1] = (int32_t) *(volatile uint32_t*) counters;
-			*cb = 0u;
+			depth[(level + 1) % 3] = 0;
+			levelStarts[level] = (int32_t) start; // n + 2 entries: every depth holds a node
+		}
+		for (uint32_t at = start + 4 * warp; at < end; at += 4 * warps) {
+			const uint32_t idx = at + group;
+			const bool valid = idx < end;
+			collapsedev::CollapseTask task{0, 0};
+			if (valid) {
+				task = level == 0 ? collapsedev::rootTask(bin, n) : queue[idx];
+			}
+			collapsedev::collapseGroups<false>(valid, idx, task, in, out, ctr, end, done, (uint32_t) n);
 		}
 		__syncthreads();
-		if (cnt == 0u || level > n + 1) {
-			break;
+		const collapsedev::DepthCounter got = *(volatile collapsedev::DepthCounter*) ctr;
+		start = end;
+		end += (uint32_t) got;
+		done += (uint32_t) (got >> 32);
+		if (end > (uint32_t) n || done > (uint32_t) n) {
+			break; // not a proper tree
 		}
-		const CollapseOutputs out{wide, leaves, counters, counters + 1, qb, cb, boxes};
-		for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-			const int2 it = qa[i];
-			collapseItem(it.x, (uint32_t) it.y, in, out);
-		}
-		int2* tq = qa;
-		qa = qb;
-		qb = tq;
-		uint32_t* tc = ca;
-		ca = cb;
-		cb = tc;
 	}
 	if (threadIdx.x == 0) {
+		levelStarts[level] = (int32_t) end;
 		*nLevels = level;
 	}
 }
@@ -631,7 +659,7 @@ void rebuildTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 	countLaunch();
 	enqueueSahTopologySmall(t.lo, t.hi, n, t.sahScratch, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds, s);
 	const CollapseInputs ci{t.bin, t.rangeFirst, t.rangeLast, reinterpret_cast<const int32_t*>(t.sortedIds), t.lo, t.hi, nullptr, nullptr, 1};
-	kCollapseSmall<<<1, 256, smallCollapseLayout(n).bytes, s>>>(ci, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), t.levelStarts,
+	kCollapseSmall<<<1, kSmallThreads, smallCollapseLayout(n).bytes, s>>>(ci, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), t.levelStarts,
 	                                                            t.nLevels, n);
 	countLaunch();
 }
@@ -664,21 +692,9 @@ void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBu
 	// Pageable sources: each copy is staged before the call returns.
 	RGL_CUDA_OK(cudaMemcpyAsync(lo, hLo.data(), sizeof(float4) * (size_t) n, cudaMemcpyHostToDevice, s));
 	RGL_CUDA_OK(cudaMemcpyAsync(hi, hHi.data(), sizeof(float4) * (size_t) n, cudaMemcpyHostToDevice, s));
-	std::vector<int32_t> starts;
-	const WideBuildResult r = buildWide(lo, hi, cb, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s,
-	                                    true, &starts);
+	const WideBuildResult r = buildWide(lo, hi, cb, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s, true,
+	                                    LevelRecord{t.levelStarts, t.nLevels, t.levelCapacity});
 	t.nodeCount = r.nodeCount;
-	// Depths past the deepest node hold no nodes (their starts equal the node count): dropped.
-	int levels = (int) starts.size() - 1;
-	while (levels > 1 && starts[(size_t) levels - 1] == (int32_t) r.nodeCount) {
-		--levels;
-	}
-	if (starts.back() != (int32_t) r.nodeCount || starts[(size_t) levels] != (int32_t) r.nodeCount || levels + 1 > t.levelCapacity) {
-		throw std::runtime_error("TLAS build: depth ranges do not cover the nodes");
-	}
-	RGL_CUDA_OK(cudaMemcpyAsync(t.levelStarts, starts.data(), sizeof(int32_t) * (size_t) (levels + 1), cudaMemcpyHostToDevice, s));
-	RGL_CUDA_OK(cudaMemcpyAsync(t.nLevels, &levels, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-	RGL_CUDA_OK(cudaStreamSynchronize(s));
 }
 
 void updateTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
