@@ -118,13 +118,22 @@ RGL_HD bool intersectTriangle(Vec3 a, Vec3 b, Vec3 c, Vec3 o, const Watertight& 
 	return true;
 }
 
+// Inverse of a direction component for the slab tests only, which are conservative and need no exact
+// inverse: the device's approximate reciprocal (relative error up to 2^-23) is one instruction where a
+// correctly rounded division is a sequence with a slow path, three times per frame change.
 RGL_HD float safeInv(float d)
 {
 	const float tiny = 1e-30f;
 	if (absf_(d) < tiny) {
 		d = d < 0.0f ? -tiny : tiny;
 	}
+#if defined(__CUDA_ARCH__)
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+	return r;
+#else
 	return 1.0f / d;
+#endif
 }
 
 RGL_HD float exp2Byte(uint8_t e)
@@ -157,7 +166,8 @@ RGL_HD int popc8(uint32_t x)
 //   node group      (childBase, imask | remaining-hits << 8), remaining hits != 0, so >= 256;
 //                   bit j of the hits selects slot j ^ octant of the frame the group was pushed in;
 //   enter instance  (instance index, kEnterInstance): transform the ray into the instance's frame;
-//   leave instance  (0, kLeaveInstance): back to the world frame.
+//   leave instance  (same frame, kLeaveInstance): back to the world frame; the first word is 1 when
+//                   the instance's frame is the world's (identity pose), so there is nothing to restore.
 // Entries pushed inside an instance sit above its leave entry, so each group is popped in the frame
 // it was pushed in. `Stack` provides push(a, b), pop(a&, b&), size().
 
@@ -165,8 +175,8 @@ RGL_HD int popc8(uint32_t x)
 // fma(1 + q 2^-15, S, D -+ e) with S = 2^15 A, A = s * inv (one grid step in t, exact: s is a power of
 // two), C = (p - o) * inv and D = C - S (see the node loop). Against the exact distance of the ray
 // with direction 1/inv it errs by at most
-//  * relative: inv, the FMA and the |t| share of the C terms, 6u|t| (u = 2^-24); entry and exit
-//    together 12u, covered by entry <= exit * (1 + 2e-6) (34u);
+//  * relative: inv (up to 2u), the FMA and the |t| share of the C terms, 7u|t| (u = 2^-24); entry and
+//    exit together 14u, covered by entry <= exit * (1 + 2e-6) (34u);
 //  * absolute: C rounds twice and D and D -+ e once each, 4u|C| + 2^-8 |A| with |C| <= |t| + 255 |A|,
 //    i.e. (2^-8 + 1020u) |A| < 0.0041 |A| beyond the relative part; near planes are moved earlier and
 //    far planes later by e = 0.01 |A| (kPlaneSlack).
@@ -216,6 +226,16 @@ RGL_HD float byteMantissa(uint32_t w, int k)
 	return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | ((uint32_t) k << 4)));
 #else
 	return asFloat(0x3F800000u | (((w >> (8 * k)) & 0xffu) << 8));
+#endif
+}
+
+// (mask << 1) | sign bit of f.
+RGL_HD uint32_t shiftInSign(uint32_t mask, float f)
+{
+#if defined(__CUDA_ARCH__)
+	return __funnelshift_l(__float_as_uint(f), mask, 1);
+#else
+	return (mask << 1) | (asUint(f) >> 31);
 #endif
 }
 
@@ -294,7 +314,7 @@ RGL_HD FrameRay frameRay(Vec3 o, Vec3 d)
 	r.o = o;
 	r.d = d;
 	r.inv = {safeInv(d.x), safeInv(d.y), safeInv(d.z)};
-	r.oct = (r.inv.x < 0.0f ? 1u : 0u) | (r.inv.y < 0.0f ? 2u : 0u) | (r.inv.z < 0.0f ? 4u : 0u);
+	r.oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
 	return r;
 }
 
@@ -463,11 +483,11 @@ RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, St
 		const uint32_t nx0 = negx ? w3.z : w2.x, nx1 = negx ? w3.w : w2.y, fx0 = negx ? w2.x : w3.z, fx1 = negx ? w2.y : w3.w;
 		const uint32_t ny0 = negy ? w4.x : w2.z, ny1 = negy ? w4.y : w2.w, fy0 = negy ? w2.z : w4.x, fy1 = negy ? w2.w : w4.y;
 		const uint32_t nz0 = negz ? w4.z : w3.x, nz1 = negz ? w4.w : w3.y, fz0 = negz ? w3.x : w4.z, fz1 = negz ? w3.y : w4.w;
-		uint32_t hitSlots = 0; // bit s: child slot s is hit
+		uint32_t missed = 0; // bit s: child slot s is not hit
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-		for (int s = 0; s < kWideArity; ++s) {
+		for (int s = kWideArity - 1; s >= 0; --s) {
 			const int k = s & 3;
 			const bool hiw = s >= 4;
 			const float tnx = fmaf(byteMantissa(hiw ? nx1 : nx0, k), Sx, Dnx), tfx = fmaf(byteMantissa(hiw ? fx1 : fx0, k), Sx, Dfx);
@@ -475,8 +495,12 @@ RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, St
 			const float tnz = fmaf(byteMantissa(hiw ? nz1 : nz0, k), Sz, Dnz), tfz = fmaf(byteMantissa(hiw ? fz1 : fz0, k), Sz, Dfz);
 			const float tEntry = max4(tnx, tny, tnz, 0.0f);
 			const float tExit = min4(tfx, tfy, tfz, best.t);
-			hitSlots |= (tEntry <= tExit * kSlabRelSlack) ? (1u << s) : 0u;
+			// Hit when entry <= exit * slack: the sign of the difference, shifted in from below (an FMA and
+			// a funnel shift; a multiplication, a comparison and a select per child before, two of them on
+			// the ALU pipe that bounds this loop).
+			missed = shiftInSign(missed, fmaf(tExit, kSlabRelSlack, -tEntry));
 		}
+		const uint32_t hitSlots = missed ^ 0xffu;
 		// Internal and leaf hits in traversal order j (slot = j ^ oct): one permutation for both.
 		const uint32_t ordered = octantPermute((hitSlots & imask) | ((hitSlots & ~imask & 0xffu) << 8), r.oct);
 		uint32_t internalHits = ordered & 0xffu, leafHits = ordered >> 8;
@@ -521,15 +545,23 @@ RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, St
 			uint32_t a, b;
 			st.pop(a, b);
 			if (b == kLeaveInstance) {
-				r = frameRay(oW, dW);
+				if (a == 0u) {
+					r = frameRay(oW, dW);
+				}
 				nodes = sc.tlas;
 				leaves = sc.tlasLeaves;
 				inst = -1;
 			} else if (b == kEnterInstance) {
 				const InstanceRec& ir = load.instance(sc.instances, (int32_t) a);
-				st.push(0u, kLeaveInstance);
-				const Vec3 od = ir.worldToObject.vector(dW);
-				r = frameRay(worldToInstance(ir, oW), od);
+				// An identity pose (a scene-sized mesh, most rays' last instance) maps the ray to itself
+				// exactly: the frame stays, here and on leaving.
+				const bool identity = (ir.flags & kInstanceIdentity) != 0;
+				st.push(identity ? 1u : 0u, kLeaveInstance);
+				Vec3 od = dW;
+				if (!identity) {
+					od = ir.worldToObject.vector(dW);
+					r = frameRay(worldToInstance(ir, oW), od);
+				}
 				wt = setupWatertight(od);
 				nodes = ir.nodes;
 				leaves = ir.tris;
