@@ -230,8 +230,7 @@ void BatchRun::uploadJobs(const rgl::BatchSchedule& s, cudaStream_t st)
 		rgl::BatchJob& b = jobs[j];
 		b.order = (s.order != rgl::kOrderNatural && orderHeld == s.order) ? dOrder.as<uint32_t>() + beamBase[j] : nullptr;
 		base[j] = (int32_t) tasks;
-		const int per = rgl::batchBeamsPerTask(s.packing, b.p.nSamples);
-		tasks += (b.p.nRays + per - 1) / per;
+		tasks += rgl::setJobTasks(b, s.packing, beams);
 	}
 	base[n] = (int32_t) tasks;
 	for (int w = 0; w < waveCount(); ++w) {

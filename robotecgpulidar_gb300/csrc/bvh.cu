@@ -537,6 +537,7 @@ __host__ __device__ SmallCollapseLayout smallCollapseLayout(int n)
 // and the number of depths. 94 instances: 172 us with one thread per node.
 constexpr int kSmallThreads = 256;
 __global__ void __launch_bounds__(kSmallThreads) kCollapseSmall(CollapseInputs gin, WideNode* wide, TriRecord* leaves, Box* boxes,
+                                                                const InstanceRec* __restrict__ inst, EnterRec* enter,
                                                                 int32_t* levelStarts, int32_t* nLevels, int n)
 {
 	extern __shared__ __align__(16) uint8_t smem[];
@@ -596,6 +597,21 @@ __global__ void __launch_bounds__(kSmallThreads) kCollapseSmall(CollapseInputs g
 		levelStarts[level] = (int32_t) end;
 		*nLevels = level;
 	}
+	for (int i = threadIdx.x; i < n; i += blockDim.x) {
+		const int32_t k = leaves[i].primId; // written by this block before its last barrier
+		enter[i] = enterRecord(inst[k], k);
+	}
+}
+
+// Enter records of the TLAS's leaf records (after a build or a refit of more than kSahSmallMax instances;
+// the one-block collapse writes them itself).
+__global__ void kEnterRecords(const TriRecord* __restrict__ leaves, const InstanceRec* __restrict__ inst, int n, EnterRec* enter)
+{
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i < n) {
+		const int32_t k = leaves[i].primId;
+		enter[i] = enterRecord(inst[k], k);
+	}
 }
 
 } // namespace
@@ -627,6 +643,7 @@ void allocTlas(TlasBuild& t, int n)
 		t.capacity = n;
 		RGL_CUDA_OK(cudaMalloc(&t.nodes, sizeof(WideNode) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.leaves, sizeof(TriRecord) * (size_t) n));
+		RGL_CUDA_OK(cudaMalloc(&t.enter, sizeof(EnterRec) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.boxes, sizeof(Box) * (size_t) n));
 		t.levelCapacity = n + 2;
 		RGL_CUDA_OK(cudaMalloc(&t.levelStarts, sizeof(int32_t) * (size_t) t.levelCapacity));
@@ -659,8 +676,8 @@ void rebuildTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 	countLaunch();
 	enqueueSahTopologySmall(t.lo, t.hi, n, t.sahScratch, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds, s);
 	const CollapseInputs ci{t.bin, t.rangeFirst, t.rangeLast, reinterpret_cast<const int32_t*>(t.sortedIds), t.lo, t.hi, nullptr, nullptr, 1};
-	kCollapseSmall<<<1, kSmallThreads, smallCollapseLayout(n).bytes, s>>>(ci, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), t.levelStarts,
-	                                                            t.nLevels, n);
+	kCollapseSmall<<<1, kSmallThreads, smallCollapseLayout(n).bytes, s>>>(ci, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), dInst,
+	                                                                      t.enter, t.levelStarts, t.nLevels, n);
 	countLaunch();
 }
 
@@ -695,6 +712,8 @@ void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBu
 	const WideBuildResult r = buildWide(lo, hi, cb, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s, true,
 	                                    LevelRecord{t.levelStarts, t.nLevels, t.levelCapacity});
 	t.nodeCount = r.nodeCount;
+	kEnterRecords<<<blocks(n, 128), 128, 0, s>>>(t.leaves, dInst, n, t.enter);
+	countLaunch();
 }
 
 void updateTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
@@ -715,13 +734,14 @@ void refitTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 		return;
 	}
 	kRefitTlas<<<1, 256, 0, s>>>(t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), dInst, t.levelStarts, t.nLevels);
-	countLaunch();
+	kEnterRecords<<<blocks(t.nInstances, 128), 128, 0, s>>>(t.leaves, dInst, t.nInstances, t.enter);
+	countLaunch(2);
 }
 
 void freeTlas(TlasBuild& t)
 {
 	freeSmallScratch(t);
-	void* ptrs[] = {t.nodes, t.leaves, t.boxes, t.levelStarts, t.nLevels};
+	void* ptrs[] = {t.nodes, t.leaves, t.enter, t.boxes, t.levelStarts, t.nLevels};
 	for (void* p : ptrs) {
 		cudaFree(p);
 	}

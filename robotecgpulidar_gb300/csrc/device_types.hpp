@@ -94,6 +94,37 @@ constexpr int32_t kInstanceIdentity = 1;
 // 400 m from the world origin would otherwise shift ray origins by ~3e-5 m).
 RGL_HD Vec3 worldToInstance(const InstanceRec& ir, Vec3 pW) { return ir.worldToObject.vector(pW - ir.objectToWorld.translation()); }
 
+// What a ray needs to enter an instance, in the TLAS's leaf order (a TLAS leaf record and its enter
+// record have the same index) and with the size of a wide node: the traversal loads one like the other,
+// with five 128-bit loads, and a leaf hit needs no lookup of its instance first.
+struct alignas(16) EnterRec
+{
+	float m[3][4];           // rows of the world->object rotation and scale; last column: the instance's origin
+	const WideNode* nodes;
+	const TriRecord* tris;
+	int32_t inst;            // instance index
+	int32_t flags;
+	int32_t pad[2];
+};
+static_assert(sizeof(EnterRec) == sizeof(WideNode), "enter records load like wide nodes");
+
+RGL_HD EnterRec enterRecord(const InstanceRec& ir, int32_t index)
+{
+	EnterRec e;
+	for (int r = 0; r < 3; ++r) {
+		for (int c = 0; c < 3; ++c) {
+			e.m[r][c] = ir.worldToObject.m[r][c];
+		}
+		e.m[r][3] = ir.objectToWorld.m[r][3];
+	}
+	e.nodes = ir.nodes;
+	e.tris = ir.tris;
+	e.inst = index;
+	e.flags = ir.flags;
+	e.pad[0] = e.pad[1] = 0;
+	return e;
+}
+
 // Device view of a scene, read by the traversal kernel through one pointer so a captured CUDA graph
 // stays valid when the acceleration structure is rebuilt.
 struct SceneView
@@ -103,6 +134,7 @@ struct SceneView
 	const InstanceRec* instances;
 	int32_t nInstances;
 	int32_t pad;
+	const EnterRec* enter;        // enter records, by TLAS leaf record
 };
 
 // Sub-ray table and per-launch parameters of a raytrace (reference RaytraceRequestContext,
@@ -178,15 +210,16 @@ struct TraceParams
 };
 
 // One sensor (or served request) of a batched traversal launch (trace_batch.cu): its raytrace
-// parameters including its scene, its sub-ray rotations, an optional beam visiting order, the
-// lane-group width of lane-group packing, and optionally a sensor pose applied to sensor-local rays
+// parameters including its scene, its sub-ray rotations, an optional beam visiting order, how its
+// beams are cut into tasks, and optionally a sensor pose applied to sensor-local rays
 // and an inline range.
 struct BatchJob
 {
 	TraceParams p;         // p.ranges == null: inlineRange applies to every ray
 	const Mat34* samples;  // p.nSamples rotations (entry 0 is the primary ray and is not read)
 	const uint32_t* order; // permutation of [0, p.nRays), or null for the natural order
-	int32_t groupSize;     // min(p.nSamples, 32)
+	int32_t beamsPerTask;  // beams that one warp takes at a time (setJobTasks)
+	uint32_t sampleMagic;  // ceil(65536 / p.nSamples): i / p.nSamples = (i * magic) >> 16 within a task
 	int32_t hasRayTransform; // world ray = mul(rayTransform, ray), as a rays-transform node computes it
 	Mat34 rayTransform;
 	float inlineRange[2];

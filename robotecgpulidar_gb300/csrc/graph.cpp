@@ -580,7 +580,6 @@ void RaytraceNode::fillJob(rgl::BatchJob& b)
 	b.p = traceParams();
 	b.samples = sampleTable.as<Mat34>();
 	b.order = nullptr;
-	b.groupSize = std::min(b.p.nSamples, 32);
 	if (foldedTransform) {
 		b.p.rays = foldedTransform->sourceRaysDev();
 		b.hasRayTransform = 1;
@@ -628,10 +627,9 @@ void RaytraceNode::stageJob(cudaStream_t s)
 	}
 	const rgl::TraceParams& p = b.p;
 	(void) job.device();
-	const int per = rgl::batchBeamsPerTask(schedule.packing, p.nSamples);
 	rgl::TaskRange& tr = job.host().tasks;
 	tr.base[0] = 0;
-	tr.base[1] = (p.nRays + per - 1) / per;
+	tr.base[1] = rgl::setJobTasks(b, schedule.packing, b.p.nRays);
 	shading = rgl::needsShadingKernel(p);
 	if (counter.get() == nullptr) {
 		RGL_CHECK_CUDA(cudaMemset(counter.ensure(rgl::kTraceCounterBytes), 0, rgl::kTraceCounterBytes));

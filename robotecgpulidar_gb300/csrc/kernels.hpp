@@ -56,6 +56,7 @@ struct TlasBuild
 {
 	WideNode* nodes = nullptr;       // wide nodes over the instances (at most nInstances)
 	TriRecord* leaves = nullptr;     // one record per instance; primId = instance index
+	EnterRec* enter = nullptr;       // enter record of every leaf record
 	float* boxes = nullptr;          // float box (6 floats) of every wide node, kept for the refit
 	int32_t* levelStarts = nullptr;  // first node index of each depth, nLevels + 1 entries (device)
 	int32_t* nLevels = nullptr;      // number of depths (device word, read by the refit)
@@ -105,7 +106,7 @@ void launchUpdateVertices(int nVertices, float* newToDisplacement, float* oldToN
 constexpr int kMaxBatchJobs = 1024;
 enum BatchPacking : int32_t
 {
-	kPackLaneGroup = 0, // a beam's samples on adjacent lanes, in-order shuffle reduction
+	kPackLaneGroup = 0, // a beam's samples on adjacent lanes: lane groups, or pooled samples for larger patterns
 	kPackSerial = 1,    // one lane per beam, samples traced one after another
 };
 enum BeamOrder : int32_t
@@ -135,8 +136,23 @@ inline bool needsShadingKernel(const TraceParams& p)
 	return p.needIntensity != 0 || p.out.normal != nullptr || p.out.incidentAngle != nullptr || p.out.absVelocity != nullptr ||
 	       p.out.relVelocity != nullptr || p.out.radialSpeed != nullptr || p.distortion != 0;
 }
-// Beams covered by one task (one warp's worth of work) of a sensor with `nSamples` samples.
-int batchBeamsPerTask(int packing, int nSamples);
+// Lane groups take patterns of up to this many samples. Beyond, lanes idle (17 samples leave 15 of 32) and
+// the selection, done by one lane per beam, weighs more: 58 samples on two rounds of 32 lanes took
+// 2276 us for 65,536 beams over 1M triangles, pooled 1195 us; 5 samples took 302 us for 262,144 beams
+// in groups, pooled 327 us (the pool and the poses read again for six beams a task).
+constexpr int kLaneGroupSamples = 8;
+// Samples that a warp keeps in shared memory between tracing a task's beams and selecting their returns.
+constexpr int kPoolSamples = 352; // 6 beams of 58: two blocks of 256 threads with shading keep 98 KB each
+static_assert(kPoolSamples >= kMaxBeamSamples, "a beam's samples fit the pool");
+// Cuts a job's beams into tasks (one warp's work each) for a packing: sets the job's beamsPerTask and
+// sampleMagic and returns the number of tasks. launchBeams: beams of all jobs of the launch. A launch
+// that does not fill the chip twice over takes fewer beams per task, because a warp ends with its
+// slowest ray and fewer rays diverge less: with 32 beams, 16, 8 and 1 per task, 3,600 beams took 35 / 33
+// / 37 / 32 us, 32,768 beams 39 / 37 / 36 / 101 us, 76,920 beams 112 / 97 / 99 / 365 us, 131,072 beams 92
+// / 89 / 98 / 474 us. Pooled samples want about eight tasks per warp (58 samples, 65,536 beams: 1221 /
+// 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per task): fewer leave a long tail.
+constexpr int kResidentWarps = 16; // per SM, at 128 registers
+int setJobTasks(BatchJob& job, int packing, int64_t launchBeams);
 // Resolves and caches the launch configuration (occupancy, shared-memory opt-in) of a schedule;
 // call it outside stream capture before the first captured launch of that schedule.
 void prepareTraceBatch(int nJobs, int maxSamples, bool shading, const BatchSchedule& s);

@@ -466,6 +466,7 @@ void Scene::prepare(cudaStream_t s)
 	v->instances = dInst;
 	v->nInstances = n;
 	v->pad = 0;
+	v->enter = tlas.enter;
 	RGL_CHECK_CUDA(cudaMemcpyAsync(dView.ensure(sizeof(rgl::SceneView)), v, sizeof(rgl::SceneView), cudaMemcpyHostToDevice, s));
 	RGL_CHECK_CUDA(cudaEventRecord(ready, s));
 	readyRecorded = true;

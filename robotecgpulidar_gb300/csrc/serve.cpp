@@ -445,9 +445,10 @@ void Server::configure(const rgl::BatchSchedule& s, int64_t maxBeams)
 void Server::launch(Slot& slot, const rgl::BatchSchedule& sched, Slot* after)
 {
 	const int n = (int) slot.reqs.size();
-	int64_t points = 0;
+	int64_t points = 0, beams = 0;
 	for (auto* r : slot.reqs) {
 		points += r->points;
+		beams += r->beams;
 	}
 	int64_t maxTiles = 0;
 	for (auto* r : slot.reqs) {
@@ -496,14 +497,13 @@ void Server::launch(Slot& slot, const rgl::BatchSchedule& sched, Slot* after)
 		b.order = sched.order == rgl::kOrderNatural     ? nullptr
 		          : sched.order == rgl::kOrderElevation ? patterns[r.pattern]->rowOrder.as<uint32_t>()
 		                                                : patterns[r.pattern]->order.as<uint32_t>();
-		b.groupSize = 1;
 		b.hasRayTransform = 1;
 		b.rayTransform = r.pose;
 		b.inlineRange[0] = r.minRange;
 		b.inlineRange[1] = r.maxRange;
-		jobs[j] = b;
 		taskBase[j] = (int32_t) tasks;
-		tasks += (r.beams + 31) / 32;
+		tasks += rgl::setJobTasks(b, sched.packing, beams);
+		jobs[j] = b;
 
 		rgl::SegCompactJob sg{};
 		sg.flags = flags + pointBase;

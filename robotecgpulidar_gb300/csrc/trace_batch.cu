@@ -9,11 +9,12 @@
 //
 // Each job names its own scene, so one launch may cover sensors of several resident scenes.
 //
-// Scheduling: the beams of sensor j form tasks of one warp's worth of work (32 / G beams with the
-// lane-group packing, 32 beams with the serial packing). A persistent grid of
+// Scheduling: the beams of sensor j form tasks (up to 32 beams and kPoolSamples samples with pooled
+// samples, 32 beams with one lane per beam). A persistent grid of
 // (SM count x resident blocks) blocks fetches `chunk` tasks at a time from one global counter; a
 // warp maps a task to its sensor by binary search over the task prefix sums staged in shared memory.
 // Sensors of uneven size therefore share the GPU without a tail per sensor.
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -66,7 +67,7 @@ __device__ __forceinline__ uint32_t quant(float x, uint32_t levels)
 // folded onto the octahedron, 11 bits per coordinate, interleaved. Morton: the point 5 % of the world
 // diagonal along the ray, 7 bits per axis over the world box, interleaved.
 __global__ void kBeamKeys(const Mat34* __restrict__ rays, Mat34 tf, int hasTf, int n, uint32_t jobIndex, int order, float3 lo, float3 inv,
-                          float probe, uint32_t* __restrict__ keys, uint32_t* __restrict__ values)
+                          float probe, float3 worldLo, float3 worldHi, uint32_t* __restrict__ keys, uint32_t* __restrict__ values)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) {
@@ -91,12 +92,19 @@ __global__ void kBeamKeys(const Mat34* __restrict__ rays, Mat34 tf, int hasTf, i
 		}
 		code = (spread2(quant(u * 0.5f + 0.5f, 2048u)) << 1) | spread2(quant(v * 0.5f + 0.5f, 2048u));
 	} else if (order == kOrderElevation) {
-		// Rows of a scan: the sine of the elevation above the world xy plane in the high 11 bits, a
-		// pseudo-angle of the azimuth (monotonic in atan2(y, x), in (-2, 2]) in the low 11 bits.
+		// Rows of a scan: the sine of the elevation above the world xy plane in the middle 10 bits, a
+		// pseudo-angle of the azimuth (monotonic in atan2(y, x), in (-2, 2]) in the low 10 bits. Above
+		// them, a class of the ray's way through the world box, the longest ways first (more than 1/4,
+		// 1/8, 1/16 of the box's diagonal): these rays take the most steps (35-58 against 10), and a
+		// launch that reaches them last ends with a few warps busy.
 		const float l1 = fabsf(d.x) + fabsf(d.y);
 		const float pa = l1 > 0.0f ? 1.0f - d.x / l1 : 0.0f;
 		const float az = d.y < 0.0f ? -pa : pa;
-		code = (quant(d.z * 0.5f + 0.5f, 2048u) << 11) | quant(az * 0.25f + 0.5f, 2048u);
+		const float wx = ((d.x > 0.0f ? worldHi.x : worldLo.x) - o.x) / d.x, wy = ((d.y > 0.0f ? worldHi.y : worldLo.y) - o.y) / d.y,
+		            wz = ((d.z > 0.0f ? worldHi.z : worldLo.z) - o.z) / d.z;
+		const float way = fminf(fminf(wx, wy), wz); // to the box's far side; 20 * probe is its diagonal
+		const uint32_t cls = way > 5.0f * probe ? 0u : (way > 2.5f * probe ? 1u : (way > 1.25f * probe ? 2u : 3u));
+		code = (cls << 20) | (quant(d.z * 0.5f + 0.5f, 1024u) << 10) | quant(az * 0.25f + 0.5f, 1024u);
 	} else {
 		const float px = (o.x + d.x * probe - lo.x) * inv.x;
 		const float py = (o.y + d.y * probe - lo.y) * inv.y;
@@ -120,6 +128,12 @@ const void* batchKernel(int regs)
 	                  : reinterpret_cast<const void*>(&kTraceBatch<MODE, SHADING, 128>);
 }
 
+size_t poolBytes(bool shading, int block)
+{
+	const size_t entry = shading ? sizeof(PoolEntry<true>) : sizeof(PoolEntry<false>);
+	return entry * (size_t) kPoolSamples * (size_t) (block / 32);
+}
+
 int residentBlocks(const void* fn, int block, size_t smem)
 {
 	static std::mutex m;
@@ -134,7 +148,7 @@ int residentBlocks(const void* fn, int block, size_t smem)
 	if (!optedIn[fn]) {
 		// Opt in once to the largest launch of this kernel (256-thread stack + the largest job
 		// table), so no later launch, whatever its shape, exceeds the limit.
-		const int most = (int) (sizeof(uint2) * kSmemStack * 256 + sizeof(int32_t) * (kMaxBatchJobs + 2));
+		const int most = (int) (sizeof(uint2) * kSmemStack * 256 + poolBytes(true, 256) + sizeof(int32_t) * (kMaxBatchJobs + 2));
 		RGL_BATCH_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 		optedIn[fn] = true;
 	}
@@ -158,13 +172,19 @@ int smCount()
 
 } // namespace
 
-int batchBeamsPerTask(int packing, int nSamples)
+int setJobTasks(BatchJob& job, int packing, int64_t launchBeams)
 {
-	if (packing == kPackSerial) {
-		return 32;
+	const int S = job.p.nSamples;
+	int beams = 32;
+	if (packing != kPackSerial) {
+		const int64_t resident = (int64_t) smCount() * kResidentWarps;
+		const int64_t want = S <= kLaneGroupSamples ? (launchBeams + 2 * resident - 1) / (2 * resident) : launchBeams / (8 * resident);
+		const int most = S <= kLaneGroupSamples ? 32 / S : std::min(32, kPoolSamples / S);
+		beams = (int) std::max<int64_t>(1, std::min<int64_t>(want, most));
 	}
-	const int G = nSamples < 32 ? nSamples : 32;
-	return 32 / G;
+	job.beamsPerTask = beams;
+	job.sampleMagic = (uint32_t) ((65536 + S - 1) / S);
+	return (job.p.nRays + beams - 1) / beams;
 }
 
 namespace {
@@ -179,7 +199,8 @@ LaunchShape batchLaunchShape(int nJobs, int maxSamples, bool shading, const Batc
 {
 	// Sensor count (<= kMaxBatchJobs) and block size (64, 128 or 256) are checked by the caller.
 	const int block = s.block;
-	const int mode = s.packing == kPackSerial ? 2 : (maxSamples > 32 ? 1 : 0);
+	// Any job with more samples than lane groups hold takes the whole launch to pooled samples.
+	const int mode = s.packing == kPackSerial ? 1 : (maxSamples > kLaneGroupSamples ? 2 : 0);
 	const void* fn = nullptr;
 	switch (mode * 2 + (shading ? 1 : 0)) {
 		case 0: fn = batchKernel<0, false>(s.regs); break;
@@ -189,7 +210,8 @@ LaunchShape batchLaunchShape(int nJobs, int maxSamples, bool shading, const Batc
 		case 4: fn = batchKernel<2, false>(s.regs); break;
 		default: fn = batchKernel<2, true>(s.regs); break;
 	}
-	const size_t smem = sizeof(uint2) * kSmemStack * block + sizeof(int32_t) * ((nJobs + 2) & ~1);
+	const size_t smem =
+	    sizeof(uint2) * kSmemStack * block + (mode == 2 ? poolBytes(shading, block) : 0) + sizeof(int32_t) * ((nJobs + 2) & ~1);
 	return LaunchShape{fn, smem, smCount() * residentBlocks(fn, block, smem)};
 }
 } // namespace
@@ -252,7 +274,9 @@ void launchBeamKeys(const Mat34* rays, const Mat34* transform, int n, uint32_t j
 	lo.z -= probe;
 	const float3 inv = make_float3(1.0f / (ex + 2 * probe), 1.0f / (ey + 2 * probe), 1.0f / (ez + 2 * probe));
 	const Mat34 tf = transform ? *transform : Mat34::identity();
-	kBeamKeys<<<(n + 255) / 256, 256, 0, stream>>>(rays, tf, transform ? 1 : 0, n, jobIndex, order, lo, inv, probe, keys, values);
+	kBeamKeys<<<(n + 255) / 256, 256, 0, stream>>>(rays, tf, transform ? 1 : 0, n, jobIndex, order, lo, inv, probe,
+	                                               make_float3(worldLo[0], worldLo[1], worldLo[2]), make_float3(worldHi[0], worldHi[1], worldHi[2]), keys,
+	                                               values);
 	countLaunch();
 }
 

@@ -442,6 +442,140 @@ RGL_HD HitRec refineClosest(const SceneView& sc, Vec3 oW, Vec3 dW, HitRec best, 
 	return best;
 }
 
+// A wide node as loaded, and what traversal reads of it.
+struct NodeWords
+{
+	uint4 w0, w1, w2, w3, w4;
+	RGL_HD uint32_t imask() const { return w0.w >> 24; }
+	RGL_HD uint32_t childBase() const { return w1.x; }
+	// Leaf child in slot s: first triangle record and count.
+	RGL_HD void leaf(uint32_t s, int& first, int& count) const
+	{
+		const uint32_t meta = ((s < 4 ? w1.z : w1.w) >> ((s & 3) * 8)) & 0xffu;
+		first = (int) w1.y + (int) (meta & 31u);
+		count = (int) (meta >> 5);
+	}
+};
+
+// Child slots of a node whose boxes the ray enters at or before tBest (bit s: slot s).
+RGL_HD uint32_t slabHits(const NodeWords& n, Vec3 o, Vec3 inv, uint32_t oct, float tBest)
+{
+	const float sx = exp2Byte((uint8_t) (n.w0.w & 0xffu)), sy = exp2Byte((uint8_t) ((n.w0.w >> 8) & 0xffu)),
+	            sz = exp2Byte((uint8_t) ((n.w0.w >> 16) & 0xffu));
+	const float Ax = sx * inv.x, Ay = sy * inv.y, Az = sz * inv.z;
+	const float Cx = (asFloat(n.w0.x) - o.x) * inv.x, Cy = (asFloat(n.w0.y) - o.y) * inv.y, Cz = (asFloat(n.w0.z) - o.z) * inv.z;
+	// Plane distance q * A + C evaluated as fma(1 + q * 2^-15, 2^15 * A, C - 2^15 * A): 2^15 * A and
+	// the product term are exact; the error bound and the slacks that cover it are derived above
+	// kSlabRelSlack.
+	const float Sx = 32768.0f * Ax, Sy = 32768.0f * Ay, Sz = 32768.0f * Az;
+	const float Dx = Cx - Sx, Dy = Cy - Sy, Dz = Cz - Sz;
+	// Near planes earlier, far planes later, by kPlaneSlack grid steps.
+	const float ex = kPlaneSlack * absf_(Sx), ey = kPlaneSlack * absf_(Sy), ez = kPlaneSlack * absf_(Sz);
+	const float Dnx = Dx - ex, Dny = Dy - ey, Dnz = Dz - ez, Dfx = Dx + ex, Dfy = Dy + ey, Dfz = Dz + ez;
+	// near/far quantised planes per axis (packed bytes), swapped for negative directions
+	const bool negx = (oct & 1u) != 0, negy = (oct & 2u) != 0, negz = (oct & 4u) != 0;
+	const uint32_t nx0 = negx ? n.w3.z : n.w2.x, nx1 = negx ? n.w3.w : n.w2.y, fx0 = negx ? n.w2.x : n.w3.z, fx1 = negx ? n.w2.y : n.w3.w;
+	const uint32_t ny0 = negy ? n.w4.x : n.w2.z, ny1 = negy ? n.w4.y : n.w2.w, fy0 = negy ? n.w2.z : n.w4.x, fy1 = negy ? n.w2.w : n.w4.y;
+	const uint32_t nz0 = negz ? n.w4.z : n.w3.x, nz1 = negz ? n.w4.w : n.w3.y, fz0 = negz ? n.w3.x : n.w4.z, fz1 = negz ? n.w3.y : n.w4.w;
+	uint32_t missed = 0; // bit s: child slot s is not hit
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+	for (int s = kWideArity - 1; s >= 0; --s) {
+		const int k = s & 3;
+		const bool hiw = s >= 4;
+		const float tnx = fmaf(byteMantissa(hiw ? nx1 : nx0, k), Sx, Dnx), tfx = fmaf(byteMantissa(hiw ? fx1 : fx0, k), Sx, Dfx);
+		const float tny = fmaf(byteMantissa(hiw ? ny1 : ny0, k), Sy, Dny), tfy = fmaf(byteMantissa(hiw ? fy1 : fy0, k), Sy, Dfy);
+		const float tnz = fmaf(byteMantissa(hiw ? nz1 : nz0, k), Sz, Dnz), tfz = fmaf(byteMantissa(hiw ? fz1 : fz0, k), Sz, Dfz);
+		const float tEntry = max4(tnx, tny, tnz, 0.0f);
+		const float tExit = min4(tfx, tfy, tfz, tBest);
+		// Hit when entry <= exit * slack: the sign of the difference, shifted in from below (an FMA and
+		// a funnel shift; a multiplication, a comparison and a select per child before, two of them on
+		// the ALU pipe that bounds this loop).
+		missed = shiftInSign(missed, fmaf(tExit, kSlabRelSlack, -tEntry));
+	}
+	return missed ^ 0xffu;
+}
+
+// Tests the triangles of a BLAS node's leaf children among `leafHits` (bit j: slot j ^ oct), in ray
+// order, keeping the closest in `best`.
+template<class NodeLoader>
+RGL_HD void testLeaves(const NodeWords& n, uint32_t leafHits, uint32_t oct, const TriRecord* leaves, int32_t inst, Vec3 o, const Watertight& wt,
+                       HitRec& best, const NodeLoader& load)
+{
+	while (leafHits) {
+		const uint32_t s = lowestBit(leafHits) ^ oct;
+		leafHits &= leafHits - 1u;
+		int first, cnt;
+		n.leaf(s, first, cnt);
+		// A leaf's triangles are loaded together before the first is tested: a step of the walk waits for
+		// its loads one after another (with a load per test the 1M-triangle scan took 305 us, so 293).
+		TriRecord tr[kLeafMaxTris];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+		for (int k = 0; k < kLeafMaxTris; ++k) {
+			if (k < cnt) {
+				tr[k] = load.tri(leaves, first + k);
+			}
+		}
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+		for (int k = 0; k < kLeafMaxTris; ++k) {
+			float t;
+			if (k < cnt &&
+			    intersectTriangle(v3(tr[k].v0x, tr[k].v0y, tr[k].v0z), v3(tr[k].v1x, tr[k].v1y, tr[k].v1z), v3(tr[k].v2x, tr[k].v2y, tr[k].v2z),
+			                      o, wt, best.t, t) &&
+			    closerHit(t, inst, tr[k].primId, best)) {
+				best.t = t;
+				best.inst = inst;
+				best.tri = first + k;
+				best.prim = tr[k].primId;
+			}
+		}
+	}
+}
+
+// The stack entry of a TLAS leaf, and what entering it needs. On the device a leaf record's index leads to
+// its enter record directly (the scan above: 293 us with the instance looked up first and its record
+// read field by field, so 286); without enter records, on the host, the leaf record names the instance.
+template<class NodeLoader>
+RGL_HD uint32_t tlasLeafEntry(const TriRecord* leaves, int first, const NodeLoader& load)
+{
+#if defined(__CUDA_ARCH__)
+	(void) leaves;
+	(void) load;
+	return (uint32_t) first;
+#else
+	return (uint32_t) load.leafPrim(leaves, first);
+#endif
+}
+template<class NodeLoader>
+RGL_HD EnterRec loadEnter(const SceneView& sc, uint32_t entry, const NodeLoader& load)
+{
+#if defined(__CUDA_ARCH__)
+	NodeWords n;
+	load.nodeWords(reinterpret_cast<const WideNode*>(sc.enter), entry, n.w0, n.w1, n.w2, n.w3, n.w4);
+	EnterRec e;
+	const uint4 rows[3] = {n.w0, n.w1, n.w2};
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		e.m[k][0] = asFloat(rows[k].x);
+		e.m[k][1] = asFloat(rows[k].y);
+		e.m[k][2] = asFloat(rows[k].z);
+		e.m[k][3] = asFloat(rows[k].w);
+	}
+	e.nodes = reinterpret_cast<const WideNode*>(((unsigned long long) n.w3.y << 32) | n.w3.x);
+	e.tris = reinterpret_cast<const TriRecord*>(((unsigned long long) n.w3.w << 32) | n.w3.z);
+	e.inst = (int32_t) n.w4.x;
+	e.flags = (int32_t) n.w4.y;
+	return e;
+#else
+	return enterRecord(load.instance(sc.instances, (int32_t) entry), (int32_t) entry);
+#endif
+}
+
 // Closest hit over all instances for a world-space ray o + t d, t in (0, tmax].
 template<class Stack, class NodeLoader>
 RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, Stack& st, const NodeLoader& load)
@@ -458,85 +592,30 @@ RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, St
 	FrameRay r = frameRay(oW, dW);
 	Watertight wt = setupWatertight(dW); // valid inside an instance
 	const WideNode* nodes = sc.tlas;
-	const TriRecord* leaves = sc.tlasLeaves;
-	int32_t inst = -1; // -1: the TLAS (world frame)
+	const TriRecord* leaves = nullptr; // of the instance entered
+	int32_t inst = -1;                 // -1: the TLAS (world frame)
 	uint32_t node = 0;
 	for (;;) {
-		uint4 w0, w1, w2, w3, w4;
-		load.nodeWords(nodes, node, w0, w1, w2, w3, w4);
-		const float sx = exp2Byte((uint8_t) (w0.w & 0xffu)), sy = exp2Byte((uint8_t) ((w0.w >> 8) & 0xffu)),
-		            sz = exp2Byte((uint8_t) ((w0.w >> 16) & 0xffu));
-		const uint32_t imask = w0.w >> 24;
-		const uint32_t childBase = w1.x, triBase = w1.y;
-		const float Ax = sx * r.inv.x, Ay = sy * r.inv.y, Az = sz * r.inv.z;
-		const float Cx = (asFloat(w0.x) - r.o.x) * r.inv.x, Cy = (asFloat(w0.y) - r.o.y) * r.inv.y, Cz = (asFloat(w0.z) - r.o.z) * r.inv.z;
-		// Plane distance q * A + C evaluated as fma(1 + q * 2^-15, 2^15 * A, C - 2^15 * A): 2^15 * A and
-		// the product term are exact; the error bound and the slacks that cover it are derived above
-		// kSlabRelSlack.
-		const float Sx = 32768.0f * Ax, Sy = 32768.0f * Ay, Sz = 32768.0f * Az;
-		const float Dx = Cx - Sx, Dy = Cy - Sy, Dz = Cz - Sz;
-		// Near planes earlier, far planes later, by kPlaneSlack grid steps.
-		const float ex = kPlaneSlack * absf_(Sx), ey = kPlaneSlack * absf_(Sy), ez = kPlaneSlack * absf_(Sz);
-		const float Dnx = Dx - ex, Dny = Dy - ey, Dnz = Dz - ez, Dfx = Dx + ex, Dfy = Dy + ey, Dfz = Dz + ez;
-		// near/far quantised planes per axis (packed bytes), swapped for negative directions
-		const bool negx = (r.oct & 1u) != 0, negy = (r.oct & 2u) != 0, negz = (r.oct & 4u) != 0;
-		const uint32_t nx0 = negx ? w3.z : w2.x, nx1 = negx ? w3.w : w2.y, fx0 = negx ? w2.x : w3.z, fx1 = negx ? w2.y : w3.w;
-		const uint32_t ny0 = negy ? w4.x : w2.z, ny1 = negy ? w4.y : w2.w, fy0 = negy ? w2.z : w4.x, fy1 = negy ? w2.w : w4.y;
-		const uint32_t nz0 = negz ? w4.z : w3.x, nz1 = negz ? w4.w : w3.y, fz0 = negz ? w3.x : w4.z, fz1 = negz ? w3.y : w4.w;
-		uint32_t missed = 0; // bit s: child slot s is not hit
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-		for (int s = kWideArity - 1; s >= 0; --s) {
-			const int k = s & 3;
-			const bool hiw = s >= 4;
-			const float tnx = fmaf(byteMantissa(hiw ? nx1 : nx0, k), Sx, Dnx), tfx = fmaf(byteMantissa(hiw ? fx1 : fx0, k), Sx, Dfx);
-			const float tny = fmaf(byteMantissa(hiw ? ny1 : ny0, k), Sy, Dny), tfy = fmaf(byteMantissa(hiw ? fy1 : fy0, k), Sy, Dfy);
-			const float tnz = fmaf(byteMantissa(hiw ? nz1 : nz0, k), Sz, Dnz), tfz = fmaf(byteMantissa(hiw ? fz1 : fz0, k), Sz, Dfz);
-			const float tEntry = max4(tnx, tny, tnz, 0.0f);
-			const float tExit = min4(tfx, tfy, tfz, best.t);
-			// Hit when entry <= exit * slack: the sign of the difference, shifted in from below (an FMA and
-			// a funnel shift; a multiplication, a comparison and a select per child before, two of them on
-			// the ALU pipe that bounds this loop).
-			missed = shiftInSign(missed, fmaf(tExit, kSlabRelSlack, -tEntry));
-		}
-		const uint32_t hitSlots = missed ^ 0xffu;
+		NodeWords n;
+		load.nodeWords(nodes, node, n.w0, n.w1, n.w2, n.w3, n.w4);
+		const uint32_t imask = n.imask();
+		const uint32_t hitSlots = slabHits(n, r.o, r.inv, r.oct, best.t);
 		// Internal and leaf hits in traversal order j (slot = j ^ oct): one permutation for both.
 		const uint32_t ordered = octantPermute((hitSlots & imask) | ((hitSlots & ~imask & 0xffu) << 8), r.oct);
 		uint32_t internalHits = ordered & 0xffu, leafHits = ordered >> 8;
-		const uint32_t metaLo = w1.z, metaHi = w1.w;
 		if (inst < 0) {
 			// TLAS leaves are instances (one per leaf child): queued, the nearest on top.
 			while (leafHits) {
 				const uint32_t j = highestBit(leafHits);
 				leafHits &= ~(1u << j);
-				const uint32_t s = j ^ r.oct;
-				const uint32_t meta = ((s < 4 ? metaLo : metaHi) >> ((s & 3) * 8)) & 0xffu;
-				st.push((uint32_t) load.leafPrim(leaves, (int) triBase + (int) (meta & 31u)), kEnterInstance);
+				int first, cnt;
+				n.leaf(j ^ r.oct, first, cnt);
+				st.push(tlasLeafEntry(sc.tlasLeaves, first, load), kEnterInstance);
 			}
 		} else {
-			// BLAS leaves: their triangles now, in ray order.
-			while (leafHits) {
-				const uint32_t s = lowestBit(leafHits) ^ r.oct;
-				leafHits &= leafHits - 1u;
-				const uint32_t meta = ((s < 4 ? metaLo : metaHi) >> ((s & 3) * 8)) & 0xffu;
-				const int first = (int) triBase + (int) (meta & 31u);
-				const int cnt = (int) (meta >> 5);
-				for (int k = 0; k < cnt; ++k) {
-					TriRecord tr = load.tri(leaves, first + k);
-					float t;
-					if (intersectTriangle(v3(tr.v0x, tr.v0y, tr.v0z), v3(tr.v1x, tr.v1y, tr.v1z), v3(tr.v2x, tr.v2y, tr.v2z), r.o, wt,
-					                      best.t, t) &&
-					    closerHit(t, inst, tr.primId, best)) {
-						best.t = t;
-						best.inst = inst;
-						best.tri = first + k;
-						best.prim = tr.primId;
-					}
-				}
-			}
+			testLeaves(n, leafHits, r.oct, leaves, inst, r.o, wt, best, load);
 		}
-		uint32_t groupBase = childBase, groupMask = imask, hits = internalHits;
+		uint32_t groupBase = n.childBase(), groupMask = imask, hits = internalHits;
 		bool enterRoot = false;
 		while (hits == 0) {
 			if (st.size() == base) {
@@ -549,23 +628,23 @@ RGL_HD HitRec traceClosest(const SceneView& sc, Vec3 oW, Vec3 dW, float tmax, St
 					r = frameRay(oW, dW);
 				}
 				nodes = sc.tlas;
-				leaves = sc.tlasLeaves;
 				inst = -1;
 			} else if (b == kEnterInstance) {
-				const InstanceRec& ir = load.instance(sc.instances, (int32_t) a);
+				const EnterRec e = loadEnter(sc, a, load);
 				// An identity pose (a scene-sized mesh, most rays' last instance) maps the ray to itself
 				// exactly: the frame stays, here and on leaving.
-				const bool identity = (ir.flags & kInstanceIdentity) != 0;
+				const bool identity = (e.flags & kInstanceIdentity) != 0;
 				st.push(identity ? 1u : 0u, kLeaveInstance);
 				Vec3 od = dW;
 				if (!identity) {
-					od = ir.worldToObject.vector(dW);
-					r = frameRay(worldToInstance(ir, oW), od);
+					const Mat34 m{{{e.m[0][0], e.m[0][1], e.m[0][2], 0.0f}, {e.m[1][0], e.m[1][1], e.m[1][2], 0.0f}, {e.m[2][0], e.m[2][1], e.m[2][2], 0.0f}}};
+					od = m.vector(dW);
+					r = frameRay(m.vector(oW - v3(e.m[0][3], e.m[1][3], e.m[2][3])), od);
 				}
 				wt = setupWatertight(od);
-				nodes = ir.nodes;
-				leaves = ir.tris;
-				inst = (int32_t) a;
+				nodes = e.nodes;
+				leaves = e.tris;
+				inst = e.inst;
 				enterRoot = true;
 				break;
 			} else {

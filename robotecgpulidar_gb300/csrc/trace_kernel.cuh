@@ -19,8 +19,8 @@
 namespace rgl {
 namespace tracedev {
 
-constexpr int kSmemStack = 24;  // entries per thread in shared memory
-constexpr int kLocalStack = 40; // overflow entries per thread in local memory
+constexpr int kSmemStack = 12;  // entries per thread in shared memory
+constexpr int kLocalStack = 52; // overflow entries per thread in local memory
 
 // Traversal stack: the first kSmemStack entries in this thread's shared-memory column (stride =
 // threads per block), the rest in a local-memory array the kernel declares. Overflow past both is
@@ -94,27 +94,18 @@ struct DevLoader
 	__device__ __forceinline__ int32_t leafPrim(const TriRecord* base, int32_t i) const { return __ldg(&base[i].primId); }
 };
 
-// One traced sample. For non-hits `dist` holds the non-hit distance (near or far).
+// One traced sample: distance (for non-hits the near or far non-hit distance), the hit's instance index |
+// sample index << kSampleShift (kNoHit without a hit), and in the SHADING variants the intensity and the
+// hit's triangle record. Entity id, laser retro, normal, incident angle and velocities are read or
+// computed from these when a selected return is written.
 struct SampleVal
 {
-	uint32_t hit;
 	float dist;
-	float intensity;
-	int32_t inst; // hit: instance index | sample index << 24 (entity id, laser retro, velocity read when written)
-	float nx, ny, nz, cosInc;
-	int32_t tri;  // SHADING: the hit's triangle record (velocity of animated meshes)
-};
-
-struct Selected
-{
-	float dist;
-	float intensity;
 	int32_t inst;
-	float nx, ny, nz, cosInc;
+	float intensity;
 	int32_t tri;
 };
-
-__device__ __forceinline__ SampleVal emptySample() { return SampleVal{0u, 0.0f, 0.0f, 0, 0.0f, 0.0f, 0.0f, 0.0f, -1}; }
+constexpr int32_t kNoHit = -1;
 
 __device__ __forceinline__ Mat34 loadMat(const Mat34* p)
 {
@@ -156,39 +147,43 @@ __device__ __noinline__ float texturedIntensity(const InstanceRec& inst, const T
 	return (float) tex2D<unsigned char>((cudaTextureObject_t) inst.intensityTexture, tu, tv);
 }
 
-template<bool SHADING>
-__device__ __forceinline__ SampleVal sampleFromHit(float nearNonHit, float farNonHit, float defaultIntensity, const SceneView& sc,
-                                                   const HitRec& h, Vec3 o, Vec3 d, float minRange, int sample)
+// World normal of the hit triangle and |cos| of the incidence of ray direction d.
+__device__ __forceinline__ Vec3 hitNormal(const InstanceRec& inst, const TriRecord& tr, Vec3 d, float& cosInc)
 {
-	DevLoader ld;
-	SampleVal v = emptySample();
-	v.dist = farNonHit;
+	const Vec3 wa = inst.objectToWorld.point(v3(tr.v0x, tr.v0y, tr.v0z));
+	const Vec3 wb = inst.objectToWorld.point(v3(tr.v1x, tr.v1y, tr.v1z));
+	const Vec3 wc = inst.objectToWorld.point(v3(tr.v2x, tr.v2y, tr.v2z));
+	const Vec3 n = normalized(cross(wb - wa, wc - wa));
+	cosInc = fabsf(dot(n, d));
+	return n;
+}
+
+template<bool SHADING>
+__device__ __forceinline__ SampleVal sampleFromHit(const TraceParams& p, const SceneView& sc, const HitRec& h, Vec3 o, Vec3 d, float minRange,
+                                                   int sample)
+{
+	SampleVal v{p.farNonHitDistance, kNoHit, 0.0f, -1};
 	if (h.inst >= 0) {
 		const float dist = fmul(h.t, length(d));
 		if (dist < minRange) {
-			v.dist = nearNonHit;
+			v.dist = p.nearNonHitDistance;
 		} else {
-			const InstanceRec& inst = sc.instances[h.inst];
-			v.hit = 1;
 			v.dist = dist;
 			v.inst = h.inst | (sample << kSampleShift);
 			if (SHADING) {
-				const TriRecord tr = ld.tri(inst.tris, h.tri);
-				const Vec3 wa = inst.objectToWorld.point(v3(tr.v0x, tr.v0y, tr.v0z));
-				const Vec3 wb = inst.objectToWorld.point(v3(tr.v1x, tr.v1y, tr.v1z));
-				const Vec3 wc = inst.objectToWorld.point(v3(tr.v2x, tr.v2y, tr.v2z));
-				const Vec3 n = normalized(cross(wb - wa, wc - wa));
-				const float c = fabsf(dot(n, d));
-				v.nx = n.x;
-				v.ny = n.y;
-				v.nz = n.z;
-				v.cosInc = c;
-				float base = defaultIntensity;
-				if (inst.intensityTexture != 0) {
-					base = texturedIntensity(inst, tr, worldToInstance(inst, o + d * h.t));
-				}
-				v.intensity = fmul(base, c);
 				v.tri = h.tri;
+				if (p.needIntensity) {
+					DevLoader ld;
+					const InstanceRec& inst = sc.instances[h.inst];
+					const TriRecord tr = ld.tri(inst.tris, h.tri);
+					float c;
+					(void) hitNormal(inst, tr, d, c);
+					float base = p.defaultIntensity;
+					if (inst.intensityTexture != 0) {
+						base = texturedIntensity(inst, tr, worldToInstance(inst, o + d * h.t));
+					}
+					v.intensity = fmul(base, c);
+				}
 			}
 		}
 	}
@@ -196,18 +191,13 @@ __device__ __forceinline__ SampleVal sampleFromHit(float nearNonHit, float farNo
 }
 
 template<bool SHADING>
-__device__ __forceinline__ SampleVal traceSample(float nearNonHit, float farNonHit, float defaultIntensity, const SceneView& sc,
-                                                 const Mat34& sr, float minRange, float maxRange, DevStack& st, int sample)
+__device__ __forceinline__ SampleVal traceSample(const TraceParams& p, const SceneView& sc, const Mat34& sr, float minRange, float maxRange,
+                                                 DevStack& st, int sample)
 {
 	DevLoader ld;
 	const Vec3 d = sr.rayDir();
 	const HitRec h = traceClosest(sc, sr.rayOrigin(), d, maxRange, st, ld);
-	return sampleFromHit<SHADING>(nearNonHit, farNonHit, defaultIntensity, sc, h, sr.rayOrigin(), d, minRange, sample);
-}
-
-__device__ __forceinline__ Selected toSelected(const SampleVal& v)
-{
-	return Selected{v.dist, v.intensity, v.inst, v.nx, v.ny, v.nz, v.cosInc, v.tri};
+	return sampleFromHit<SHADING>(p, sc, h, sr.rayOrigin(), d, minRange, sample);
 }
 
 // In-order selection over a beam's samples; add() must see samples 0, 1, 2, ... in order.
@@ -215,16 +205,17 @@ struct ReturnReducer
 {
 	bool haveFirst;
 	float nonHitDist;
-	Selected first, second, last, strongest, secondStrongest;
+	SampleVal first, second, last, strongest, secondStrongest;
 
 	__device__ __forceinline__ void init(float farNonHit)
 	{
 		haveFirst = false;
 		nonHitDist = farNonHit;
-		first = second = last = strongest = secondStrongest = Selected{0.0f, 0.0f, 0, 0.0f, 0.0f, 0.0f, 0.0f, -1};
+		first = second = last = strongest = secondStrongest = SampleVal{0.0f, 0, 0.0f, -1};
 	}
-	__device__ __forceinline__ void add(int s, uint32_t hit, const Selected& cur)
+	__device__ __forceinline__ void add(int s, const SampleVal& cur)
 	{
+		const bool hit = cur.inst != kNoHit;
 		if (s == 0 && !hit) {
 			nonHitDist = cur.dist;
 		}
@@ -400,7 +391,7 @@ __device__ __forceinline__ void writeReturns(const TraceParams& p, const SceneVi
 			if (out.radialSpeed) out.radialSpeed[pi] = 0.0f;
 			continue;
 		}
-		Selected sel;
+		SampleVal sel;
 		if (type == 4u) sel = red.first;
 		else if (type == 3u) sel = red.second;
 		else if (type == 2u) sel = red.last;
@@ -420,17 +411,27 @@ __device__ __forceinline__ void writeReturns(const TraceParams& p, const SceneVi
 		if (out.returnType) out.returnType[pi] = (uint8_t) type;
 		if (out.intensityF32) out.intensityF32[pi] = sel.intensity;
 		if (out.intensityU8) out.intensityU8[pi] = sel.intensity < 255.0f ? (uint8_t) roundf(sel.intensity) : (uint8_t) 255;
-		if (out.normal) {
-			out.normal[3 * pi] = sel.nx;
-			out.normal[3 * pi + 1] = sel.ny;
-			out.normal[3 * pi + 2] = sel.nz;
-		}
-		if (out.incidentAngle) out.incidentAngle[pi] = acosf(sel.cosInc);
 		if (out.laserRetro) out.laserRetro[pi] = hitInst.laserRetro;
-		if (SHADING && (out.absVelocity || out.relVelocity || out.radialSpeed)) {
-			const int sample = sel.inst >> kSampleShift;
-			const Mat34 traced = distortRay(p, beam, ray);
-			const Mat34 sr = sample == 0 ? traced : mul(traced, loadMat(samples + sample));
+		const bool velocities = out.absVelocity || out.relVelocity || out.radialSpeed;
+		if (!SHADING || !(out.normal || out.incidentAngle || velocities)) {
+			continue;
+		}
+		// The pose the selected sample was cast from.
+		const int sample = sel.inst >> kSampleShift;
+		const Mat34 traced = distortRay(p, beam, ray);
+		const Mat34 sr = sample == 0 ? traced : mul(traced, loadMat(samples + sample));
+		if (out.normal || out.incidentAngle) {
+			DevLoader ld;
+			float c;
+			const Vec3 n = hitNormal(hitInst, ld.tri(hitInst.tris, sel.tri), sr.rayDir(), c);
+			if (out.normal) {
+				out.normal[3 * pi] = n.x;
+				out.normal[3 * pi + 1] = n.y;
+				out.normal[3 * pi + 2] = n.z;
+			}
+			if (out.incidentAngle) out.incidentAngle[pi] = acosf(c);
+		}
+		if (velocities) {
 			Vec3 absV, relV;
 			float radial;
 			hitVelocities(p, hitInst, sr, sel.dist, sel.tri, absV, relV, radial);
@@ -445,39 +446,6 @@ __device__ __forceinline__ void writeReturns(const TraceParams& p, const SceneVi
 				out.relVelocity[3 * pi + 2] = relV.z;
 			}
 			if (out.radialSpeed) out.radialSpeed[pi] = radial;
-		}
-	}
-}
-
-__device__ __forceinline__ float pick(int r, float a, float b) { return r == 0 ? a : b; }
-__device__ __forceinline__ uint32_t pickU(int r, uint32_t a, uint32_t b) { return r == 0 ? a : b; }
-
-// Lane-group packing: the S samples of a beam sit on G = min(S, 32) adjacent lanes (lane k of the
-// group holds samples k and k + G in sv[0], sv[1]); every lane of the warp takes part in the
-// shuffles, and the group's first lane (`leader`) feeds the samples in order to `red`.
-template<int ROUNDS, bool SHADING>
-__device__ __forceinline__ void reduceGroup(const SampleVal (&sv)[ROUNDS], int nSamples, int G, int groupLane0, bool leader,
-                                            ReturnReducer& red)
-{
-	for (int s = 0; s < nSamples; ++s) {
-		const int r = (ROUNDS == 1) ? 0 : s / G;
-		const int src = groupLane0 + (s - r * G);
-		const uint32_t hit = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].hit : pickU(r, sv[0].hit, sv[ROUNDS - 1].hit), src);
-		const float dist = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].dist : pick(r, sv[0].dist, sv[ROUNDS - 1].dist), src);
-		const int32_t ent = __shfl_sync(
-		    0xffffffffu, ROUNDS == 1 ? sv[0].inst : (int32_t) pickU(r, (uint32_t) sv[0].inst, (uint32_t) sv[ROUNDS - 1].inst), src);
-		Selected cur{dist, 0.0f, ent, 0.0f, 0.0f, 0.0f, 0.0f, -1};
-		if (SHADING) {
-			cur.intensity = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].intensity : pick(r, sv[0].intensity, sv[ROUNDS - 1].intensity), src);
-			cur.nx = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].nx : pick(r, sv[0].nx, sv[ROUNDS - 1].nx), src);
-			cur.ny = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].ny : pick(r, sv[0].ny, sv[ROUNDS - 1].ny), src);
-			cur.nz = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].nz : pick(r, sv[0].nz, sv[ROUNDS - 1].nz), src);
-			cur.cosInc = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].cosInc : pick(r, sv[0].cosInc, sv[ROUNDS - 1].cosInc), src);
-			cur.tri = __shfl_sync(0xffffffffu, ROUNDS == 1 ? sv[0].tri : (int32_t) pickU(r, (uint32_t) sv[0].tri, (uint32_t) sv[ROUNDS - 1].tri),
-			                      src);
-		}
-		if (leader) {
-			red.add(s, hit, cur);
 		}
 	}
 }
