@@ -168,6 +168,14 @@ class StagedParam
 public:
 	T& host() { return *static_cast<T*>(h_.ensure(sizeof(T))); }
 	const T* device() { return static_cast<const T*>(d_.ensure(sizeof(T))); }
+	// The staged block itself through the device's mapping of pinned memory, for a kernel that reads it
+	// once per block: no copy in the run. It stays where it is once host() has been called.
+	const T* mapped()
+	{
+		void* d = nullptr;
+		RGL_CHECK_CUDA(cudaHostGetDevicePointer(&d, &host(), 0));
+		return static_cast<const T*>(d);
+	}
 	const T* enqueue(cudaStream_t s)
 	{
 		if (deferredParamCopies != nullptr) {

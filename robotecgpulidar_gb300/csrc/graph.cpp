@@ -829,7 +829,7 @@ void CompactByFieldPointsNode::compact(const std::vector<rgl_field_t>& which, cu
 	}
 	if (absorbs && (ops.xyzField >= 0 || ops.distField >= 0)) {
 		for (auto& pw : chain) {
-			pw->appendPointOp(ops, s);
+			pw->appendPointOp(ops);
 		}
 		ops.srcXyz = static_cast<const float*>(chainSource->fieldDev(RGL_FIELD_XYZ_VEC3_F32));
 		ops.srcDist = chainSource->hasField(RGL_FIELD_DISTANCE_F32) ? static_cast<const float*>(chainSource->fieldDev(RGL_FIELD_DISTANCE_F32))
@@ -915,9 +915,9 @@ void TransformPointsNode::enqueueImpl(cudaStream_t s)
 	}
 }
 
-void TransformPointsNode::appendPointOp(rgl::PointOps& ops, cudaStream_t s)
+void TransformPointsNode::appendPointOp(rgl::PointOps& ops)
 {
-	ops.op[ops.count++] = rgl::PointOp{rgl::kOpTransform, 0, staged.enqueue(s)};
+	ops.op[ops.count++] = rgl::PointOp{rgl::kOpTransform, 0, staged.mapped()};
 }
 
 const void* TransformPointsNode::fieldDev(rgl_field_t f)
@@ -973,9 +973,9 @@ void GaussianNoiseAngularHitpointNode::enqueueImpl(cudaStream_t s)
 	}
 }
 
-void GaussianNoiseAngularHitpointNode::appendPointOp(rgl::PointOps& ops, cudaStream_t s)
+void GaussianNoiseAngularHitpointNode::appendPointOp(rgl::PointOps& ops)
 {
-	ops.op[ops.count++] = rgl::PointOp{rgl::kOpNoiseAngularHitpoint, withDistance ? 1 : 0, staged.enqueue(s)};
+	ops.op[ops.count++] = rgl::PointOp{rgl::kOpNoiseAngularHitpoint, withDistance ? 1 : 0, staged.mapped()};
 }
 
 const void* GaussianNoiseAngularHitpointNode::fieldDev(rgl_field_t f)
@@ -1028,9 +1028,9 @@ void GaussianNoiseDistanceNode::enqueueImpl(cudaStream_t s)
 	}
 }
 
-void GaussianNoiseDistanceNode::appendPointOp(rgl::PointOps& ops, cudaStream_t s)
+void GaussianNoiseDistanceNode::appendPointOp(rgl::PointOps& ops)
 {
-	ops.op[ops.count++] = rgl::PointOp{rgl::kOpNoiseDistance, 1, staged.enqueue(s)};
+	ops.op[ops.count++] = rgl::PointOp{rgl::kOpNoiseDistance, 1, staged.mapped()};
 }
 
 const void* GaussianNoiseDistanceNode::fieldDev(rgl_field_t f)

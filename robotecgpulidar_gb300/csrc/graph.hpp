@@ -259,7 +259,7 @@ struct PointwisePointsNode : PointsNodeSingleInput
 		absorbed = false;
 	}
 	// Stages this node's parameters on `s` and appends its operation.
-	virtual void appendPointOp(rgl::PointOps& ops, cudaStream_t s) = 0;
+	virtual void appendPointOp(rgl::PointOps& ops) = 0;
 	std::shared_ptr<PointsNode> source() const { return input; }
 	bool absorbed = false;
 
@@ -451,7 +451,7 @@ struct TransformPointsNode : PointwisePointsNode
 	}
 	const void* fieldDev(rgl_field_t f) override;
 	bool lastUpdateContentOnly() const override { return true; } // the transform is staged every run
-	void appendPointOp(rgl::PointOps& ops, cudaStream_t s) override;
+	void appendPointOp(rgl::PointOps& ops) override;
 
 protected:
 	void allocateOutputs() override;
@@ -477,7 +477,7 @@ struct GaussianNoiseAngularHitpointNode : PointwisePointsNode
 	void enqueueImpl(cudaStream_t s) override;
 	const void* fieldDev(rgl_field_t f) override;
 	bool lastUpdateContentOnly() const override { return true; } // parameters are staged every run
-	void appendPointOp(rgl::PointOps& ops, cudaStream_t s) override;
+	void appendPointOp(rgl::PointOps& ops) override;
 
 protected:
 	void allocateOutputs() override;
@@ -506,7 +506,7 @@ struct GaussianNoiseDistanceNode : PointwisePointsNode
 	void enqueueImpl(cudaStream_t s) override;
 	const void* fieldDev(rgl_field_t f) override;
 	bool lastUpdateContentOnly() const override { return true; } // parameters are staged every run
-	void appendPointOp(rgl::PointOps& ops, cudaStream_t s) override;
+	void appendPointOp(rgl::PointOps& ops) override;
 
 protected:
 	void allocateOutputs() override;

@@ -275,7 +275,7 @@ struct PointOp
 {
 	int32_t kind;
 	int32_t withDistance;
-	const void* params; // device copy, staged by the absorbed node
+	const void* params; // staged by the absorbed node: pinned host memory through the device's mapping
 };
 struct PointOps
 {

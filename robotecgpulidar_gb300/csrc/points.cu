@@ -257,10 +257,13 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 		tileShared = (int) atomicAdd(scratch, 1u);
 		lbFail = 0;
 	}
+	// The absorbed operations' parameters straight from the pinned blocks the nodes staged them in: at most
+	// 576 bytes a block, about 1 us of latency that other blocks cover. As copy nodes between the traversal
+	// and this kernel they held it up by 16 us (three operations).
 	for (int k = 0; k < ops.count; ++k) {
 		const int words = ops.op[k].kind == kOpTransform ? (int) (sizeof(Mat34) / 4) : kOpParamWords;
 		for (int w = tid; w < words; w += kBlock) {
-			opParams[k][w] = __ldg(static_cast<const uint32_t*>(ops.op[k].params) + w);
+			opParams[k][w] = __ldcv(static_cast<const uint32_t*>(ops.op[k].params) + w);
 		}
 	}
 	__syncthreads();
