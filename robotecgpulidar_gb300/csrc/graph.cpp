@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <map>
 
 #include "scene.hpp"
 
@@ -1326,6 +1327,7 @@ GraphRunCtx::GraphRunCtx()
 GraphRunCtx::~GraphRunCtx()
 {
 	releaseGraph();
+	releaseBranches();
 	cudaEventDestroy(done);
 	cudaEventDestroy(runStart);
 	cudaEventDestroy(runStop);
@@ -1386,6 +1388,106 @@ void GraphRunCtx::releaseGraph()
 	}
 }
 
+void GraphRunCtx::releaseBranches()
+{
+	for (auto& p : placements) {
+		if (p.done) {
+			cudaEventDestroy(p.done);
+		}
+	}
+	for (cudaEvent_t e : branchEvents) {
+		cudaEventDestroy(e);
+	}
+	for (cudaStream_t b : branches) {
+		cudaStreamDestroy(b);
+	}
+	placements.clear();
+	branchEvents.clear();
+	branches.clear();
+}
+
+// Graphs with several raytraces (sensors fused into one cloud) enqueue their branches side by side: a node
+// goes on after its first input when it is the first to do so, else on another stream that waits for its
+// inputs. A scan of some 30,000 rays leaves most of the chip idle for most of its time (its longest rays
+// decide), so four of them took four times as long as one. Graphs with one raytrace stay on one stream.
+void GraphRunCtx::planBranches()
+{
+	releaseBranches();
+	size_t raytraces = 0;
+	for (auto& n : order) {
+		raytraces += std::dynamic_pointer_cast<RaytraceNode>(n) ? 1 : 0;
+	}
+	if (raytraces < 2) {
+		return;
+	}
+	constexpr int kMaxBranches = 8; // beyond, branches share streams
+	std::map<Node*, size_t> at;
+	for (size_t i = 0; i < order.size(); ++i) {
+		at[order[i].get()] = i;
+	}
+	placements.resize(order.size());
+	std::vector<bool> continued(order.size(), false);
+	int next = 0;
+	for (size_t i = 0; i < order.size(); ++i) {
+		Placement& p = placements[i];
+		const auto& in = order[i]->inputs;
+		if (!in.empty() && !continued[at[in[0].get()]]) {
+			p.branch = placements[at[in[0].get()]].branch;
+			continued[at[in[0].get()]] = true;
+		} else {
+			p.branch = next++ % (kMaxBranches + 1);
+		}
+		for (auto& n : in) {
+			const size_t k = at[n.get()];
+			if (placements[k].branch != p.branch) {
+				p.waits.push_back(k);
+				if (placements[k].done == nullptr) {
+					RGL_CHECK_CUDA(cudaEventCreateWithFlags(&placements[k].done, cudaEventDisableTiming));
+				}
+			}
+		}
+	}
+	for (int b = 0; b < std::min(next, kMaxBranches + 1) - 1; ++b) {
+		cudaStream_t st = nullptr;
+		RGL_CHECK_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+		branches.push_back(st);
+	}
+	for (size_t b = 0; b <= branches.size(); ++b) {
+		cudaEvent_t e = nullptr;
+		RGL_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+		branchEvents.push_back(e);
+	}
+}
+
+void GraphRunCtx::enqueueNodes()
+{
+	if (placements.empty()) {
+		for (auto& n : order) {
+			n->enqueueImpl(stream_);
+		}
+		return;
+	}
+	RGL_CHECK_CUDA(cudaEventRecord(branchEvents.back(), stream_));
+	for (cudaStream_t b : branches) {
+		RGL_CHECK_CUDA(cudaStreamWaitEvent(b, branchEvents.back(), 0));
+	}
+	for (size_t i = 0; i < order.size(); ++i) {
+		const Placement& p = placements[i];
+		const cudaStream_t s = p.branch == 0 ? stream_ : branches[(size_t) p.branch - 1];
+		for (size_t k : p.waits) {
+			RGL_CHECK_CUDA(cudaStreamWaitEvent(s, placements[k].done, 0));
+		}
+		order[i]->enqueueImpl(s);
+		if (p.done) {
+			RGL_CHECK_CUDA(cudaEventRecord(p.done, s));
+		}
+	}
+	for (size_t b = 0; b < branches.size(); ++b) {
+		RGL_CHECK_CUDA(cudaEventRecord(branchEvents[b], branches[b]));
+		RGL_CHECK_CUDA(cudaStreamWaitEvent(stream_, branchEvents[b], 0));
+	}
+}
+
 // One run: validation and the prepare phase on the host, then the nodes' device work. The device
 // work is captured into a CUDA graph once and replayed by later runs while no node's kernel
 // parameters changed (parameter versions) and no device buffer moved (allocation epoch); otherwise it is
@@ -1396,6 +1498,7 @@ void GraphRunCtx::run()
 	if (order.empty()) {
 		order = findExecutionOrder(nodes);
 		releaseGraph();
+		planBranches();
 	}
 	uint64_t version = 0;
 	for (auto& n : order) {
@@ -1416,9 +1519,7 @@ void GraphRunCtx::run()
 		if (timed) {
 			recordEvent(runStart, stream_);
 		}
-		for (auto& n : order) {
-			n->enqueueImpl(stream_);
-		}
+		enqueueNodes();
 		if (timed) {
 			recordEvent(runStop, stream_);
 		}
@@ -1431,9 +1532,7 @@ void GraphRunCtx::run()
 				if (timed) {
 					recordEvent(runStart, stream_);
 				}
-				for (auto& n : order) {
-					n->enqueueImpl(stream_);
-				}
+				enqueueNodes();
 				if (timed) {
 					recordEvent(runStop, stream_);
 				}
@@ -1473,6 +1572,7 @@ uint64_t GraphRunCtx::validateForBatch()
 	if (order.empty()) {
 		order = findExecutionOrder(nodes);
 		releaseGraph();
+		planBranches();
 		validated = false;
 	}
 	const uint64_t epoch = graphEditEpoch();

@@ -651,6 +651,20 @@ private:
 	GraphRunCtx();
 	static std::vector<Node::Ptr> findExecutionOrder(std::set<Node::Ptr> nodes);
 	void releaseGraph();
+	// Where a node is enqueued when the graph has branches that may run at the same time: its stream, the
+	// inputs enqueued elsewhere it waits for, and its own event when a node elsewhere waits for it.
+	struct Placement
+	{
+		int branch = 0; // 0: stream_, else branches[branch - 1]
+		std::vector<size_t> waits; // positions in `order`
+		cudaEvent_t done = nullptr;
+	};
+	void planBranches();
+	void enqueueNodes();
+	std::vector<Placement> placements; // by position in `order`; empty: everything on stream_
+	std::vector<cudaStream_t> branches;
+	std::vector<cudaEvent_t> branchEvents; // one per branch (join), then the fork's
+	void releaseBranches();
 	std::vector<Node::Ptr> order;
 	cudaStream_t stream_ = nullptr;
 	cudaEvent_t done = nullptr, runStart = nullptr, runStop = nullptr;
