@@ -496,17 +496,6 @@ __global__ void __launch_bounds__(256) kRefitTlas(WideNode* nodes, const TriReco
 	}
 }
 
-// World boxes of the instances (their records' padded boxes) as the builder's primitive boxes.
-__global__ void kTlasBoxes(const InstanceRec* __restrict__ inst, int n, float4* lo, float4* hi)
-{
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) {
-		const InstanceRec& r = inst[i];
-		lo[i] = make_float4(r.lox, r.loy, r.loz, 0.0f);
-		hi[i] = make_float4(r.hix, r.hiy, r.hiz, 0.0f);
-	}
-}
-
 // Shared-memory layout of the one-block collapse over n primitives (16-byte aligned parts): primitive
 // boxes lo[n] | hi[n] | binary nodes[n - 1] | queue[n] | sorted ids[n] | ranges first[n - 1],
 // last[n - 1] | depth counters[3].
@@ -624,12 +613,11 @@ namespace {
 
 void freeSmallScratch(TlasBuild& t)
 {
-	void* ptrs[] = {t.lo, t.hi, t.sahScratch, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds};
+	void* ptrs[] = {t.lo, t.hi, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds};
 	for (void* p : ptrs) {
 		cudaFree(p);
 	}
 	t.lo = t.hi = nullptr;
-	t.sahScratch = nullptr;
 	t.bin = nullptr;
 	t.rangeFirst = t.rangeLast = nullptr;
 	t.sortedIds = nullptr;
@@ -655,11 +643,11 @@ void allocTlas(TlasBuild& t, int n)
 		freeSmallScratch(t);
 		RGL_CUDA_OK(cudaMalloc(&t.lo, sizeof(float4) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.hi, sizeof(float4) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.sahScratch, sahSmallScratchBytes(n)));
 		RGL_CUDA_OK(cudaMalloc(&t.bin, sizeof(BinNode) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.rangeFirst, sizeof(int32_t) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.rangeLast, sizeof(int32_t) * (size_t) n));
 		RGL_CUDA_OK(cudaMalloc(&t.sortedIds, sizeof(uint32_t) * (size_t) n));
+		prepareSahBlock();
 		// Shared memory of the one-block collapse, set outside any capture and for the largest scene: the limit
 		// is the kernel's, so a small scene must not lower it under a large one.
 		RGL_CUDA_OK(cudaFuncSetAttribute(kCollapseSmall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smallCollapseLayout(kSahSmallMax).bytes));
@@ -667,14 +655,12 @@ void allocTlas(TlasBuild& t, int n)
 	}
 }
 
-// The rebuild of up to kSahSmallMax instances from their device records: four launches, no host
+// The rebuild of up to kSahSmallMax instances from their device records: two launches, no host
 // interaction, so a captured frame can hold it.
 void rebuildTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 {
 	const int n = t.nInstances;
-	kTlasBoxes<<<blocks(n, 128), 128, 0, s>>>(dInst, n, t.lo, t.hi);
-	countLaunch();
-	enqueueSahTopologySmall(t.lo, t.hi, n, t.sahScratch, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds, s);
+	enqueueSahTopologySmall(dInst, t.lo, t.hi, n, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds, s);
 	const CollapseInputs ci{t.bin, t.rangeFirst, t.rangeLast, reinterpret_cast<const int32_t*>(t.sortedIds), t.lo, t.hi, nullptr, nullptr, 1};
 	kCollapseSmall<<<1, kSmallThreads, smallCollapseLayout(n).bytes, s>>>(ci, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), dInst,
 	                                                                      t.enter, t.levelStarts, t.nLevels, n);

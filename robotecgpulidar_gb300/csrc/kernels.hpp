@@ -41,12 +41,13 @@ void buildBlas(const float* dVertices, int nVertices, const int32_t* dIndices, i
 // (sah_build.hpp buildBinnedSahTree) computed on the device; output in the collapse's input format.
 void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
                             uint32_t* sortedIds, cudaStream_t stream);
-// The same topology for 1..kSahSmallMax boxes, built by one block with no host interaction (so it can
-// be captured in a CUDA graph); `scratch` holds sahSmallScratchBytes(n) bytes.
+// The same topology for the world boxes of 1..kSahSmallMax instances, built by one block with no host
+// interaction (so it can be captured in a CUDA graph, after prepareSahBlock outside it); the boxes are
+// left in lo / hi.
 constexpr int kSahSmallMax = 2048;
-size_t sahSmallScratchBytes(int n);
-void enqueueSahTopologySmall(const float4* lo, const float4* hi, int n, void* scratch, BinNode* bin, int32_t* rangeFirst,
-                             int32_t* rangeLast, uint32_t* sortedIds, cudaStream_t stream);
+void prepareSahBlock();
+void enqueueSahTopologySmall(const InstanceRec* inst, float4* lo, float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
+                             uint32_t* sortedIds, cudaStream_t s);
 // Builds the BLAS of a mesh on the host from host vertices/indices (binned SAH topology, the same wide
 // collapse) and uploads it; storage of `out` is reused when large enough.
 void buildBlasHost(const float* hVertices, int nVertices, const int32_t* hIndices, int nTris, BlasBuild& out);
@@ -68,7 +69,6 @@ struct TlasBuild
 	int32_t smallCapacity = 0;
 	float4* lo = nullptr;
 	float4* hi = nullptr;
-	void* sahScratch = nullptr;
 	BinNode* bin = nullptr;
 	int32_t* rangeFirst = nullptr;
 	int32_t* rangeLast = nullptr;

@@ -44,9 +44,9 @@ constexpr int kBins = 32;
 constexpr int kBinWords = 7;                    // lo xyz, hi xyz (ordered bits), count
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 constexpr int kBigTask = 2048;                  // larger ranges split in the level loop
-constexpr int kChunk = 2048;                    // elements per block in the level loop
+constexpr int kChunk = 512;                     // elements per block in the level loop: 256 blocks for 131,072 triangles
 constexpr int kThreads = 256;
-constexpr int kItems = kChunk / kThreads;       // 8 elements per thread
+constexpr int kItems = kChunk / kThreads;       // 2 elements per thread
 constexpr int kSmallTask = 32;                  // ranges up to this size: one warp
 constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kEmptyLo = 0xffffffffu;      // identity of min over ordered bits
@@ -63,10 +63,10 @@ struct SahSplit
 	int32_t axis, bin, nLeft, pad; // axis -1: split in the middle
 };
 
-// Control words: [0] node counter, [1] next-level task count, [2] block task count, [3] chunks of the
+// Control words: [0] node counter, [1] next-level task count, [2] block task count, [3] tasks of the
 // current level, [4] error: a partition or stack index outside its range (never expected: the counts
 // and the partition use the same bin function), the offending write is skipped.
-enum { kCtrNodes = 0, kCtrNext = 1, kCtrBlock = 2, kCtrChunks = 3, kCtrError = 4, kCtrWords = 8 };
+enum { kCtrNodes = 0, kCtrNext = 1, kCtrBlock = 2, kCtrCur = 3, kCtrError = 4, kCtrWords = 8 };
 
 __device__ __forceinline__ uint32_t ordered(float f)
 {
@@ -263,13 +263,19 @@ __global__ void kSahInit(const float4* __restrict__ lo, const float4* __restrict
 	}
 }
 
-// Chunk prefix sums of the level's ranges and their bounds cleared (one block).
-__global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int nTasks, int32_t* chunkBase, uint32_t* bounds, uint32_t* ctr)
+// The level's task count (what the level before counted), the chunk prefix sums of its ranges and their
+// bounds cleared (one block). The kernels of a level read the count from the control words, so levels
+// follow each other without the host.
+__global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int32_t* chunkBase, uint32_t* bounds, uint32_t* ctr)
 {
 	__shared__ int32_t sWarp[32];
 	__shared__ int32_t sCarry;
+	const int nTasks = (int) ctr[kCtrNext];
+	__syncthreads();
 	if (threadIdx.x == 0) {
 		sCarry = 0;
+		ctr[kCtrCur] = (uint32_t) nTasks;
+		ctr[kCtrNext] = 0u;
 	}
 	for (int i = threadIdx.x; i < nTasks * 12; i += blockDim.x) {
 		bounds[i] = isMinWord(i % 12) ? kEmptyLo : kEmptyHi;
@@ -316,15 +322,15 @@ __global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int nTasks, int
 	}
 	if (threadIdx.x == 0) {
 		chunkBase[nTasks] = sCarry;
-		ctr[kCtrChunks] = (uint32_t) sCarry;
 	}
 }
 
 // Range of chunk c: the task whose chunk prefix covers it.
-__device__ __forceinline__ bool chunkRange(const int32_t* chunkBase, int nTasks, const SahTask* tasks, int c, int& t, int& start, int& end,
-                                           int& first)
+__device__ __forceinline__ bool chunkRange(const int32_t* chunkBase, const uint32_t* ctr, const SahTask* tasks, int c, int& t, int& start,
+                                           int& end, int& first)
 {
-	if (c >= chunkBase[nTasks]) {
+	const int nTasks = (int) ctr[kCtrCur];
+	if (nTasks == 0 || c >= chunkBase[nTasks]) {
 		return false;
 	}
 	int lo = 0, hi = nTasks; // chunkBase[lo] <= c < chunkBase[hi]
@@ -368,14 +374,14 @@ __device__ __forceinline__ void blockReduceBounds(Bounds12& b, uint32_t (*sRed)[
 	}
 }
 
-__global__ void __launch_bounds__(kThreads) kSahBounds(const SahTask* __restrict__ tasks, int nTasks, const int32_t* __restrict__ chunkBase,
+__global__ void __launch_bounds__(kThreads) kSahBounds(const SahTask* __restrict__ tasks, const uint32_t* ctr, const int32_t* __restrict__ chunkBase,
                                                        const uint32_t* __restrict__ ids, const float4* __restrict__ lo,
                                                        const float4* __restrict__ hi, const float4* __restrict__ cen, uint32_t* bounds,
                                                        uint32_t* bins)
 {
 	__shared__ uint32_t sRed[kWarps][12];
 	int t, start, end, first;
-	if (!chunkRange(chunkBase, nTasks, tasks, blockIdx.x, t, start, end, first)) {
+	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
 		return;
 	}
 	if ((int) blockIdx.x == first) { // the range's first chunk clears its bins for the binning pass
@@ -394,14 +400,14 @@ __global__ void __launch_bounds__(kThreads) kSahBounds(const SahTask* __restrict
 	blockReduceBounds(b, sRed, bounds + (size_t) t * 12);
 }
 
-__global__ void __launch_bounds__(kThreads) kSahBins(const SahTask* __restrict__ tasks, int nTasks, const int32_t* __restrict__ chunkBase,
+__global__ void __launch_bounds__(kThreads) kSahBins(const SahTask* __restrict__ tasks, const uint32_t* ctr, const int32_t* __restrict__ chunkBase,
                                                      const uint32_t* __restrict__ ids, const float4* __restrict__ lo,
                                                      const float4* __restrict__ hi, const float4* __restrict__ cen,
                                                      const uint32_t* __restrict__ bounds, uint32_t* bins)
 {
 	__shared__ uint32_t sb[kTaskBinWords];
 	int t, start, end, first;
-	if (!chunkRange(chunkBase, nTasks, tasks, blockIdx.x, t, start, end, first)) {
+	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
 		return;
 	}
 	for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
@@ -452,13 +458,13 @@ __global__ void __launch_bounds__(kThreads) kSahBins(const SahTask* __restrict__
 }
 
 // One warp per range: the split, the node, its children (next level, block phase or leaves).
-__global__ void kSahSplit(const SahTask* __restrict__ tasks, int nTasks, const uint32_t* __restrict__ bounds,
+__global__ void kSahSplit(const SahTask* __restrict__ tasks, const uint32_t* __restrict__ bounds,
                           const uint32_t* __restrict__ bins, SahSplit* splits, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
                           SahTask* next, SahTask* blockTasks, uint32_t* ctr)
 {
 	const int w = (int) ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
 	const int lane = threadIdx.x & 31;
-	if (w >= nTasks) {
+	if (w >= (int) ctr[kCtrCur]) {
 		return;
 	}
 	const SahTask tk = tasks[w];
@@ -498,14 +504,14 @@ __device__ __forceinline__ bool goesLeft(uint32_t id, int pos, const SahTask& tk
 	return binOf(comp3(cen[id], s.axis), f.cmin, f.scale) < s.bin;
 }
 
-__global__ void __launch_bounds__(kThreads) kSahPartCount(const SahTask* __restrict__ tasks, int nTasks,
+__global__ void __launch_bounds__(kThreads) kSahPartCount(const SahTask* __restrict__ tasks, const uint32_t* ctr,
                                                           const int32_t* __restrict__ chunkBase, const uint32_t* __restrict__ ids,
                                                           const float4* __restrict__ cen, const uint32_t* __restrict__ bounds,
                                                           const SahSplit* __restrict__ splits, int32_t* chunkLeft)
 {
 	__shared__ int sW[kWarps];
 	int t, start, end, first;
-	if (!chunkRange(chunkBase, nTasks, tasks, blockIdx.x, t, start, end, first)) {
+	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
 		return;
 	}
 	const SahTask tk = tasks[t];
@@ -530,6 +536,7 @@ __global__ void __launch_bounds__(kThreads) kSahPartCount(const SahTask* __restr
 }
 
 // Block-wide exclusive scan of one int per thread; returns the prefix and the block total.
+template<int WARPS = kWarps>
 __device__ __forceinline__ int blockExclusiveScan(int v, int* sW, int& total)
 {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -547,7 +554,7 @@ __device__ __forceinline__ int blockExclusiveScan(int v, int* sW, int& total)
 	__syncthreads();
 	int before = 0;
 	total = 0;
-	for (int w = 0; w < kWarps; ++w) {
+	for (int w = 0; w < WARPS; ++w) {
 		const int x = sW[w];
 		before += w < warp ? x : 0;
 		total += x;
@@ -556,15 +563,15 @@ __device__ __forceinline__ int blockExclusiveScan(int v, int* sW, int& total)
 	return before + incl - v;
 }
 
-__global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __restrict__ tasks, int nTasks,
+__global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __restrict__ tasks, uint32_t* ctr,
                                                             const int32_t* __restrict__ chunkBase, const uint32_t* __restrict__ ids,
                                                             const float4* __restrict__ cen, const uint32_t* __restrict__ bounds,
                                                             const SahSplit* __restrict__ splits, const int32_t* __restrict__ chunkLeft,
-                                                            uint32_t* __restrict__ idsOut, uint32_t* __restrict__ sorted, uint32_t* ctr)
+                                                            uint32_t* __restrict__ idsOut, uint32_t* __restrict__ sorted)
 {
 	__shared__ int sW[kWarps];
 	int t, start, end, first;
-	if (!chunkRange(chunkBase, nTasks, tasks, blockIdx.x, t, start, end, first)) {
+	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
 		return;
 	}
 	const SahTask tk = tasks[t];
@@ -622,205 +629,448 @@ __global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __res
 
 // ------------------------------------------------------------------ block phase (ranges 2..kBigTask)
 
-// A range of up to 32 elements built to its leaves by one warp. Lane j holds the element at relative
-// position j of the range; `sx` is the warp's 32-int exchange area, `st` its 16-entry range stack.
-__device__ void warpBuild(int a, int cnt, int node, int base, uint32_t* sIds, const float4* __restrict__ gLo,
-                          const float4* __restrict__ gHi, const float4* __restrict__ gCen, int* sx, int4* st, BinNode* bin,
-                          int32_t* rangeFirst, int32_t* rangeLast, uint32_t* ctr)
-{
-	const int lane = threadIdx.x & 31;
-	const bool has = lane < cnt;
-	uint32_t id = has ? sIds[a + lane] : 0u;
-	float4 l = has ? gLo[id] : make_float4(0, 0, 0, 0);
-	float4 h = has ? gHi[id] : make_float4(0, 0, 0, 0);
-	float4 c = has ? gCen[id] : make_float4(0, 0, 0, 0);
-	int top = 0;
-	if (lane == 0) {
-		st[0] = make_int4(0, cnt, node, 0);
-	}
-	top = 1;
-	__syncwarp();
-	while (top > 0) {
-		const int4 tk = st[top - 1];
-		__syncwarp();
-		--top;
-		const int x = tk.x, y = tk.y, nd = tk.z;
-		const bool in = lane >= x && lane < y;
-		Bounds12 b;
-		b.clear();
-		if (in) {
-			b.add(l, h, c);
-		}
-		b.warpReduce();
-		AxisFrame fr[3];
-		int myBin[3];
-#pragma unroll
-		for (int ax = 0; ax < 3; ++ax) {
-			fr[ax] = axisFrame(b.w, ax);
-			myBin[ax] = fr[ax].valid ? binOf(comp3(c, ax), fr[ax].cmin, fr[ax].scale) : 0;
-		}
-		// Candidate split `lane` (between bins lane-1 and lane) of each axis: left = elements with a
-		// smaller bin.
-		uint32_t L[3][6], R[3][6];
-		int lc[3] = {0, 0, 0}, rc[3] = {0, 0, 0};
-#pragma unroll
-		for (int ax = 0; ax < 3; ++ax) {
-#pragma unroll
-			for (int k = 0; k < 6; ++k) {
-				L[ax][k] = R[ax][k] = k < 3 ? kEmptyLo : kEmptyHi;
-			}
-		}
-		for (int j = x; j < y; ++j) {
-			const uint32_t w0 = __shfl_sync(0xffffffffu, ordered(l.x), j), w1 = __shfl_sync(0xffffffffu, ordered(l.y), j),
-			               w2 = __shfl_sync(0xffffffffu, ordered(l.z), j), w3 = __shfl_sync(0xffffffffu, ordered(h.x), j),
-			               w4 = __shfl_sync(0xffffffffu, ordered(h.y), j), w5 = __shfl_sync(0xffffffffu, ordered(h.z), j);
-#pragma unroll
-			for (int ax = 0; ax < 3; ++ax) {
-				const int bj = __shfl_sync(0xffffffffu, myBin[ax], j);
-				const bool left = bj < lane;
-				uint32_t* D = left ? L[ax] : R[ax];
-				D[0] = min(D[0], w0);
-				D[1] = min(D[1], w1);
-				D[2] = min(D[2], w2);
-				D[3] = max(D[3], w3);
-				D[4] = max(D[4], w4);
-				D[5] = max(D[5], w5);
-				lc[ax] += left ? 1 : 0;
-				rc[ax] += left ? 0 : 1;
-			}
-		}
-		float bestCost = kInf;
-		int bestKey = 1 << 30, bestLeft = 0;
-#pragma unroll
-		for (int ax = 0; ax < 3; ++ax) {
-			if (fr[ax].valid && lane >= 1 && lc[ax] > 0 && rc[ax] > 0) {
-				const float ha = halfAreaOf(unordered(L[ax][0]), unordered(L[ax][1]), unordered(L[ax][2]), unordered(L[ax][3]),
-				                            unordered(L[ax][4]), unordered(L[ax][5]));
-				const float hb = halfAreaOf(unordered(R[ax][0]), unordered(R[ax][1]), unordered(R[ax][2]), unordered(R[ax][3]),
-				                            unordered(R[ax][4]), unordered(R[ax][5]));
-				const float cost = __fadd_rn(__fmul_rn(ha, (float) lc[ax]), __fmul_rn(hb, (float) rc[ax]));
-				if (cost < bestCost) {
-					bestCost = cost;
-					bestKey = ax * kBins + lane;
-					bestLeft = lc[ax];
-				}
-			}
-		}
-#pragma unroll
-		for (int off = 16; off >= 1; off >>= 1) {
-			const float oc = __shfl_xor_sync(0xffffffffu, bestCost, off);
-			const int ok = __shfl_xor_sync(0xffffffffu, bestKey, off);
-			const int ol = __shfl_xor_sync(0xffffffffu, bestLeft, off);
-			if (oc < bestCost || (oc == bestCost && ok < bestKey)) {
-				bestCost = oc;
-				bestKey = ok;
-				bestLeft = ol;
-			}
-		}
-		const bool mid = bestKey >= (1 << 30);
-		const int axis = mid ? -1 : bestKey / kBins, split = mid ? 0 : bestKey % kBins;
-		const int nLeft = mid ? (x + y) / 2 - x : bestLeft;
-		// stable partition of lanes [x, y)
-		const bool goLeft = in && (mid ? lane < x + nLeft : myBin[axis] < split);
-		const uint32_t ballot = __ballot_sync(0xffffffffu, goLeft);
-		const int leftRank = __popc(ballot & ((1u << lane) - 1u));
-		int dst = !in ? lane : (goLeft ? x + leftRank : x + nLeft + (lane - x - leftRank));
-		if (dst < 0 || dst >= 32) {
-			atomicExch(&ctr[kCtrError], 1u);
-			dst = lane;
-		}
-		sx[dst] = lane;
-		__syncwarp();
-		const int src = sx[lane];
-		__syncwarp();
-		id = __shfl_sync(0xffffffffu, id, src);
-		l = make_float4(__shfl_sync(0xffffffffu, l.x, src), __shfl_sync(0xffffffffu, l.y, src), __shfl_sync(0xffffffffu, l.z, src), 0.0f);
-		h = make_float4(__shfl_sync(0xffffffffu, h.x, src), __shfl_sync(0xffffffffu, h.y, src), __shfl_sync(0xffffffffu, h.z, src), 0.0f);
-		c = make_float4(__shfl_sync(0xffffffffu, c.x, src), __shfl_sync(0xffffffffu, c.y, src), __shfl_sync(0xffffffffu, c.z, src), 0.0f);
-		const int pushes = (y - (x + nLeft) >= 2 ? 1 : 0) + (nLeft >= 2 ? 1 : 0);
-		if (lane == 0) {
-			const int g0 = base + a; // global sorted position of relative position 0
-			int32_t left, right;
-			emitNode(nd, g0 + x, g0 + y, nLeft, b.w, bin, rangeFirst, rangeLast, ctr, left, right);
-			if (top + pushes > 16) {
-				atomicExch(&ctr[kCtrError], 1u);
-			} else {
-				if (y - (x + nLeft) >= 2) {
-					st[top] = make_int4(x + nLeft, y, right, 0);
-				}
-				if (nLeft >= 2) {
-					st[top + ((y - (x + nLeft) >= 2) ? 1 : 0)] = make_int4(x, x + nLeft, left, 0);
-				}
-			}
-		}
-		top = top + pushes > 16 ? top : top + pushes;
-		__syncwarp();
-	}
-	if (has) {
-		sIds[a + lane] = id;
-	}
-}
+// A block builds its range to the leaves in shared memory, its elements' boxes held there from the start:
+//  * ranges above kMidTask elements: split by the whole block, one after another (a handful);
+//  * ranges of 33..kMidTask: one warp each, all ranges of a depth side by side;
+//  * ranges up to 32: one warp each, one element per lane, all subranges of a depth at once (smallBuild).
+// What bounds a block is the chain of splits below each other, so what matters is that splits which do
+// not depend on each other run together. With every range above 32 split by the whole block in turn and
+// every subrange of a small one split alone, the 131,072-triangle mesh took 885 us here, 94 instances 58.
+constexpr int kBlockThreads = 512;
+constexpr int kBlockWarps = kBlockThreads / 32;
+constexpr int kMidTask = 256;
 
 struct BlockShared
 {
-	uint32_t ids[kBigTask];
-	uint32_t tmp[kBigTask];
-	uint32_t bins[kTaskBinWords];
-	uint32_t red[kWarps][12];
+	float box[6][kBigTask];                        // by local element: lo xyz, hi xyz
+	uint32_t gid[kBigTask];                        // by local element: primitive
+	uint16_t ids[kBigTask], tmp[kBigTask];         // local elements in sorted order
+	uint32_t bins[kBlockWarps][kTaskBinWords];     // per warp; the first also for whole-block splits
+	int4 stack[16];                                // ranges above kMidTask: disjoint, at most kBigTask / 257
+	int4 mid[2][kBigTask / (kSmallTask + 1) + 1];  // ranges of 33..kMidTask of this depth and the next
+	int4 small[kBigTask / 2];                      // ranges of 2..32
+	uint32_t red[kBlockWarps][12];
 	uint32_t bounds[12];
-	int scan[kWarps];
-	int4 stack[64];          // pending ranges above kSmallTask: disjoint, so at most kBigTask / 33
-	int4 small[kBigTask / 2]; // ranges of 2..kSmallTask elements, built by warps at the end
-	int4 warpStack[kWarps][16];
-	int warpX[kWarps][32];
-	int top, nSmall;
-	int have; // the range popped for this iteration exists (written by thread 0, read by all)
+	int scan[kBlockWarps];
+	uint8_t perm[kBlockWarps][32];
+	int top, nMid[2], nSmall;
+	uint32_t nextNode;
 	int4 cur;
 	SahSplit split;
+
+	__device__ __forceinline__ void add(Bounds12& b, int e) const
+	{
+		const float4 l = make_float4(box[0][e], box[1][e], box[2][e], 0.0f), h = make_float4(box[3][e], box[4][e], box[5][e], 0.0f);
+		b.add(l, h, make_float4(centroid(e, 0), centroid(e, 1), centroid(e, 2), 0.0f));
+	}
+	// The host's centroid expression.
+	__device__ __forceinline__ float centroid(int e, int a) const { return __fmul_rn(0.5f, __fadd_rn(box[a][e], box[3 + a][e])); }
+	__device__ __forceinline__ void bin(uint32_t* to, int e, const AxisFrame (&fr)[3]) const
+	{
+#pragma unroll
+		for (int a = 0; a < 3; ++a) {
+			if (!fr[a].valid) {
+				continue;
+			}
+			uint32_t* bb = to + (a * kBins + binOf(centroid(e, a), fr[a].cmin, fr[a].scale)) * kBinWords;
+			atomicMin(&bb[0], ordered(box[0][e]));
+			atomicMin(&bb[1], ordered(box[1][e]));
+			atomicMin(&bb[2], ordered(box[2][e]));
+			atomicMax(&bb[3], ordered(box[3][e]));
+			atomicMax(&bb[4], ordered(box[4][e]));
+			atomicMax(&bb[5], ordered(box[5][e]));
+			atomicAdd(&bb[6], 1u);
+		}
+	}
+	__device__ __forceinline__ bool left(int e, int pos, int first, const SahSplit& s, const AxisFrame& f) const
+	{
+		return s.axis < 0 ? pos < first + s.nLeft : binOf(centroid(e, s.axis), f.cmin, f.scale) < s.bin;
+	}
 };
 
-__global__ void __launch_bounds__(kThreads) kSahBlock(const SahTask* __restrict__ tasks, const float4* __restrict__ gLo,
-                                                      const float4* __restrict__ gHi, const float4* __restrict__ gCen,
-                                                      uint32_t* __restrict__ sorted, BinNode* bin, int32_t* rangeFirst,
-                                                      int32_t* rangeLast, uint32_t* ctr)
+// Where a block's nodes go.
+struct NodeSink
 {
-	__shared__ BlockShared S;
-	const SahTask task = tasks[blockIdx.x];
+	BinNode* bin;
+	int32_t* rangeFirst;
+	int32_t* rangeLast;
+	uint32_t* ctr; // control words, or null (a one-block build: no other block, nobody reads the error word)
+	__device__ __forceinline__ void error() const
+	{
+		if (ctr != nullptr) {
+			atomicExch(&ctr[kCtrError], 1u);
+		}
+	}
+	__device__ __forceinline__ void write(int node, int lo, int hi, const uint32_t* b12, int32_t left, int32_t right) const
+	{
+		float4* p = reinterpret_cast<float4*>(bin + node);
+		p[0] = make_float4(unordered(b12[0]), unordered(b12[1]), unordered(b12[2]), __int_as_float(left));
+		p[1] = make_float4(unordered(b12[3]), unordered(b12[4]), unordered(b12[5]), __int_as_float(right));
+		rangeFirst[node] = lo;
+		rangeLast[node] = hi - 1;
+	}
+};
+
+__device__ __forceinline__ void clearBins(uint32_t* bins, int first, int step)
+{
+	for (int k = first; k < kTaskBinWords; k += step) {
+		const int w = k % kBinWords;
+		bins[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
+	}
+}
+
+// One thread: the node of range [a, b) split after nLeft elements, and its children queued by size.
+// Positions are the block's; `base` is the block's first sorted position.
+__device__ __forceinline__ void emitRange(BlockShared& S, int a, int b, int node, int nLeft, const uint32_t* b12, int base, int midList,
+                                          const NodeSink& out)
+{
+	const int cut[3] = {a, a + nLeft, b};
+	int32_t child[2];
+#pragma unroll
+	for (int q = 0; q < 2; ++q) {
+		child[q] = cut[q + 1] - cut[q] == 1 ? ~(base + cut[q]) : (int32_t) atomicAdd(&S.nextNode, 1u);
+	}
+	out.write(node, base + a, base + b, b12, child[0], child[1]);
+#pragma unroll
+	for (int q = 0; q < 2; ++q) {
+		const int n = cut[q + 1] - cut[q];
+		const int4 r = make_int4(cut[q], cut[q + 1], child[q], 0);
+		if (n > kMidTask) {
+			if (S.top < 16) { // whole-block splits only: no other thread pushes
+				S.stack[S.top++] = r;
+			} else {
+				out.error();
+			}
+		} else if (n > kSmallTask) {
+			const int k = atomicAdd(&S.nMid[midList], 1);
+			if (k <= kBigTask / (kSmallTask + 1)) {
+				S.mid[midList][k] = r;
+			} else {
+				out.error();
+			}
+		} else if (n >= 2) {
+			const int k = atomicAdd(&S.nSmall, 1);
+			if (k < kBigTask / 2) {
+				S.small[k] = r;
+			} else {
+				out.error();
+			}
+		}
+	}
+}
+
+// A range of 33..kMidTask elements split by one warp.
+__device__ void warpSplit(BlockShared& S, const int4 range, int base, int midList, const NodeSink& out)
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int a = range.x, b = range.y;
+	uint32_t* bins = S.bins[warp];
+	Bounds12 bd;
+	bd.clear();
+	for (int i = a + lane; i < b; i += 32) {
+		S.add(bd, S.ids[i]);
+	}
+	bd.warpReduce();
+	clearBins(bins, lane, 32);
+	AxisFrame fr[3];
+#pragma unroll
+	for (int ax = 0; ax < 3; ++ax) {
+		fr[ax] = axisFrame(bd.w, ax);
+	}
+	__syncwarp();
+	for (int i = a + lane; i < b; i += 32) {
+		S.bin(bins, S.ids[i], fr);
+	}
+	__syncwarp();
+	SahSplit s = warpBestSplit(bins, bd.w, lane);
+	if (s.axis < 0) {
+		s.nLeft = (a + b) / 2 - a;
+	}
+	const AxisFrame f = s.axis >= 0 ? (s.axis == 0 ? fr[0] : (s.axis == 1 ? fr[1] : fr[2])) : AxisFrame{0.0f, 0.0f, false};
+	// stable partition, 32 elements at a time
+	int before = 0; // left elements of the earlier ones
+	for (int i0 = a; i0 < b; i0 += 32) {
+		const int i = i0 + lane;
+		const uint16_t e = i < b ? S.ids[i] : (uint16_t) 0;
+		const bool l = i < b && S.left(e, i, a, s, f);
+		const uint32_t m = __ballot_sync(0xffffffffu, l);
+		const int rank = before + __popc(m & ((1u << lane) - 1u));
+		const int dst = l ? a + rank : a + s.nLeft + (i - a - rank);
+		if (i < b) {
+			if (dst >= a && dst < b) {
+				S.tmp[dst] = e;
+			} else {
+				out.error();
+			}
+		}
+		before += __popc(m);
+	}
+	__syncwarp();
+	for (int i = a + lane; i < b; i += 32) {
+		S.ids[i] = S.tmp[i];
+	}
+	if (lane == 0) {
+		emitRange(S, a, b, range.z, s.nLeft, bd.w, base, midList, out);
+	}
+	__syncwarp();
+}
+
+// A range of 2..32 elements built to its leaves by one warp: lane j holds the element at position j, and
+// all subranges of a depth are split together. Every lane takes its own element's bin as the last one left
+// of a split (the splits between two neighbouring elements' bins are the same split; the host takes the
+// first, after the left one's bin) and gathers both sides' boxes from its subrange, element by element,
+// along each axis; the best of the subrange's candidates, in the host's order, is its split.
+__device__ void smallBuild(BlockShared& S, const int4 range, int base, const NodeSink& out)
+{
+	constexpr uint32_t kAll = 0xffffffffu;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int a = range.x, cnt = range.y - range.x;
+	const bool has = lane < cnt;
+	int e = has ? S.ids[a + lane] : 0;
+	uint32_t w[6]; // box, ordered bits
+	float c[3];
+#pragma unroll
+	for (int k = 0; k < 6; ++k) {
+		w[k] = has ? ordered(S.box[k][e]) : 0u;
+	}
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		c[k] = has ? S.centroid(e, k) : 0.0f;
+	}
+	int x = 0, y = has ? cnt : 0, node = range.z; // this lane's subrange and its node
+	for (;;) {
+		const int len = y - x;
+		const bool active = has && len >= 2;
+		const int longest = __reduce_max_sync(kAll, active ? len : 0);
+		if (longest == 0) {
+			break;
+		}
+		// Bounds of the subrange: every lane goes once around it.
+		uint32_t b12[12];
+#pragma unroll
+		for (int k = 0; k < 6; ++k) {
+			b12[k] = w[k];
+		}
+#pragma unroll
+		for (int k = 0; k < 3; ++k) {
+			b12[6 + k] = b12[9 + k] = ordered(c[k]);
+		}
+		int j = lane;
+		for (int k = 1; k < longest; ++k) {
+			j = j + 1 < y ? j + 1 : x;
+			const int src = active ? j : lane; // once around: further turns meet the same elements again
+#pragma unroll
+			for (int q = 0; q < 6; ++q) {
+				const uint32_t v = __shfl_sync(kAll, w[q], src);
+				b12[q] = q < 3 ? min(b12[q], v) : max(b12[q], v);
+			}
+#pragma unroll
+			for (int q = 0; q < 3; ++q) {
+				const uint32_t v = ordered(__shfl_sync(kAll, c[q], src));
+				b12[6 + q] = min(b12[6 + q], v);
+				b12[9 + q] = max(b12[9 + q], v);
+			}
+		}
+		uint32_t myBin[3], packed = 0;
+		bool valid[3];
+#pragma unroll
+		for (int ax = 0; ax < 3; ++ax) {
+			const AxisFrame f = axisFrame(b12, ax);
+			valid[ax] = f.valid;
+			myBin[ax] = f.valid ? (uint32_t) binOf(c[ax], f.cmin, f.scale) : 0u;
+			packed |= myBin[ax] << (8 * ax);
+		}
+		// Both sides of this lane's candidate on each axis.
+		uint32_t L[3][6], R[3][6];
+		int lc[3] = {1, 1, 1};
+#pragma unroll
+		for (int ax = 0; ax < 3; ++ax) {
+#pragma unroll
+			for (int q = 0; q < 6; ++q) {
+				L[ax][q] = w[q];
+				R[ax][q] = q < 3 ? kEmptyLo : kEmptyHi;
+			}
+		}
+		j = lane;
+		for (int k = 1; k < longest; ++k) {
+			j = j + 1 < y ? j + 1 : x;
+			const int src = active ? j : lane;
+			const bool counts = k < len;
+			const uint32_t theirs = __shfl_sync(kAll, packed, src);
+			uint32_t v[6];
+#pragma unroll
+			for (int q = 0; q < 6; ++q) {
+				v[q] = __shfl_sync(kAll, w[q], src);
+			}
+#pragma unroll
+			for (int ax = 0; ax < 3; ++ax) {
+				const bool l = ((theirs >> (8 * ax)) & 0xffu) <= myBin[ax];
+				lc[ax] += l && counts ? 1 : 0;
+#pragma unroll
+				for (int q = 0; q < 6; ++q) {
+					const uint32_t empty = q < 3 ? kEmptyLo : kEmptyHi;
+					const uint32_t vl = l ? v[q] : empty, vr = l ? empty : v[q];
+					L[ax][q] = q < 3 ? min(L[ax][q], vl) : max(L[ax][q], vl);
+					R[ax][q] = q < 3 ? min(R[ax][q], vr) : max(R[ax][q], vr);
+				}
+			}
+		}
+		// The lane's best candidate as (cost bits, axis and bin, left count): costs are not negative, so their
+		// bits are ordered, and among equal costs the first (axis, bin) is the smaller word.
+		float bestCost = kInf;
+		uint32_t bestKey = 0xffffffffu;
+#pragma unroll
+		for (int ax = 0; ax < 3; ++ax) {
+			const int rc = len - lc[ax];
+			if (active && valid[ax] && rc > 0) {
+				const float ha = halfAreaOf(unordered(L[ax][0]), unordered(L[ax][1]), unordered(L[ax][2]), unordered(L[ax][3]), unordered(L[ax][4]),
+				                            unordered(L[ax][5]));
+				const float hb = halfAreaOf(unordered(R[ax][0]), unordered(R[ax][1]), unordered(R[ax][2]), unordered(R[ax][3]), unordered(R[ax][4]),
+				                            unordered(R[ax][5]));
+				const float cost = __fadd_rn(__fmul_rn(ha, (float) lc[ax]), __fmul_rn(hb, (float) rc));
+				if (cost < bestCost) {
+					bestCost = cost;
+					bestKey = ((uint32_t) (ax * kBins) + myBin[ax] + 1u) << 8 | (uint32_t) lc[ax];
+				}
+			}
+		}
+		__syncwarp();
+		// The best of the subrange.
+		const float mineCost = bestCost;
+		const uint32_t mineKey = bestKey;
+		j = lane;
+		for (int k = 1; k < longest; ++k) {
+			j = j + 1 < y ? j + 1 : x;
+			const int src = active ? j : lane;
+			const float oc = __shfl_sync(kAll, mineCost, src);
+			const uint32_t ok = __shfl_sync(kAll, mineKey, src);
+			if (oc < bestCost || (oc == bestCost && ok < bestKey)) {
+				bestCost = oc;
+				bestKey = ok;
+			}
+		}
+		const bool middle = bestKey == 0xffffffffu;
+		const int nLeft = middle ? len / 2 : (int) (bestKey & 0xffu);
+		const uint32_t key = bestKey >> 8;
+		const uint32_t axis = key / kBins, cut = key % kBins; // a cut after bin 31 has no right side
+		const uint32_t mine = axis == 0u ? myBin[0] : (axis == 1u ? myBin[1] : myBin[2]);
+		const bool goLeft = active && (middle ? lane < x + nLeft : mine < cut);
+		// stable partition within the subrange
+		const uint32_t below = (1u << lane) - 1u, fromX = ~((1u << x) - 1u);
+		const int leftRank = __popc(__ballot_sync(kAll, goLeft) & below & fromX);
+		int dst = !active ? lane : (goLeft ? x + leftRank : x + nLeft + (lane - x - leftRank));
+		if (dst < 0 || dst >= 32) {
+			out.error();
+			dst = lane;
+		}
+		S.perm[warp][dst] = (uint8_t) lane;
+		// Nodes: each subrange's first lane writes it and takes numbers for its inner children.
+		const bool leads = active && lane == x;
+		int32_t child[2] = {~(base + a + x), ~(base + a + x + nLeft)};
+		const uint32_t wantL = __ballot_sync(kAll, leads && nLeft > 1), wantR = __ballot_sync(kAll, leads && len - nLeft > 1);
+		uint32_t first = 0;
+		if (lane == 0 && (wantL | wantR) != 0u) {
+			first = atomicAdd(&S.nextNode, (uint32_t) (__popc(wantL) + __popc(wantR)));
+		}
+		first = __shfl_sync(kAll, first, 0);
+		if (leads) {
+			if (nLeft > 1) {
+				child[0] = (int32_t) (first + (uint32_t) __popc(wantL & below));
+			}
+			if (len - nLeft > 1) {
+				child[1] = (int32_t) (first + (uint32_t) __popc(wantL) + (uint32_t) __popc(wantR & below));
+			}
+			out.write(node, base + a + x, base + a + y, b12, child[0], child[1]);
+		}
+		__syncwarp();
+		const int32_t cl = __shfl_sync(kAll, child[0], x), cr = __shfl_sync(kAll, child[1], x);
+		const int src = S.perm[warp][lane];
+		__syncwarp();
+		e = __shfl_sync(kAll, e, src);
+#pragma unroll
+		for (int q = 0; q < 6; ++q) {
+			w[q] = __shfl_sync(kAll, w[q], src);
+		}
+#pragma unroll
+		for (int q = 0; q < 3; ++q) {
+			c[q] = __shfl_sync(kAll, c[q], src);
+		}
+		if (active) {
+			const int mid = x + nLeft;
+			node = lane < mid ? cl : cr;
+			(lane < mid ? y : x) = mid;
+		}
+	}
+	if (has) {
+		S.ids[a + lane] = (uint16_t) e;
+	}
+	__syncwarp();
+}
+
+// tasks: one range per block, or null for a one-block build of primitives [0, n) in the given order. Boxes
+// come from gLo / gHi, or, for a TLAS, from the instance records, and are then stored there for the collapse.
+__global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __restrict__ tasks, int n, const InstanceRec* __restrict__ inst,
+                                                           float4* gLo, float4* gHi, uint32_t* __restrict__ sorted, NodeSink out)
+{
+	extern __shared__ __align__(16) uint8_t smem[];
+	BlockShared& S = *reinterpret_cast<BlockShared*>(smem);
+	const SahTask task = tasks != nullptr ? tasks[blockIdx.x] : SahTask{0, n, 0, 0};
 	const int base = task.lo, cnt = task.hi - task.lo;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-		S.ids[i] = sorted[base + i];
+		const uint32_t id = tasks != nullptr ? sorted[base + i] : (uint32_t) i;
+		float4 l, h;
+		if (inst != nullptr) {
+			const InstanceRec& r = inst[id];
+			l = make_float4(r.lox, r.loy, r.loz, 0.0f);
+			h = make_float4(r.hix, r.hiy, r.hiz, 0.0f);
+			gLo[id] = l;
+			gHi[id] = h;
+		} else {
+			l = gLo[id];
+			h = gHi[id];
+		}
+		S.gid[i] = id;
+		S.ids[i] = (uint16_t) i;
+		S.box[0][i] = l.x;
+		S.box[1][i] = l.y;
+		S.box[2][i] = l.z;
+		S.box[3][i] = h.x;
+		S.box[4][i] = h.y;
+		S.box[5][i] = h.z;
 	}
 	if (threadIdx.x == 0) {
-		S.top = 0;
-		S.nSmall = 0;
-		if (cnt > kSmallTask) {
-			S.stack[S.top++] = make_int4(0, cnt, task.node, 0);
-		} else {
-			S.small[S.nSmall++] = make_int4(0, cnt, task.node, 0);
+		S.top = S.nMid[0] = S.nMid[1] = S.nSmall = 0;
+		// A range of cnt primitives has cnt - 1 nodes: its own, and the rest numbered from here.
+		S.nextNode = out.ctr != nullptr ? atomicAdd(&out.ctr[kCtrNodes], (uint32_t) (cnt - 2)) : 1u;
+		const int4 r = make_int4(0, cnt, task.node, 0);
+		if (cnt > kMidTask) {
+			S.stack[S.top++] = r;
+		} else if (cnt > kSmallTask) {
+			S.mid[0][S.nMid[0]++] = r;
+		} else if (cnt >= 2) {
+			S.small[S.nSmall++] = r;
 		}
 	}
 	__syncthreads();
 	for (;;) {
-		// Thread 0 pops; every thread decides from the same popped flag after the barrier, which thread 0
-		// rewrites only after the body's barriers (a loop test on S.top itself would race with the pop).
-		if (threadIdx.x == 0) {
-			S.have = S.top > 0 ? 1 : 0;
-			if (S.have) {
-				S.cur = S.stack[--S.top];
-			}
-		}
+		// Every thread reads the stack's top between two barriers, so none sees the pop or the pushes of
+		// this turn.
+		const int top = S.top;
+		const int4 cur = S.stack[top > 0 ? top - 1 : 0];
 		__syncthreads();
-		if (!S.have) {
+		if (top == 0) {
 			break;
 		}
-		const int a = S.cur.x, b = S.cur.y, node = S.cur.z;
+		const int a = cur.x, b = cur.y, node = cur.z;
+		if (threadIdx.x == 0) {
+			S.top = top - 1;
+		}
 		// bounds
 		Bounds12 bd;
 		bd.clear();
 		for (int i = a + (int) threadIdx.x; i < b; i += blockDim.x) {
-			const uint32_t id = S.ids[i];
-			bd.add(gLo[id], gHi[id], gCen[id]);
+			S.add(bd, S.ids[i]);
 		}
 		bd.warpReduce();
 		if (lane == 0) {
@@ -829,15 +1079,12 @@ __global__ void __launch_bounds__(kThreads) kSahBlock(const SahTask* __restrict_
 				S.red[warp][k] = bd.w[k];
 			}
 		}
-		for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
-			const int w = k % kBinWords;
-			S.bins[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
-		}
+		clearBins(S.bins[0], (int) threadIdx.x, kBlockThreads);
 		__syncthreads();
 		if (threadIdx.x < 12) {
 			const int k = threadIdx.x;
 			uint32_t v = S.red[0][k];
-			for (int w = 1; w < kWarps; ++w) {
+			for (int w = 1; w < kBlockWarps; ++w) {
 				v = isMinWord(k) ? min(v, S.red[w][k]) : max(v, S.red[w][k]);
 			}
 			S.bounds[k] = v;
@@ -850,26 +1097,11 @@ __global__ void __launch_bounds__(kThreads) kSahBlock(const SahTask* __restrict_
 			fr[ax] = axisFrame(S.bounds, ax);
 		}
 		for (int i = a + (int) threadIdx.x; i < b; i += blockDim.x) {
-			const uint32_t id = S.ids[i];
-			const float4 l = gLo[id], h = gHi[id], c = gCen[id];
-#pragma unroll
-			for (int ax = 0; ax < 3; ++ax) {
-				if (!fr[ax].valid) {
-					continue;
-				}
-				uint32_t* bb = S.bins + (ax * kBins + binOf(comp3(c, ax), fr[ax].cmin, fr[ax].scale)) * kBinWords;
-				atomicMin(&bb[0], ordered(l.x));
-				atomicMin(&bb[1], ordered(l.y));
-				atomicMin(&bb[2], ordered(l.z));
-				atomicMax(&bb[3], ordered(h.x));
-				atomicMax(&bb[4], ordered(h.y));
-				atomicMax(&bb[5], ordered(h.z));
-				atomicAdd(&bb[6], 1u);
-			}
+			S.bin(S.bins[0], S.ids[i], fr);
 		}
 		__syncthreads();
 		if (warp == 0) {
-			SahSplit s = warpBestSplit(S.bins, S.bounds, lane);
+			SahSplit s = warpBestSplit(S.bins[0], S.bounds, lane);
 			if (s.axis < 0) {
 				s.nLeft = (a + b) / 2 - a;
 			}
@@ -880,60 +1112,58 @@ __global__ void __launch_bounds__(kThreads) kSahBlock(const SahTask* __restrict_
 		__syncthreads();
 		const SahSplit s = S.split;
 		// stable partition of [a, b): runs of consecutive elements per thread
-		const int len = b - a;
-		const int per = (len + kThreads - 1) / kThreads;
+		const int per = (b - a + kBlockThreads - 1) / kBlockThreads;
 		const int p0 = a + (int) threadIdx.x * per;
 		const int p1 = min(b, p0 + per);
-		const AxisFrame f = s.axis >= 0 ? fr[s.axis] : AxisFrame{0.0f, 0.0f, false};
+		const AxisFrame f = s.axis >= 0 ? (s.axis == 0 ? fr[0] : (s.axis == 1 ? fr[1] : fr[2])) : AxisFrame{0.0f, 0.0f, false};
 		int mine = 0;
 		for (int p = p0; p < p1; ++p) {
-			const bool gl = s.axis < 0 ? p < a + s.nLeft : binOf(comp3(gCen[S.ids[p]], s.axis), f.cmin, f.scale) < s.bin;
-			mine += gl ? 1 : 0;
+			mine += S.left(S.ids[p], p, a, s, f) ? 1 : 0;
 		}
 		int total;
-		int rank = blockExclusiveScan(mine, S.scan, total);
+		int rank = blockExclusiveScan<kBlockWarps>(mine, S.scan, total);
 		for (int p = p0; p < p1; ++p) {
-			const uint32_t id = S.ids[p];
-			const bool gl = s.axis < 0 ? p < a + s.nLeft : binOf(comp3(gCen[id], s.axis), f.cmin, f.scale) < s.bin;
+			const uint16_t e = S.ids[p];
+			const bool gl = S.left(e, p, a, s, f);
 			const int dst = gl ? a + rank : a + s.nLeft + (p - a - rank);
 			rank += gl ? 1 : 0;
 			if (dst < a || dst >= b) {
-				atomicExch(&ctr[kCtrError], 1u);
+				out.error();
 				continue;
 			}
-			S.tmp[dst] = id;
+			S.tmp[dst] = e;
 		}
 		__syncthreads();
 		for (int i = a + (int) threadIdx.x; i < b; i += blockDim.x) {
 			S.ids[i] = S.tmp[i];
 		}
 		if (threadIdx.x == 0) {
-			int32_t left, right;
-			emitNode(node, base + a, base + b, s.nLeft, S.bounds, bin, rangeFirst, rangeLast, ctr, left, right);
-			const int mid = a + s.nLeft;
-			const int r0[2] = {a, mid}, r1[2] = {mid, b};
-			const int cl[2] = {left, right};
-			for (int q = 0; q < 2; ++q) {
-				const int n = r1[q] - r0[q];
-				if (n > kSmallTask && S.top < 64) {
-					S.stack[S.top++] = make_int4(r0[q], r1[q], cl[q], 0);
-				} else if (n >= 2 && n <= kSmallTask && S.nSmall < kBigTask / 2) {
-					S.small[S.nSmall++] = make_int4(r0[q], r1[q], cl[q], 0);
-				} else if (n >= 2) {
-					atomicExch(&ctr[kCtrError], 1u);
-				}
-			}
+			emitRange(S, a, b, node, s.nLeft, S.bounds, base, 0, out);
 		}
 		__syncthreads();
 	}
-	// ranges of up to 32 elements, one warp each
-	for (int k = warp; k < S.nSmall; k += kWarps) {
-		const int4 t = S.small[k];
-		warpBuild(t.x, t.y - t.x, t.z, base, S.ids, gLo, gHi, gCen, S.warpX[warp], S.warpStack[warp], bin, rangeFirst, rangeLast, ctr);
+	// ranges of 33..kMidTask, depth by depth
+	for (int list = 0;; list ^= 1) {
+		const int m = min(S.nMid[list], kBigTask / (kSmallTask + 1) + 1);
+		if (m == 0) {
+			break;
+		}
+		for (int k = warp; k < m; k += kBlockWarps) {
+			warpSplit(S, S.mid[list][k], base, list ^ 1, out);
+		}
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			S.nMid[list] = 0; // this list takes the depth after next
+		}
+		__syncthreads();
+	}
+	// ranges of up to 32 elements
+	for (int k = warp; k < min(S.nSmall, kBigTask / 2); k += kBlockWarps) {
+		smallBuild(S, S.small[k], base, out);
 	}
 	__syncthreads();
 	for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-		sorted[base + i] = S.ids[i];
+		sorted[base + i] = S.gid[S.ids[i]];
 	}
 }
 
@@ -948,6 +1178,15 @@ T* sahAlloc(size_t count, cudaStream_t s)
 }
 
 } // namespace
+
+void prepareSahBlock()
+{
+	static const bool done = [] {
+		RGL_SAH_OK(cudaFuncSetAttribute(kSahBlock, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(BlockShared)));
+		return true;
+	}();
+	(void) done;
+}
 
 void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
                             uint32_t* sortedIds, cudaStream_t s)
@@ -983,10 +1222,9 @@ void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* 
 
 	uint32_t init[kCtrWords] = {1u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 	const SahTask root{0, n, 0, 0};
-	int nCur = 0;
 	if (n > kBigTask) {
 		RGL_SAH_OK(cudaMemcpyAsync(cur, &root, sizeof(root), cudaMemcpyHostToDevice, s));
-		nCur = 1;
+		init[kCtrNext] = 1u;
 	} else {
 		RGL_SAH_OK(cudaMemcpyAsync(blockTasks, &root, sizeof(root), cudaMemcpyHostToDevice, s));
 		init[kCtrBlock] = 1u;
@@ -994,28 +1232,38 @@ void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* 
 	RGL_SAH_OK(cudaMemcpyAsync(ctr, init, sizeof(init), cudaMemcpyHostToDevice, s));
 	uint32_t* idsCur = idsA;
 	uint32_t* idsNext = idsB;
-	while (nCur > 0) {
-		kSahLevelPrep<<<1, 1024, 0, s>>>(cur, nCur, chunkBase, bounds, ctr);
-		const int grid = n / kChunk + nCur + 1; // bound on the level's chunks; blocks past them return
-		kSahBounds<<<grid, kThreads, 0, s>>>(cur, nCur, chunkBase, idsCur, lo, hi, cen, bounds, bins);
-		kSahBins<<<grid, kThreads, 0, s>>>(cur, nCur, chunkBase, idsCur, lo, hi, cen, bounds, bins);
-		RGL_SAH_OK(cudaMemsetAsync(ctr + kCtrNext, 0, sizeof(uint32_t), s));
-		kSahSplit<<<blocksFor(nCur * 32, 128), 128, 0, s>>>(cur, nCur, bounds, bins, splits, bin, rangeFirst, rangeLast, nxt, blockTasks,
-		                                                   ctr);
-		kSahPartCount<<<grid, kThreads, 0, s>>>(cur, nCur, chunkBase, idsCur, cen, bounds, splits, chunkLeft);
-		kSahPartScatter<<<grid, kThreads, 0, s>>>(cur, nCur, chunkBase, idsCur, cen, bounds, splits, chunkLeft, idsNext, sortedIds, ctr);
-		countLaunch(6);
+	// Levels run without the host: as many as an even tree takes and two more, then a look at what is left
+	// (a level with nothing left costs six empty launches, about 12 us; a look costs about 20).
+	int levels = 0;
+	while (n > kBigTask && (kBigTask << levels) < n) {
+		++levels;
+	}
+	levels += levels > 0 ? 2 : 0;
+	const int grid = n / kChunk + maxBig + 1; // bound on a level's chunks; blocks past them return
+	for (;;) {
+		for (int l = 0; l < levels; ++l) {
+			kSahLevelPrep<<<1, 1024, 0, s>>>(cur, chunkBase, bounds, ctr);
+			kSahBounds<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, lo, hi, cen, bounds, bins);
+			kSahBins<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, lo, hi, cen, bounds, bins);
+			kSahSplit<<<blocksFor(maxBig * 32, 128), 128, 0, s>>>(cur, bounds, bins, splits, bin, rangeFirst, rangeLast, nxt, blockTasks, ctr);
+			kSahPartCount<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, cen, bounds, splits, chunkLeft);
+			kSahPartScatter<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, cen, bounds, splits, chunkLeft, idsNext, sortedIds);
+			countLaunch(6);
+			std::swap(cur, nxt);
+			std::swap(idsCur, idsNext);
+		}
 		RGL_SAH_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
 		RGL_SAH_OK(cudaStreamSynchronize(s));
-		nCur = (int) hostCtr[kCtrNext];
-		std::swap(cur, nxt);
-		std::swap(idsCur, idsNext);
+		if (hostCtr[kCtrNext] == 0u) {
+			break;
+		}
+		levels = 4;
 	}
-	RGL_SAH_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
-	RGL_SAH_OK(cudaStreamSynchronize(s));
 	const int nBlock = (int) hostCtr[kCtrBlock];
 	if (nBlock > 0) {
-		kSahBlock<<<nBlock, kThreads, 0, s>>>(blockTasks, lo, hi, cen, sortedIds, bin, rangeFirst, rangeLast, ctr);
+		prepareSahBlock();
+		kSahBlock<<<nBlock, kBlockThreads, sizeof(BlockShared), s>>>(blockTasks, n, nullptr, const_cast<float4*>(lo), const_cast<float4*>(hi),
+		                                                             sortedIds, NodeSink{bin, rangeFirst, rangeLast, ctr});
 		countLaunch();
 	}
 	RGL_SAH_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
@@ -1034,64 +1282,16 @@ void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* 
 	}
 }
 
-namespace {
 static_assert(kBigTask == kSahSmallMax, "one block builds ranges up to kSahSmallMax primitives");
 
-// Root task and control words of a one-block build.
-__global__ void kSahSmallRoot(SahTask* task, uint32_t* ctr, int n)
-{
-	if (threadIdx.x < kCtrWords) {
-		ctr[threadIdx.x] = (threadIdx.x == kCtrNodes || threadIdx.x == kCtrBlock) ? 1u : 0u;
-	}
-	if (threadIdx.x == 0) {
-		task[0] = SahTask{0, n, 0, 0};
-	}
-}
-
-struct SmallScratch
-{
-	float4* cen;
-	uint32_t* ids;
-	SahTask* task;
-	uint32_t* ctr;
-};
-SmallScratch carveSmall(void* scratch, int n)
-{
-	uint8_t* p = static_cast<uint8_t*>(scratch);
-	auto take = [&](size_t bytes) {
-		uint8_t* q = p;
-		p += (bytes + 255) & ~size_t{255};
-		return q;
-	};
-	SmallScratch s;
-	s.cen = reinterpret_cast<float4*>(take(sizeof(float4) * (size_t) n));
-	s.ids = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (size_t) n));
-	s.task = reinterpret_cast<SahTask*>(take(sizeof(SahTask)));
-	s.ctr = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * kCtrWords));
-	return s;
-}
-} // namespace
-
-size_t sahSmallScratchBytes(int n)
-{
-	auto up = [](size_t b) { return (b + 255) & ~size_t{255}; };
-	return up(sizeof(float4) * (size_t) n) + up(sizeof(uint32_t) * (size_t) n) + up(sizeof(SahTask)) + up(sizeof(uint32_t) * kCtrWords);
-}
-
-void enqueueSahTopologySmall(const float4* lo, const float4* hi, int n, void* scratch, BinNode* bin, int32_t* rangeFirst,
-                             int32_t* rangeLast, uint32_t* sortedIds, cudaStream_t s)
+void enqueueSahTopologySmall(const InstanceRec* inst, float4* lo, float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
+                             uint32_t* sortedIds, cudaStream_t s)
 {
 	if (n <= 0 || n > kSahSmallMax) {
 		throw std::runtime_error("SAH build: one-block topology takes 1.." + std::to_string(kSahSmallMax) + " primitives");
 	}
-	const SmallScratch sc = carveSmall(scratch, n);
-	kSahInit<<<blocksFor(n, 256), 256, 0, s>>>(lo, hi, n, sc.cen, sc.ids, sortedIds);
+	kSahBlock<<<1, kBlockThreads, sizeof(BlockShared), s>>>(nullptr, n, inst, lo, hi, sortedIds, NodeSink{bin, rangeFirst, rangeLast, nullptr});
 	countLaunch();
-	if (n >= 2) {
-		kSahSmallRoot<<<1, 32, 0, s>>>(sc.task, sc.ctr, n);
-		kSahBlock<<<1, kThreads, 0, s>>>(sc.task, lo, hi, sc.cen, sortedIds, bin, rangeFirst, rangeLast, sc.ctr);
-		countLaunch(2);
-	}
 }
 
 } // namespace rgl
