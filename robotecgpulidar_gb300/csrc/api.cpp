@@ -19,6 +19,7 @@
 #include <rgl/api/extensions/tape.h>
 
 #include "batch.hpp"
+#include "build_memory.hpp"
 #include "tape.hpp"
 #include "serve.hpp"
 #include "graph.hpp"
@@ -333,6 +334,7 @@ RGL_API rgl_status_t rgl_cleanup(void)
 		Entities::map().clear();
 		Meshes::map().clear();
 		Textures::map().clear();
+		rgl::trimBuildMemory();
 	});
 	RGL_TAPE_RECORD();
 	return status;

@@ -1,0 +1,90 @@
+// Device memory that comes and goes with scene objects: temporaries of acceleration-structure builds,
+// and the storage of meshes and their structures.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace rgl {
+
+// Scene storage (mesh vertices, indices, BLAS nodes), from a pool that keeps up to kKeepBytes for the
+// next mesh. The memory is usable on every stream once `s` has reached the call's point; freeing waits
+// for the device first, as cudaFree of a plain allocation does.
+void* allocateStorage(size_t bytes, cudaStream_t s);
+void freeStorage(void* p);
+
+// Temporaries of one build on one stream: one stream-ordered allocation, given back in the stream's
+// order when the object goes.
+class BuildScratch
+{
+public:
+	explicit BuildScratch(cudaStream_t s) : stream_(s) {}
+	BuildScratch(const BuildScratch&) = delete;
+	BuildScratch& operator=(const BuildScratch&) = delete;
+	~BuildScratch();
+
+	// Places arrays in the order in which `layout` names them, each on a 256-byte boundary; called once.
+	class Carver
+	{
+	public:
+		template<class T>
+		void operator()(T*& p, size_t count)
+		{
+			used_ = (used_ + 255) & ~(size_t) 255;
+			p = reinterpret_cast<T*>(base_ + used_);
+			used_ += sizeof(T) * (count > 0 ? count : 1);
+		}
+
+	private:
+		friend class BuildScratch;
+		uintptr_t base_ = 0;
+		size_t used_ = 0;
+	};
+	template<class Layout>
+	void carve(Layout&& layout)
+	{
+		Carver size;
+		layout(size);
+		Carver place;
+		place.base_ = allocate(size.used_);
+		layout(place);
+	}
+
+private:
+	uintptr_t allocate(size_t bytes);
+	cudaStream_t stream_;
+	void* base_ = nullptr;
+};
+
+// What a device build tells the host: written by the build's last kernel straight into mapped pinned
+// memory and read after the stream has been synchronised, without a copy.
+struct BuildReport
+{
+	int32_t done;               // 1 once written
+	int32_t sortFailed;         // the radix sort's look-back did not complete
+	uint32_t nodes, leaves;     // wide nodes and leaf records written
+	uint32_t sahPending;        // ranges that the levels so far left unsplit: nothing was collapsed
+	uint32_t sahNodes, sahError; // binary nodes of the SAH topology, an index left its range
+	float box[6];               // root box lo xyz, hi xyz
+};
+class HostReport
+{
+public:
+	HostReport();
+	HostReport(const HostReport&) = delete;
+	HostReport& operator=(const HostReport&) = delete;
+	~HostReport();
+	volatile BuildReport* host() const { return host_; }
+	BuildReport* device() const { return device_; }
+
+private:
+	volatile BuildReport* host_ = nullptr;
+	BuildReport* device_ = nullptr;
+};
+
+// Returns what the pools and the report list keep beyond what is in use; false when nothing was ever kept.
+bool trimBuildMemory();
+
+} // namespace rgl

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -45,13 +46,14 @@ __host__ __device__ __forceinline__ float orderedFloat(uint32_t u)
 #endif
 }
 
-// Triangle boxes, centroids and the centroid bounds (6 ordered uints: min xyz, max xyz).
+// Triangle boxes, centroids and, if asked for, the centroid bounds: 6 ordered uints, the minima xyz
+// complemented so that all of them start at zero and grow, then the maxima xyz.
 __global__ void kTriBounds(const float* __restrict__ v, const int32_t* __restrict__ idx, int nTris, float4* lo, float4* hi,
                            uint32_t* cbounds)
 {
 	__shared__ uint32_t sh[6];
 	if (threadIdx.x < 6) {
-		sh[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+		sh[threadIdx.x] = 0u;
 	}
 	__syncthreads();
 	int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,18 +65,18 @@ __global__ void kTriBounds(const float* __restrict__ v, const int32_t* __restric
 		float4 h = make_float4(fmaxf(fmaxf(a[0], b[0]), c[0]), fmaxf(fmaxf(a[1], b[1]), c[1]), fmaxf(fmaxf(a[2], b[2]), c[2]), 0.f);
 		lo[t] = l;
 		hi[t] = h;
-		float cx = 0.5f * (l.x + h.x), cy = 0.5f * (l.y + h.y), cz = 0.5f * (l.z + h.z);
-		atomicMin(&sh[0], orderedBits(cx));
-		atomicMin(&sh[1], orderedBits(cy));
-		atomicMin(&sh[2], orderedBits(cz));
-		atomicMax(&sh[3], orderedBits(cx));
-		atomicMax(&sh[4], orderedBits(cy));
-		atomicMax(&sh[5], orderedBits(cz));
+		if (cbounds != nullptr) {
+			float cx = 0.5f * (l.x + h.x), cy = 0.5f * (l.y + h.y), cz = 0.5f * (l.z + h.z);
+			atomicMax(&sh[0], ~orderedBits(cx));
+			atomicMax(&sh[1], ~orderedBits(cy));
+			atomicMax(&sh[2], ~orderedBits(cz));
+			atomicMax(&sh[3], orderedBits(cx));
+			atomicMax(&sh[4], orderedBits(cy));
+			atomicMax(&sh[5], orderedBits(cz));
+		}
 	}
 	__syncthreads();
-	if (threadIdx.x < 3) {
-		atomicMin(&cbounds[threadIdx.x], sh[threadIdx.x]);
-	} else if (threadIdx.x < 6) {
+	if (cbounds != nullptr && threadIdx.x < 6) {
 		atomicMax(&cbounds[threadIdx.x], sh[threadIdx.x]);
 	}
 }
@@ -86,7 +88,7 @@ __global__ void kMorton(const float4* __restrict__ lo, const float4* __restrict_
 	if (t >= n) {
 		return;
 	}
-	Box cb{orderedFloat(cbounds[0]), orderedFloat(cbounds[1]), orderedFloat(cbounds[2]),
+	Box cb{orderedFloat(~cbounds[0]), orderedFloat(~cbounds[1]), orderedFloat(~cbounds[2]),
 	       orderedFloat(cbounds[3]), orderedFloat(cbounds[4]), orderedFloat(cbounds[5])};
 	float4 l = lo[t], h = hi[t];
 	codes[t] = morton30(0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z), cb);
@@ -165,22 +167,30 @@ __global__ void kBottomUp(int n, const uint32_t* __restrict__ ids, const float4*
 	}
 }
 
-// Counters of one collapse: three depth counters used in turn (see kCollapse), then its results.
+// Counters of one collapse: three depth counters used in turn (see kCollapse).
 struct CollapseState
 {
 	collapsedev::DepthCounter depth[3];
-	uint32_t nodes, leaves;
+};
+
+// What the collapse tells the host about the stages before it.
+struct BuildStages
+{
+	const uint32_t* sah;       // control words of the SAH topology, or null
+	const int32_t* sortFailed; // flag of the radix sort, or null
+	BuildReport* report;       // mapped host memory
 };
 
 // The whole collapse of a binary tree over n primitives in one cooperative launch, depth by depth with
 // a grid barrier between (one launch per depth, sixteen between host checks of the queue, before). A
 // depth adds to its own counter; the counter after next is cleared meanwhile, when nobody reads it.
-// `st` is zero at the start. levelStarts (optional) receives the first node of every depth and the node
+// `st` is zero at the start. A SAH topology that is not complete is not collapsed: the report says so, and
+// the host goes on with it. levelStarts (optional) receives the first node of every depth and the node
 // count, up to levelCap entries. 131,072 triangles: 516 us for sixteen launches before, see
 // collapse.cuh for what a depth cost and why.
 constexpr int kCollapseThreads = 128;
 __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* st,
-                                                              int32_t* levelStarts, int32_t* nLevels, int levelCap)
+                                                              int32_t* levelStarts, int32_t* nLevels, int levelCap, BuildStages stages)
 {
 	cooperative_groups::grid_group grid = cooperative_groups::this_grid();
 	const uint32_t warp = (blockIdx.x * kCollapseThreads + threadIdx.x) >> 5, warps = gridDim.x * (kCollapseThreads / 32);
@@ -188,6 +198,22 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in,
 	const bool first = blockIdx.x == 0 && threadIdx.x == 0;
 	uint32_t start = 0, end = 1, leaves = 0;
 	int level = 0;
+	volatile BuildReport* report = stages.report;
+	if (stages.sah != nullptr) {
+		const uint32_t pending = stages.sah[kSahNext], nodes = stages.sah[kSahNodes], error = stages.sah[kSahError];
+		if (first) {
+			report->sahPending = pending;
+			report->sahNodes = nodes;
+			report->sahError = error;
+		}
+		if (pending != 0u || error != 0u || nodes != (uint32_t) (n - 1)) {
+			if (first) {
+				report->done = 1;
+				__threadfence_system();
+			}
+			return; // every block sees the same words
+		}
+	}
 	for (; start < end; ++level) {
 		collapsedev::DepthCounter* ctr = &st->depth[level % 3];
 		if (first) {
@@ -220,8 +246,19 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in,
 		}
 	}
 	if (first) {
-		st->nodes = end;
-		st->leaves = leaves;
+		report->nodes = end;
+		report->leaves = leaves;
+		report->sortFailed = stages.sortFailed != nullptr ? *stages.sortFailed : 0;
+		const float4* root = reinterpret_cast<const float4*>(in.bin);
+		const float4 lo = n > 1 ? root[0] : in.triLo[0], hi = n > 1 ? root[1] : in.triHi[0];
+		report->box[0] = lo.x;
+		report->box[1] = lo.y;
+		report->box[2] = lo.z;
+		report->box[3] = hi.x;
+		report->box[4] = hi.y;
+		report->box[5] = hi.z;
+		report->done = 1;
+		__threadfence_system();
 		if (levelStarts != nullptr && level < levelCap) {
 			levelStarts[level] = (int32_t) end;
 			*nLevels = level;
@@ -230,18 +267,6 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in,
 }
 
 inline int blocks(int n, int b) { return (n + b - 1) / b; }
-
-template<class T>
-T* mallocAsync(size_t count, cudaStream_t s)
-{
-	void* p = nullptr;
-	RGL_CUDA_OK(cudaMallocAsync(&p, sizeof(T) * (count ? count : 1), s));
-	return static_cast<T*>(p);
-}
-
-} // namespace
-
-namespace {
 
 struct WideBuildResult
 {
@@ -257,7 +282,8 @@ struct LevelRecord
 	int capacity = 0;
 };
 
-void launchCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* state, LevelRecord levels, cudaStream_t s)
+void launchCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* state, LevelRecord levels, BuildStages stages,
+                    cudaStream_t s)
 {
 	static const int most = [] { // blocks that fit the device at once, as the grid barrier needs
 		int dev = 0, sms = 0, perSm = 0;
@@ -269,38 +295,50 @@ void launchCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, C
 	// The widest depths hold about n / 6 nodes, 16 at a time per block; a small tree takes fewer blocks,
 	// whose barrier is cheaper.
 	int grid = std::max(1, std::min(most, n / 256));
-	void* args[] = {&in, &out, &n, &state, &levels.starts, &levels.count, &levels.capacity};
+	void* args[] = {&in, &out, &n, &state, &levels.starts, &levels.count, &levels.capacity, &stages};
 	RGL_CUDA_OK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&kCollapse), dim3(grid), dim3(kCollapseThreads), args, 0, s));
 	countLaunch();
 }
 
-// Wide BVH over n primitive boxes lo/hi (device) whose centroid bounds are in cb (6 ordered uints),
-// all written on stream s: the binary topology (binned SAH when `sah`, else Morton codes, onesweep
-// sort, LBVH and bottom-up bounds), then the collapse into 8-wide nodes (one launch). Leaf records are
-// triangles (dV/dI given) or primitive indices (dV null). `levels` optionally receives the first node
-// index of every depth and the node count. Frees lo, hi, cb and its temporaries and synchronises s (a
-// one-off build).
-WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const float* dV, const int32_t* dI, int leafMax,
-                          WideNode* outNodes, TriRecord* outLeaves, Box* outBoxes, cudaStream_t s, bool sah, LevelRecord levels = {})
+// Wide BVH over n primitive boxes lo/hi (device), written on stream s: the binary topology (binned SAH, or
+// with the centroid bounds cb, 6 words of kTriBounds, Morton codes, onesweep sort, LBVH and bottom-up
+// bounds), then the collapse into 8-wide nodes (one launch). Leaf records are triangles (dV/dI given) or
+// primitive indices (dV null). `levels` optionally receives the first node index of every depth and the
+// node count. The host waits once, for the report of the last kernel, so s is synchronised at the end.
+WideBuildResult buildWide(const float4* lo, const float4* hi, const uint32_t* cb, int n, const float* dV, const int32_t* dI, int leafMax,
+                          WideNode* outNodes, TriRecord* outLeaves, Box* outBoxes, cudaStream_t s, LevelRecord levels = {})
 {
-	uint32_t* codes = mallocAsync<uint32_t>(n, s);
-	uint32_t* ids = mallocAsync<uint32_t>(n, s);
-	void* sortScratch = mallocAsync<uint8_t>(sortPairsScratchBytes(n, 30), s);
-	BinNode* bin = mallocAsync<BinNode>(n, s);
-	int32_t* rf = mallocAsync<int32_t>(n, s);
-	int32_t* rl = mallocAsync<int32_t>(n, s);
-	int32_t* pi = mallocAsync<int32_t>(n, s);
-	int32_t* pl = mallocAsync<int32_t>(n, s);
-	uint32_t* visits = mallocAsync<uint32_t>(n, s);
-	collapsedev::CollapseTask* queue = mallocAsync<collapsedev::CollapseTask>(n, s);
-	CollapseState* state = mallocAsync<CollapseState>(1, s);
-	int32_t* err = mallocAsync<int32_t>(1, s);
-	RGL_CUDA_OK(cudaMemsetAsync(visits, 0, sizeof(uint32_t) * n, s));
-	RGL_CUDA_OK(cudaMemsetAsync(state, 0, sizeof(CollapseState), s));
-	RGL_CUDA_OK(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
+	const bool sah = cb == nullptr;
+	BuildScratch scratch(s);
+	uint32_t *codes = nullptr, *ids = nullptr, *visits = nullptr;
+	uint8_t* sortScratch = nullptr;
+	BinNode* bin = nullptr;
+	int32_t *rf = nullptr, *rl = nullptr, *pi = nullptr, *pl = nullptr, *err = nullptr;
+	collapsedev::CollapseTask* queue = nullptr;
+	CollapseState* state = nullptr;
+	scratch.carve([&](BuildScratch::Carver& place) {
+		place(state, 1); // cleared together: state, err and, for the LBVH, visits
+		place(err, 1);
+		if (!sah) {
+			place(visits, n);
+			place(codes, n);
+			place(sortScratch, sortPairsScratchBytes(n, 30));
+			place(pi, n);
+			place(pl, n);
+		}
+		place(ids, n);
+		place(bin, n);
+		place(rf, n);
+		place(rl, n);
+		place(queue, n);
+	});
+	const uint8_t* cleared = reinterpret_cast<const uint8_t*>(sah ? (const void*) (err + 1) : (const void*) (visits + n));
+	RGL_CUDA_OK(cudaMemsetAsync(state, 0, (size_t) (cleared - reinterpret_cast<const uint8_t*>(state)), s));
 
+	std::optional<SahTopology> topology;
 	if (sah) {
-		buildSahTopologyDevice(lo, hi, n, bin, rf, rl, ids, s);
+		topology.emplace(lo, hi, n, bin, rf, rl, ids, s);
+		topology->enqueue();
 	} else {
 		kMorton<<<blocks(n, 256), 256, 0, s>>>(lo, hi, n, cb, codes, ids);
 		countLaunch();
@@ -312,37 +350,46 @@ WideBuildResult buildWide(float4* lo, float4* hi, uint32_t* cb, int n, const flo
 			countLaunch();
 		}
 	}
-	CollapseInputs ci{bin, rf, rl, reinterpret_cast<const int32_t*>(ids), lo, hi, dV, dI, leafMax};
-	launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, s);
-	CollapseState result{};
-	int32_t sortFailed = 0;
-	RGL_CUDA_OK(cudaMemcpyAsync(&result, state, sizeof(result), cudaMemcpyDeviceToHost, s));
-	RGL_CUDA_OK(cudaMemcpyAsync(&sortFailed, err, sizeof(sortFailed), cudaMemcpyDeviceToHost, s));
-	BinNode rootBox{};
-	float4 leafLo{}, leafHi{};
-	if (n > 1) {
-		RGL_CUDA_OK(cudaMemcpyAsync(&rootBox, bin, sizeof(BinNode), cudaMemcpyDeviceToHost, s));
-	} else {
-		RGL_CUDA_OK(cudaMemcpyAsync(&leafLo, lo, sizeof(float4), cudaMemcpyDeviceToHost, s));
-		RGL_CUDA_OK(cudaMemcpyAsync(&leafHi, hi, sizeof(float4), cudaMemcpyDeviceToHost, s));
+	HostReport report;
+	const CollapseInputs ci{bin, rf, rl, reinterpret_cast<const int32_t*>(ids), lo, hi, dV, dI, leafMax};
+	const BuildStages stages{sah ? topology->control() : nullptr, err, report.device()};
+	const volatile BuildReport& r = *report.host();
+	for (;;) {
+		launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, stages, s);
+		RGL_CUDA_OK(cudaStreamSynchronize(s));
+		if (r.done == 0) {
+			throw std::runtime_error("BVH build: the collapse did not report");
+		}
+		if (r.sahPending == 0) {
+			break;
+		}
+		topology->enqueue(); // a deeper tree than its first levels
 	}
-	void* temps[] = {lo, hi, cb, codes, ids, sortScratch, bin, rf, rl, pi, pl, visits, queue, state, err};
-	for (void* p : temps) {
-		RGL_CUDA_OK(cudaFreeAsync(p, s));
+	if (r.sahError != 0) {
+		throw std::runtime_error("SAH build: a partition or range stack index left its range");
 	}
-	RGL_CUDA_OK(cudaStreamSynchronize(s));
-	if (sortFailed != 0) {
+	if (stages.sah != nullptr && r.sahNodes != (uint32_t) (n - 1)) {
+		throw std::runtime_error("SAH build: " + std::to_string(r.sahNodes) + " binary nodes for " + std::to_string(n) + " primitives");
+	}
+	if (r.sortFailed != 0) {
 		throw std::runtime_error("BVH build: radix sort look-back did not complete");
 	}
-	if (result.leaves != (uint32_t) n || result.nodes > (uint32_t) n) {
-		throw std::runtime_error("BVH build: collapse produced an inconsistent tree (leaf records " + std::to_string(result.leaves) +
-		                         ", nodes " + std::to_string(result.nodes) + ")");
+	if (r.leaves != (uint32_t) n || r.nodes > (uint32_t) n) {
+		throw std::runtime_error("BVH build: collapse produced an inconsistent tree (leaf records " + std::to_string(r.leaves) + ", nodes " +
+		                         std::to_string(r.nodes) + ")");
 	}
-	WideBuildResult r;
-	r.nodeCount = result.nodes;
-	r.bounds = n > 1 ? Box{rootBox.lox, rootBox.loy, rootBox.loz, rootBox.hix, rootBox.hiy, rootBox.hiz}
-	                 : Box{leafLo.x, leafLo.y, leafLo.z, leafHi.x, leafHi.y, leafHi.z};
-	return r;
+	return WideBuildResult{r.nodes, Box{r.box[0], r.box[1], r.box[2], r.box[3], r.box[4], r.box[5]}};
+}
+
+void allocBlas(BlasBuild& out, int nTris, cudaStream_t s)
+{
+	// A rebuild (an animated entity) reuses the previous storage when it is large enough.
+	if (out.nodes == nullptr || out.nodeCapacity < (uint32_t) nTris) {
+		freeBlas(out);
+		out.nodes = static_cast<WideNode*>(allocateStorage(sizeof(WideNode) * (size_t) nTris, s));
+		out.tris = static_cast<TriRecord*>(allocateStorage(sizeof(TriRecord) * (size_t) nTris, s));
+		out.nodeCapacity = (uint32_t) nTris;
+	}
 }
 
 } // namespace
@@ -354,24 +401,24 @@ void buildBlas(const float* dVertices, int nVertices, const int32_t* dIndices, i
 		throw std::invalid_argument("mesh without triangles");
 	}
 	const int T = nTris;
-	float4* lo = mallocAsync<float4>(T, s);
-	float4* hi = mallocAsync<float4>(T, s);
-	uint32_t* cb = mallocAsync<uint32_t>(8, s);
-	// A rebuild (an animated entity) reuses the previous storage when it is large enough.
-	if (out.nodes == nullptr || out.nodeCapacity < (uint32_t) T) {
-		if (out.nodes != nullptr) {
-			freeBlas(out);
+	BuildScratch scratch(s);
+	float4 *lo = nullptr, *hi = nullptr;
+	uint32_t* cb = nullptr;
+	scratch.carve([&](BuildScratch::Carver& place) {
+		place(lo, T);
+		place(hi, T);
+		if (!sah) {
+			place(cb, 6);
 		}
-		RGL_CUDA_OK(cudaMalloc(&out.nodes, sizeof(WideNode) * (size_t) T));
-		RGL_CUDA_OK(cudaMalloc(&out.tris, sizeof(TriRecord) * (size_t) T));
-		out.nodeCapacity = (uint32_t) T;
-	}
+	});
+	allocBlas(out, T, s);
 	out.triCount = T;
-	uint32_t cbInit[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-	RGL_CUDA_OK(cudaMemcpyAsync(cb, cbInit, sizeof(cbInit), cudaMemcpyHostToDevice, s));
+	if (!sah) {
+		RGL_CUDA_OK(cudaMemsetAsync(cb, 0, 6 * sizeof(uint32_t), s));
+	}
 	kTriBounds<<<blocks(T, 256), 256, 0, s>>>(dVertices, dIndices, T, lo, hi, cb);
 	countLaunch();
-	const WideBuildResult r = buildWide(lo, hi, cb, T, dVertices, dIndices, kLeafMaxTris, out.nodes, out.tris, nullptr, s, sah);
+	const WideBuildResult r = buildWide(lo, hi, cb, T, dVertices, dIndices, kLeafMaxTris, out.nodes, out.tris, nullptr, s);
 	out.nodeCount = r.nodeCount;
 	out.bounds[0] = r.bounds.lox;
 	out.bounds[1] = r.bounds.loy;
@@ -421,14 +468,7 @@ void buildBlasHost(const float* hVertices, int nVertices, const int32_t* hIndice
 	if (triCounter != (uint32_t) T || wideCounter > (uint32_t) T) {
 		throw std::runtime_error("BLAS build: collapse produced an inconsistent tree");
 	}
-	if (out.nodes == nullptr || out.nodeCapacity < (uint32_t) T) {
-		if (out.nodes != nullptr) {
-			freeBlas(out);
-		}
-		RGL_CUDA_OK(cudaMalloc(&out.nodes, sizeof(WideNode) * (size_t) T));
-		RGL_CUDA_OK(cudaMalloc(&out.tris, sizeof(TriRecord) * (size_t) T));
-		out.nodeCapacity = (uint32_t) T;
-	}
+	allocBlas(out, T, nullptr);
 	RGL_CUDA_OK(cudaMemcpy(out.nodes, wide.data(), sizeof(WideNode) * wideCounter, cudaMemcpyHostToDevice));
 	RGL_CUDA_OK(cudaMemcpy(out.tris, tris.data(), sizeof(TriRecord) * (size_t) T, cudaMemcpyHostToDevice));
 	out.nodeCount = wideCounter;
@@ -444,10 +484,11 @@ void buildBlasHost(const float* hVertices, int nVertices, const int32_t* hIndice
 
 void freeBlas(BlasBuild& b)
 {
-	cudaFree(b.nodes);
-	cudaFree(b.tris);
+	freeStorage(b.nodes);
+	freeStorage(b.tris);
 	b.nodes = nullptr;
 	b.tris = nullptr;
+	b.nodeCapacity = 0;
 }
 
 namespace {
@@ -689,13 +730,16 @@ void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBu
 		hLo[i] = make_float4(r.lox, r.loy, r.loz, 0.0f);
 		hHi[i] = make_float4(r.hix, r.hiy, r.hiz, 0.0f);
 	}
-	float4* lo = mallocAsync<float4>(n, s);
-	float4* hi = mallocAsync<float4>(n, s);
-	uint32_t* cb = mallocAsync<uint32_t>(8, s); // centroid bounds: read by the Morton path only
+	BuildScratch scratch(s);
+	float4 *lo = nullptr, *hi = nullptr;
+	scratch.carve([&](BuildScratch::Carver& place) {
+		place(lo, n);
+		place(hi, n);
+	});
 	// Pageable sources: each copy is staged before the call returns.
 	RGL_CUDA_OK(cudaMemcpyAsync(lo, hLo.data(), sizeof(float4) * (size_t) n, cudaMemcpyHostToDevice, s));
 	RGL_CUDA_OK(cudaMemcpyAsync(hi, hHi.data(), sizeof(float4) * (size_t) n, cudaMemcpyHostToDevice, s));
-	const WideBuildResult r = buildWide(lo, hi, cb, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s, true,
+	const WideBuildResult r = buildWide(lo, hi, nullptr, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s,
 	                                    LevelRecord{t.levelStarts, t.nLevels, t.levelCapacity});
 	t.nodeCount = r.nodeCount;
 	kEnterRecords<<<blocks(n, 128), 128, 0, s>>>(t.leaves, dInst, n, t.enter);

@@ -1,5 +1,7 @@
 #include "common.hpp"
 
+#include "build_memory.hpp"
+
 #include <atomic>
 #include <cstring>
 #include <iostream>
@@ -173,9 +175,11 @@ DeviceBuffer::~DeviceBuffer() { release(); }
 void DeviceBuffer::release()
 {
 	if (ptr_) {
-		cudaFree(ptr_);
 		if (tracked_) {
+			cudaFree(ptr_);
 			allocEpoch.fetch_add(1, std::memory_order_relaxed);
+		} else {
+			freeStorage(ptr_);
 		}
 	}
 	ptr_ = nullptr;
@@ -189,9 +193,19 @@ void* DeviceBuffer::ensure(size_t bytes)
 	}
 	size_t want = bytes < 256 ? 256 : bytes;
 	void* p = nullptr;
-	RGL_CHECK_CUDA(cudaMalloc(&p, want));
+	if (tracked_) {
+		cudaError_t e = cudaMalloc(&p, want);
+		if (e == cudaErrorMemoryAllocation && trimBuildMemory()) {
+			cudaGetLastError();
+			e = cudaMalloc(&p, want);
+		}
+		RGL_CHECK_CUDA(e);
+	} else {
+		p = allocateStorage(want, nullptr);
+		RGL_CHECK_CUDA(cudaStreamSynchronize(nullptr)); // usable on every stream
+	}
 	if (ptr_) {
-		cudaFree(ptr_);
+		tracked_ ? (void) cudaFree(ptr_) : freeStorage(ptr_);
 	}
 	ptr_ = p;
 	cap_ = want;

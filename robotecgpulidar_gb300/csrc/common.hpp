@@ -78,7 +78,7 @@ class DeviceBuffer
 public:
 	DeviceBuffer() = default;
 	// A buffer that kernels reach only through another device-resident pointer (scene data behind the
-	// SceneView) does not invalidate captured runs when it moves.
+	// SceneView) does not invalidate captured runs when it moves; it comes from the scene storage pool.
 	explicit DeviceBuffer(bool affectsCapturedRuns) : tracked_(affectsCapturedRuns) {}
 	DeviceBuffer(const DeviceBuffer&) = delete;
 	DeviceBuffer& operator=(const DeviceBuffer&) = delete;

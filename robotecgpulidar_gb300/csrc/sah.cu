@@ -22,6 +22,7 @@
 // collapse does not depend on it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -29,6 +30,16 @@
 #include "kernels.hpp"
 
 namespace rgl {
+
+struct SahTask
+{
+	int32_t lo, hi, node, pad; // sorted positions [lo, hi), binary node index
+};
+
+struct SahSplit
+{
+	int32_t axis, bin, nLeft, pad; // axis -1: split in the middle
+};
 
 namespace {
 
@@ -52,21 +63,6 @@ constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kEmptyLo = 0xffffffffu;      // identity of min over ordered bits
 constexpr uint32_t kEmptyHi = 0u;               // identity of max
 constexpr float kInf = __builtin_huge_valf();
-
-struct SahTask
-{
-	int32_t lo, hi, node, pad; // sorted positions [lo, hi), binary node index
-};
-
-struct SahSplit
-{
-	int32_t axis, bin, nLeft, pad; // axis -1: split in the middle
-};
-
-// Control words: [0] node counter, [1] next-level task count, [2] block task count, [3] tasks of the
-// current level, [4] error: a partition or stack index outside its range (never expected: the counts
-// and the partition use the same bin function), the offending write is skipped.
-enum { kCtrNodes = 0, kCtrNext = 1, kCtrBlock = 2, kCtrCur = 3, kCtrError = 4, kCtrWords = 8 };
 
 __device__ __forceinline__ uint32_t ordered(float f)
 {
@@ -232,8 +228,8 @@ __device__ __forceinline__ void emitNode(int node, int lo, int hi, int nLeft, co
                                          int32_t* rangeLast, uint32_t* ctr, int32_t& left, int32_t& right)
 {
 	const int mid = lo + nLeft;
-	left = (mid - lo == 1) ? ~lo : (int32_t) atomicAdd(&ctr[kCtrNodes], 1u);
-	right = (hi - mid == 1) ? ~mid : (int32_t) atomicAdd(&ctr[kCtrNodes], 1u);
+	left = (mid - lo == 1) ? ~lo : (int32_t) atomicAdd(&ctr[kSahNodes], 1u);
+	right = (hi - mid == 1) ? ~mid : (int32_t) atomicAdd(&ctr[kSahNodes], 1u);
 	BinNode bn;
 	bn.lox = unordered(b12[0]);
 	bn.loy = unordered(b12[1]);
@@ -251,9 +247,16 @@ __device__ __forceinline__ void emitNode(int node, int lo, int hi, int nLeft, co
 // ------------------------------------------------------------------ level loop (ranges > kBigTask)
 
 __global__ void kSahInit(const float4* __restrict__ lo, const float4* __restrict__ hi, int n, float4* __restrict__ cen,
-                         uint32_t* __restrict__ idsA, uint32_t* __restrict__ sorted)
+                         uint32_t* __restrict__ idsA, uint32_t* __restrict__ sorted, SahTask* levelTasks, SahTask* blockTasks, uint32_t* ctr)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i < kSahWords) {
+		const bool big = n > kBigTask;
+		ctr[i] = i == kSahNodes ? 1u : (i == (big ? kSahNext : kSahBlocks) ? 1u : 0u);
+		if (i == 0) {
+			*(big ? levelTasks : blockTasks) = SahTask{0, n, 0, 0}; // the root
+		}
+	}
 	if (i < n) {
 		const float4 l = lo[i], h = hi[i];
 		cen[i] = make_float4(__fmul_rn(0.5f, __fadd_rn(l.x, h.x)), __fmul_rn(0.5f, __fadd_rn(l.y, h.y)), __fmul_rn(0.5f, __fadd_rn(l.z, h.z)),
@@ -270,12 +273,12 @@ __global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int32_t* chunkB
 {
 	__shared__ int32_t sWarp[32];
 	__shared__ int32_t sCarry;
-	const int nTasks = (int) ctr[kCtrNext];
+	const int nTasks = (int) ctr[kSahNext];
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		sCarry = 0;
-		ctr[kCtrCur] = (uint32_t) nTasks;
-		ctr[kCtrNext] = 0u;
+		ctr[kSahCur] = (uint32_t) nTasks;
+		ctr[kSahNext] = 0u;
 	}
 	for (int i = threadIdx.x; i < nTasks * 12; i += blockDim.x) {
 		bounds[i] = isMinWord(i % 12) ? kEmptyLo : kEmptyHi;
@@ -329,7 +332,7 @@ __global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int32_t* chunkB
 __device__ __forceinline__ bool chunkRange(const int32_t* chunkBase, const uint32_t* ctr, const SahTask* tasks, int c, int& t, int& start,
                                            int& end, int& first)
 {
-	const int nTasks = (int) ctr[kCtrCur];
+	const int nTasks = (int) ctr[kSahCur];
 	if (nTasks == 0 || c >= chunkBase[nTasks]) {
 		return false;
 	}
@@ -464,7 +467,7 @@ __global__ void kSahSplit(const SahTask* __restrict__ tasks, const uint32_t* __r
 {
 	const int w = (int) ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
 	const int lane = threadIdx.x & 31;
-	if (w >= (int) ctr[kCtrCur]) {
+	if (w >= (int) ctr[kSahCur]) {
 		return;
 	}
 	const SahTask tk = tasks[w];
@@ -487,9 +490,9 @@ __global__ void kSahSplit(const SahTask* __restrict__ tasks, const uint32_t* __r
 			}
 			const SahTask child{r0[c], r1[c], cl[c], 0};
 			if (cnt > kBigTask) {
-				next[atomicAdd(&ctr[kCtrNext], 1u)] = child;
+				next[atomicAdd(&ctr[kSahNext], 1u)] = child;
 			} else {
-				blockTasks[atomicAdd(&ctr[kCtrBlock], 1u)] = child;
+				blockTasks[atomicAdd(&ctr[kSahBlocks], 1u)] = child;
 			}
 		}
 	}
@@ -618,7 +621,7 @@ __global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __res
 			const int dst = fl[k] ? tk.lo + rank : tk.lo + s.nLeft + (p - tk.lo - rank);
 			rank += fl[k] ? 1 : 0;
 			if (dst < tk.lo || dst >= tk.hi) {
-				atomicExch(&ctr[kCtrError], 1u);
+				atomicExch(&ctr[kSahError], 1u);
 				continue;
 			}
 			idsOut[dst] = id[k];
@@ -637,6 +640,7 @@ __global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __res
 // not depend on each other run together. With every range above 32 split by the whole block in turn and
 // every subrange of a small one split alone, the 131,072-triangle mesh took 885 us here, 94 instances 58.
 constexpr int kBlockThreads = 512;
+constexpr int kBlockGrid = 152; // one block per SM, by shared memory
 constexpr int kBlockWarps = kBlockThreads / 32;
 constexpr int kMidTask = 256;
 
@@ -654,7 +658,7 @@ struct BlockShared
 	int scan[kBlockWarps];
 	uint8_t perm[kBlockWarps][32];
 	int top, nMid[2], nSmall;
-	uint32_t nextNode;
+	uint32_t nextNode, taken;
 	int4 cur;
 	SahSplit split;
 
@@ -698,7 +702,7 @@ struct NodeSink
 	__device__ __forceinline__ void error() const
 	{
 		if (ctr != nullptr) {
-			atomicExch(&ctr[kCtrError], 1u);
+			atomicExch(&ctr[kSahError], 1u);
 		}
 	}
 	__device__ __forceinline__ void write(int node, int lo, int hi, const uint32_t* b12, int32_t left, int32_t right) const
@@ -1007,14 +1011,10 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 	__syncwarp();
 }
 
-// tasks: one range per block, or null for a one-block build of primitives [0, n) in the given order. Boxes
-// come from gLo / gHi, or, for a TLAS, from the instance records, and are then stored there for the collapse.
-__global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __restrict__ tasks, int n, const InstanceRec* __restrict__ inst,
-                                                           float4* gLo, float4* gHi, uint32_t* __restrict__ sorted, NodeSink out)
+// One range of at most kBigTask primitives, by the whole block; see kSahBlock.
+__device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, const SahTask* tasks, const InstanceRec* inst, float4* gLo,
+                                           float4* gHi, uint32_t* sorted, const NodeSink& out)
 {
-	extern __shared__ __align__(16) uint8_t smem[];
-	BlockShared& S = *reinterpret_cast<BlockShared*>(smem);
-	const SahTask task = tasks != nullptr ? tasks[blockIdx.x] : SahTask{0, n, 0, 0};
 	const int base = task.lo, cnt = task.hi - task.lo;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __rest
 	if (threadIdx.x == 0) {
 		S.top = S.nMid[0] = S.nMid[1] = S.nSmall = 0;
 		// A range of cnt primitives has cnt - 1 nodes: its own, and the rest numbered from here.
-		S.nextNode = out.ctr != nullptr ? atomicAdd(&out.ctr[kCtrNodes], (uint32_t) (cnt - 2)) : 1u;
+		S.nextNode = out.ctr != nullptr ? atomicAdd(&out.ctr[kSahNodes], (uint32_t) (cnt - 2)) : 1u;
 		const int4 r = make_int4(0, cnt, task.node, 0);
 		if (cnt > kMidTask) {
 			S.stack[S.top++] = r;
@@ -1167,15 +1167,36 @@ __global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __rest
 	}
 }
 
-inline int blocksFor(int n, int b) { return (n + b - 1) / b; }
-
-template<class T>
-T* sahAlloc(size_t count, cudaStream_t s)
+// tasks: ranges that the blocks take in turn, or null for a one-block build of primitives [0, n) in the given order. Boxes
+// come from gLo / gHi, or, for a TLAS, from the instance records, and are then stored there for the collapse.
+__global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __restrict__ tasks, int n, const InstanceRec* __restrict__ inst,
+                                                           float4* gLo, float4* gHi, uint32_t* __restrict__ sorted, NodeSink out)
 {
-	void* p = nullptr;
-	RGL_SAH_OK(cudaMallocAsync(&p, sizeof(T) * (count ? count : 1), s));
-	return static_cast<T*>(p);
+	extern __shared__ __align__(16) uint8_t smem[];
+	BlockShared& S = *reinterpret_cast<BlockShared*>(smem);
+	if (tasks == nullptr) {
+		buildRange(S, SahTask{0, n, 0, 0}, nullptr, inst, gLo, gHi, sorted, out);
+		return;
+	}
+	if (out.ctr[kSahNext] != 0u) {
+		return; // the levels are not done: nothing is taken yet
+	}
+	const uint32_t count = out.ctr[kSahBlocks];
+	for (;;) {
+		if (threadIdx.x == 0) {
+			S.taken = atomicAdd(&out.ctr[kSahTaken], 1u);
+		}
+		__syncthreads();
+		const uint32_t k = S.taken;
+		if (k >= count) {
+			return;
+		}
+		buildRange(S, tasks[k], tasks, inst, gLo, gHi, sorted, out);
+		__syncthreads();
+	}
 }
+
+inline int blocksFor(int n, int b) { return (n + b - 1) / b; }
 
 } // namespace
 
@@ -1188,98 +1209,65 @@ void prepareSahBlock()
 	(void) done;
 }
 
-void buildSahTopologyDevice(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
-                            uint32_t* sortedIds, cudaStream_t s)
+SahTopology::SahTopology(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
+                         uint32_t* sortedIds, cudaStream_t stream)
+    : lo_(lo), hi_(hi), n_(n), bin_(bin), rangeFirst_(rangeFirst), rangeLast_(rangeLast), sorted_(sortedIds), stream_(stream), scratch_(stream)
 {
-	if (n <= 0) {
-		return;
-	}
-	float4* cen = sahAlloc<float4>(n, s);
-	uint32_t* idsA = sahAlloc<uint32_t>(n, s);
-	uint32_t* idsB = sahAlloc<uint32_t>(n, s);
-	kSahInit<<<blocksFor(n, 256), 256, 0, s>>>(lo, hi, n, cen, idsA, sortedIds);
+	maxBig_ = n / (kBigTask + 1) + 1;       // disjoint ranges above kBigTask
+	const int maxBlock = n / 2 + 1;          // disjoint ranges of at least 2
+	const int maxChunks = n / kChunk + maxBig_ + 1;
+	scratch_.carve([&](BuildScratch::Carver& place) {
+		place(cen_, n);
+		place(idsCur_, n);
+		place(idsNext_, n);
+		place(cur_, maxBig_);
+		place(next_, maxBig_);
+		place(blockTasks_, maxBlock);
+		place(splits_, maxBig_);
+		place(bounds_, (size_t) maxBig_ * 12);
+		place(bins_, (size_t) maxBig_ * kTaskBinWords);
+		place(chunkBase_, maxBig_ + 1);
+		place(chunkLeft_, maxChunks);
+		place(ctr_, kSahWords);
+	});
+	kSahInit<<<blocksFor(n, 256), 256, 0, stream>>>(lo, hi, n, cen_, idsCur_, sortedIds, cur_, blockTasks_, ctr_);
 	countLaunch();
 	if (n < 2) {
-		RGL_SAH_OK(cudaFreeAsync(cen, s));
-		RGL_SAH_OK(cudaFreeAsync(idsA, s));
-		RGL_SAH_OK(cudaFreeAsync(idsB, s));
+		ctr_ = nullptr;
 		return;
 	}
-	const int maxBig = n / (kBigTask + 1) + 1;         // disjoint ranges above kBigTask
-	const int maxBlock = n / 2 + 1;                     // disjoint ranges of at least 2
-	SahTask* cur = sahAlloc<SahTask>(maxBig, s);
-	SahTask* nxt = sahAlloc<SahTask>(maxBig, s);
-	SahTask* blockTasks = sahAlloc<SahTask>(maxBlock, s);
-	SahSplit* splits = sahAlloc<SahSplit>(maxBig, s);
-	uint32_t* bounds = sahAlloc<uint32_t>((size_t) maxBig * 12, s);
-	uint32_t* bins = sahAlloc<uint32_t>((size_t) maxBig * kTaskBinWords, s);
-	const int maxChunks = n / kChunk + maxBig + 1;
-	int32_t* chunkBase = sahAlloc<int32_t>(maxBig + 1, s);
-	int32_t* chunkLeft = sahAlloc<int32_t>(maxChunks, s);
-	uint32_t* ctr = sahAlloc<uint32_t>(kCtrWords, s);
-	uint32_t* hostCtr = nullptr;
-	RGL_SAH_OK(cudaMallocHost(&hostCtr, sizeof(uint32_t) * kCtrWords));
+	// As many levels as an even tree takes and two more (a level with nothing left costs six empty
+	// launches, about 12 us; a look at what is left about 20).
+	while (n > kBigTask && (kBigTask << levels_) < n) {
+		++levels_;
+	}
+	levels_ += levels_ > 0 ? 2 : 0;
+}
 
-	uint32_t init[kCtrWords] = {1u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-	const SahTask root{0, n, 0, 0};
-	if (n > kBigTask) {
-		RGL_SAH_OK(cudaMemcpyAsync(cur, &root, sizeof(root), cudaMemcpyHostToDevice, s));
-		init[kCtrNext] = 1u;
-	} else {
-		RGL_SAH_OK(cudaMemcpyAsync(blockTasks, &root, sizeof(root), cudaMemcpyHostToDevice, s));
-		init[kCtrBlock] = 1u;
+void SahTopology::enqueue()
+{
+	if (ctr_ == nullptr) {
+		return;
 	}
-	RGL_SAH_OK(cudaMemcpyAsync(ctr, init, sizeof(init), cudaMemcpyHostToDevice, s));
-	uint32_t* idsCur = idsA;
-	uint32_t* idsNext = idsB;
-	// Levels run without the host: as many as an even tree takes and two more, then a look at what is left
-	// (a level with nothing left costs six empty launches, about 12 us; a look costs about 20).
-	int levels = 0;
-	while (n > kBigTask && (kBigTask << levels) < n) {
-		++levels;
+	const int grid = n_ / kChunk + maxBig_ + 1; // bound on a level's chunks; blocks past them return
+	for (int l = 0; l < levels_; ++l) {
+		kSahLevelPrep<<<1, 1024, 0, stream_>>>(cur_, chunkBase_, bounds_, ctr_);
+		kSahBounds<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, lo_, hi_, cen_, bounds_, bins_);
+		kSahBins<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, lo_, hi_, cen_, bounds_, bins_);
+		kSahSplit<<<blocksFor(maxBig_ * 32, 128), 128, 0, stream_>>>(cur_, bounds_, bins_, splits_, bin_, rangeFirst_, rangeLast_, next_,
+		                                                             blockTasks_, ctr_);
+		kSahPartCount<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, cen_, bounds_, splits_, chunkLeft_);
+		kSahPartScatter<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, cen_, bounds_, splits_, chunkLeft_, idsNext_, sorted_);
+		countLaunch(6);
+		std::swap(cur_, next_);
+		std::swap(idsCur_, idsNext_);
 	}
-	levels += levels > 0 ? 2 : 0;
-	const int grid = n / kChunk + maxBig + 1; // bound on a level's chunks; blocks past them return
-	for (;;) {
-		for (int l = 0; l < levels; ++l) {
-			kSahLevelPrep<<<1, 1024, 0, s>>>(cur, chunkBase, bounds, ctr);
-			kSahBounds<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, lo, hi, cen, bounds, bins);
-			kSahBins<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, lo, hi, cen, bounds, bins);
-			kSahSplit<<<blocksFor(maxBig * 32, 128), 128, 0, s>>>(cur, bounds, bins, splits, bin, rangeFirst, rangeLast, nxt, blockTasks, ctr);
-			kSahPartCount<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, cen, bounds, splits, chunkLeft);
-			kSahPartScatter<<<grid, kThreads, 0, s>>>(cur, ctr, chunkBase, idsCur, cen, bounds, splits, chunkLeft, idsNext, sortedIds);
-			countLaunch(6);
-			std::swap(cur, nxt);
-			std::swap(idsCur, idsNext);
-		}
-		RGL_SAH_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
-		RGL_SAH_OK(cudaStreamSynchronize(s));
-		if (hostCtr[kCtrNext] == 0u) {
-			break;
-		}
-		levels = 4;
-	}
-	const int nBlock = (int) hostCtr[kCtrBlock];
-	if (nBlock > 0) {
-		prepareSahBlock();
-		kSahBlock<<<nBlock, kBlockThreads, sizeof(BlockShared), s>>>(blockTasks, n, nullptr, const_cast<float4*>(lo), const_cast<float4*>(hi),
-		                                                             sortedIds, NodeSink{bin, rangeFirst, rangeLast, ctr});
-		countLaunch();
-	}
-	RGL_SAH_OK(cudaMemcpyAsync(hostCtr, ctr, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
-	void* temps[] = {cen, idsA, idsB, cur, nxt, blockTasks, splits, bounds, bins, chunkBase, chunkLeft, ctr};
-	for (void* p : temps) {
-		RGL_SAH_OK(cudaFreeAsync(p, s));
-	}
-	RGL_SAH_OK(cudaStreamSynchronize(s));
-	const uint32_t nodes = hostCtr[kCtrNodes], error = hostCtr[kCtrError];
-	RGL_SAH_OK(cudaFreeHost(hostCtr));
-	if (error != 0) {
-		throw std::runtime_error("SAH build: a partition or range stack index left its range");
-	}
-	if (nodes != (uint32_t) (n - 1)) {
-		throw std::runtime_error("SAH build: " + std::to_string(nodes) + " binary nodes for " + std::to_string(n) + " primitives");
-	}
+	levels_ = 4; // of a tree that is deeper
+	// Blocks take ranges until none is left: their number is known on the device only.
+	prepareSahBlock();
+	kSahBlock<<<std::min(n_ / 2 + 1, kBlockGrid), kBlockThreads, sizeof(BlockShared), stream_>>>(
+	    blockTasks_, n_, nullptr, const_cast<float4*>(lo_), const_cast<float4*>(hi_), sorted_, NodeSink{bin_, rangeFirst_, rangeLast_, ctr_});
+	countLaunch();
 }
 
 static_assert(kBigTask == kSahSmallMax, "one block builds ranges up to kSahSmallMax primitives");

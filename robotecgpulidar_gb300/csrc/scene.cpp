@@ -13,8 +13,14 @@ using rgl::Mat34;
 
 Mesh::Mesh(const rgl_vec3f* vertices, int32_t vc, const rgl_vec3i* indices, int32_t ic) : vertexCount(vc), triangleCount(ic)
 {
-	// Indices are validated here (the reference leaves out-of-range indices to device asserts).
-	for (int32_t t = 0; t < ic; ++t) {
+	// Indices are validated here (the reference leaves out-of-range indices to device asserts): all at once
+	// by the largest as an unsigned number, one by one only to name the first that is outside.
+	const int32_t* flat = &indices[0].value[0];
+	uint32_t largest = 0;
+	for (size_t i = 0; i < 3 * (size_t) ic; ++i) {
+		largest = std::max(largest, (uint32_t) flat[i]);
+	}
+	for (int32_t t = 0; t < ic && largest >= (uint32_t) vc; ++t) {
 		for (int k = 0; k < 3; ++k) {
 			int32_t v = indices[t].value[k];
 			if (v < 0 || v >= vc) {
@@ -25,8 +31,6 @@ Mesh::Mesh(const rgl_vec3f* vertices, int32_t vc, const rgl_vec3i* indices, int3
 	}
 	RGL_CHECK_CUDA(cudaMemcpy(dVertices.ensure(sizeof(rgl_vec3f) * vc), vertices, sizeof(rgl_vec3f) * vc, cudaMemcpyHostToDevice));
 	RGL_CHECK_CUDA(cudaMemcpy(dIndices.ensure(sizeof(rgl_vec3i) * ic), indices, sizeof(rgl_vec3i) * ic, cudaMemcpyHostToDevice));
-	hVertices.assign(&vertices[0].value[0], &vertices[0].value[0] + 3 * (size_t) vc);
-	hIndices.assign(&indices[0].value[0], &indices[0].value[0] + 3 * (size_t) ic);
 }
 
 Mesh::~Mesh()
@@ -132,8 +136,14 @@ void Mesh::ensureBlas(cudaStream_t s)
 	const auto t0 = std::chrono::steady_clock::now();
 	switch (gBlasBuilder.load()) {
 		case RGL_GB300_BLAS_HOST_SAH:
-			rgl::buildBlasHost(hVertices.data(), vertexCount, hIndices.data(), triangleCount, blas);
+		{
+			std::vector<float> v(3 * (size_t) vertexCount);
+			std::vector<int32_t> i(3 * (size_t) triangleCount);
+			RGL_CHECK_CUDA(cudaMemcpy(v.data(), dVertices.get(), sizeof(float) * v.size(), cudaMemcpyDeviceToHost));
+			RGL_CHECK_CUDA(cudaMemcpy(i.data(), dIndices.get(), sizeof(int32_t) * i.size(), cudaMemcpyDeviceToHost));
+			rgl::buildBlasHost(v.data(), vertexCount, i.data(), triangleCount, blas);
 			break;
+		}
 		case RGL_GB300_BLAS_DEVICE_LBVH:
 			rgl::buildBlas(dVertices.as<float>(), vertexCount, dIndices.as<int32_t>(), triangleCount, blas, s, false);
 			break;
@@ -172,8 +182,8 @@ void Entity::startAnimation()
 void Entity::finishAnimation(cudaStream_t s)
 {
 	rgl::launchUpdateVertices(mesh->vertexCount, dAnimDisplacement.as<float>(), dAnimVertices.as<float>(), s);
+	// Waits for the stream: the caller's vertices may go once this returns.
 	rgl::buildBlas(dAnimVertices.as<float>(), mesh->vertexCount, mesh->dIndices.as<int32_t>(), mesh->triangleCount, animBlas, s, false);
-	RGL_CHECK_CUDA(cudaStreamSynchronize(s));
 	formerAnimTimed = animTimed;
 	formerAnimTimeNs = animTimeNs;
 	animTimed = scene->timeSet;
@@ -192,7 +202,7 @@ void Entity::applyExternalAnimation(const rgl_vec3f* vertices, int32_t count)
 		    (int) count));
 	}
 	startAnimation();
-	RGL_CHECK_CUDA(cudaMemcpy(dAnimDisplacement.get(), vertices, sizeof(float) * 3 * (size_t) count, cudaMemcpyHostToDevice));
+	RGL_CHECK_CUDA(cudaMemcpyAsync(dAnimDisplacement.get(), vertices, sizeof(float) * 3 * (size_t) count, cudaMemcpyHostToDevice, nullptr));
 	finishAnimation(nullptr);
 }
 
@@ -214,8 +224,8 @@ void Entity::setPoseAndAnimate(const rgl_mat3x4f* pose, int32_t bones)
 	}
 	startAnimation();
 	skinned = true;
-	RGL_CHECK_CUDA(cudaMemcpy(dPose.ensure(sizeof(rgl_mat3x4f) * (size_t) bones), pose, sizeof(rgl_mat3x4f) * (size_t) bones,
-	                          cudaMemcpyHostToDevice));
+	RGL_CHECK_CUDA(cudaMemcpyAsync(dPose.ensure(sizeof(rgl_mat3x4f) * (size_t) bones), pose, sizeof(rgl_mat3x4f) * (size_t) bones,
+	                               cudaMemcpyHostToDevice, nullptr));
 	rgl::launchSkin(mesh->vertexCount, mesh->dVertices.as<float>(), mesh->dBoneWeights.as<rgl::BoneWeights>(), dPose.as<Mat34>(),
 	                mesh->dRestposes.as<Mat34>(), bones, static_cast<Mat34*>(dBoneMatrices.ensure(sizeof(Mat34) * (size_t) bones)),
 	                dAnimDisplacement.as<float>(), skinError.device(), nullptr);

@@ -33,8 +33,6 @@ struct Mesh
 	int32_t triangleCount = 0;
 	rgl::DeviceBuffer dVertices{false};
 	rgl::DeviceBuffer dIndices{false};
-	std::vector<float> hVertices;   // host copies for the host BLAS build (RGL_GB300_BLAS_HOST_SAH)
-	std::vector<int32_t> hIndices;
 	rgl::BlasBuild blas;
 	bool blasBuilt = false;
 	rgl::DeviceBuffer dBoneWeights{false}, dRestposes{false};
