@@ -65,7 +65,6 @@ struct BuildReport
 	int32_t done;               // 1 once written
 	int32_t sortFailed;         // the radix sort's look-back did not complete
 	uint32_t nodes, leaves;     // wide nodes and leaf records written
-	uint32_t sahPending;        // ranges that the levels so far left unsplit: nothing was collapsed
 	uint32_t sahNodes, sahError; // binary nodes of the SAH topology, an index left its range
 	float box[6];               // root box lo xyz, hi xyz
 };

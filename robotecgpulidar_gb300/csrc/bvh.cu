@@ -7,7 +7,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <optional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -184,8 +183,7 @@ struct BuildStages
 // The whole collapse of a binary tree over n primitives in one cooperative launch, depth by depth with
 // a grid barrier between (one launch per depth, sixteen between host checks of the queue, before). A
 // depth adds to its own counter; the counter after next is cleared meanwhile, when nobody reads it.
-// `st` is zero at the start. A SAH topology that is not complete is not collapsed: the report says so, and
-// the host goes on with it. levelStarts (optional) receives the first node of every depth and the node
+// `st` is zero at the start. A SAH topology that is not complete is not collapsed: the report says so. levelStarts (optional) receives the first node of every depth and the node
 // count, up to levelCap entries. 131,072 triangles: 516 us for sixteen launches before, see
 // collapse.cuh for what a depth cost and why.
 constexpr int kCollapseThreads = 128;
@@ -200,13 +198,12 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in,
 	int level = 0;
 	volatile BuildReport* report = stages.report;
 	if (stages.sah != nullptr) {
-		const uint32_t pending = stages.sah[kSahNext], nodes = stages.sah[kSahNodes], error = stages.sah[kSahError];
+		const uint32_t nodes = stages.sah[kSahNodes], error = stages.sah[kSahError];
 		if (first) {
-			report->sahPending = pending;
 			report->sahNodes = nodes;
 			report->sahError = error;
 		}
-		if (pending != 0u || error != 0u || nodes != (uint32_t) (n - 1)) {
+		if (error != 0u || nodes != (uint32_t) (n - 1)) {
 			if (first) {
 				report->done = 1;
 				__threadfence_system();
@@ -335,10 +332,10 @@ WideBuildResult buildWide(const float4* lo, const float4* hi, const uint32_t* cb
 	const uint8_t* cleared = reinterpret_cast<const uint8_t*>(sah ? (const void*) (err + 1) : (const void*) (visits + n));
 	RGL_CUDA_OK(cudaMemsetAsync(state, 0, (size_t) (cleared - reinterpret_cast<const uint8_t*>(state)), s));
 
-	std::optional<SahTopology> topology;
+	BuildScratch sahScratch(s);
+	const uint32_t* sahControl = nullptr;
 	if (sah) {
-		topology.emplace(lo, hi, n, bin, rf, rl, ids, s);
-		topology->enqueue();
+		sahControl = enqueueSahTopology(sahScratch, lo, hi, n, bin, rf, rl, ids, s);
 	} else {
 		kMorton<<<blocks(n, 256), 256, 0, s>>>(lo, hi, n, cb, codes, ids);
 		countLaunch();
@@ -352,18 +349,12 @@ WideBuildResult buildWide(const float4* lo, const float4* hi, const uint32_t* cb
 	}
 	HostReport report;
 	const CollapseInputs ci{bin, rf, rl, reinterpret_cast<const int32_t*>(ids), lo, hi, dV, dI, leafMax};
-	const BuildStages stages{sah ? topology->control() : nullptr, err, report.device()};
+	const BuildStages stages{sahControl, err, report.device()};
 	const volatile BuildReport& r = *report.host();
-	for (;;) {
-		launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, stages, s);
-		RGL_CUDA_OK(cudaStreamSynchronize(s));
-		if (r.done == 0) {
-			throw std::runtime_error("BVH build: the collapse did not report");
-		}
-		if (r.sahPending == 0) {
-			break;
-		}
-		topology->enqueue(); // a deeper tree than its first levels
+	launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, stages, s);
+	RGL_CUDA_OK(cudaStreamSynchronize(s));
+	if (r.done == 0) {
+		throw std::runtime_error("BVH build: the collapse did not report");
 	}
 	if (r.sahError != 0) {
 		throw std::runtime_error("SAH build: a partition or range stack index left its range");

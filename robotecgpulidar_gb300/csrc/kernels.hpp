@@ -40,39 +40,14 @@ void buildBlas(const float* dVertices, int nVertices, const int32_t* dIndices, i
                bool sah);
 // ---- sah.cu: binary binned-SAH topology of n primitive boxes (device lo/hi), the host builder's tree
 // (sah_build.hpp buildBinnedSahTree) computed on the device; output in the collapse's input format.
-// Nothing waits for the host: enqueue() queues the levels of an even tree and two more, then the ranges
-// that one block builds. A deeper tree shows as control()[kSahNext] != 0 once that has run; the block
-// ranges are then not built yet, and enqueue() goes on from there.
-class SahTopology
-{
-public:
-	SahTopology(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast, uint32_t* sortedIds,
-	            cudaStream_t stream);
-	void enqueue();
-	// Control words (kSahNodes, ...); null for a single primitive, which has no topology.
-	const uint32_t* control() const { return ctr_; }
-
-private:
-	const float4 *lo_, *hi_;
-	const int n_;
-	BinNode* const bin_;
-	int32_t *const rangeFirst_, *const rangeLast_;
-	uint32_t* const sorted_;
-	const cudaStream_t stream_;
-	int levels_ = 0, maxBig_ = 0;
-	BuildScratch scratch_;
-	float4* cen_ = nullptr;
-	uint32_t *idsCur_ = nullptr, *idsNext_ = nullptr;
-	struct SahTask *cur_ = nullptr, *next_ = nullptr, *blockTasks_ = nullptr;
-	struct SahSplit* splits_ = nullptr;
-	uint32_t *bounds_ = nullptr, *bins_ = nullptr, *ctr_ = nullptr;
-	int32_t *chunkBase_ = nullptr, *chunkLeft_ = nullptr;
-};
-// Control words of a topology build: binary nodes numbered so far, ranges of the next level, ranges for
-// one block each, ranges of the current level, an error (a partition or stack index outside its range,
-// never expected: the counts and the partition use the same bin function; the offending write is
-// skipped), and the next block range to be taken.
-enum SahControl { kSahNodes = 0, kSahNext = 1, kSahBlocks = 2, kSahCur = 3, kSahError = 4, kSahTaken = 5, kSahWords = 8 };
+// Nothing waits for the host. Returns the build's control words (device, in `scratch`), to be checked
+// before the topology is used; null for a single primitive.
+const uint32_t* enqueueSahTopology(BuildScratch& scratch, const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst,
+                                   int32_t* rangeLast, uint32_t* sortedIds, cudaStream_t stream);
+// Control words: binary nodes numbered, ranges for one block each, an error (a partition or stack index
+// outside its range, never expected: the counts and the partition use the same bin function; the
+// offending write is skipped), the next block range to be taken, and the ranges of three levels in turn.
+enum SahControl { kSahNodes = 0, kSahBlocks = 1, kSahError = 2, kSahTaken = 3, kSahLevel = 4, kSahWords = 8 };
 // The same topology for the world boxes of 1..kSahSmallMax instances, built by one block with no host
 // interaction (so it can be captured in a CUDA graph, after prepareSahBlock outside it); the boxes are
 // left in lo / hi.

@@ -6,20 +6,20 @@
 // runs on the device; the wide collapse and quantisation that follow are bvh_core.hpp's.
 //
 // Algorithm (after Wald 2007, binned SAH, 32 bins per axis; parallel top-down):
-//  * ranges of more than kBigTask primitives are split level by level, each by many blocks: a bounds
-//    pass (node box and centroid bounds), a binning pass (per-bin boxes and counts, shared-memory
-//    atomics flushed to the range's global bins), one warp per range evaluating the 3 x 31 split
-//    candidates, and a stable partition (per-chunk counts, then a scatter that ranks each chunk's
-//    elements with a block scan);
-//  * ranges of 2..kBigTask primitives are built to the leaves by one block each, in shared memory:
-//    ranges above kSmallTask split with block-wide passes, smaller ones by one warp each, which keeps
-//    its elements in registers and partitions them with ballots.
+//  * ranges of more than kBigTask primitives are split level by level, each by many blocks, all levels in
+//    one cooperative launch (kSahLevels): one warp per range evaluates the 3 x 31 split candidates from
+//    the range's bins; a pass over the elements counts how many go left and gathers the children's bounds;
+//    a second one puts them in their place (stable: counts of earlier chunks, then a block scan) and adds
+//    them to their child's bins (shared-memory atomics, then the range's);
+//  * ranges of 2..kBigTask primitives are built to the leaves by one block each, in shared memory
+//    (kSahBlock); blocks take ranges until none is left.
 // Exactness: boxes and centroid bounds are min/max (order free); the centroid, the bin index, the
 // half areas and the split costs use the host's expressions with round-to-nearest intrinsics and no
 // FMA contraction; among equal costs the first candidate in (axis, bin) order wins, as in the host's
 // strict comparison; partitions are stable; a range whose centroids all coincide splits in the
 // middle. Node numbering differs from the host's (atomics instead of a depth-first counter); the
 // collapse does not depend on it.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,7 +54,10 @@ namespace {
 constexpr int kBins = 32;
 constexpr int kBinWords = 7;                    // lo xyz, hi xyz (ordered bits), count
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
-constexpr int kBigTask = 2048;                  // larger ranges split in the level loop
+// Larger ranges split in the level loop, the others are built by a block each. 131,072 triangles, 2,048 /
+// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us (two blocks per SM from 1,024 down).
+constexpr int kBigTask = 1024;
+constexpr int kMeshThreads = 512;
 constexpr int kChunk = 512;                     // elements per block in the level loop: 256 blocks for 131,072 triangles
 constexpr int kThreads = 256;
 constexpr int kItems = kChunk / kThreads;       // 2 elements per thread
@@ -146,23 +149,26 @@ __device__ SahSplit warpBestSplit(const uint32_t* bins, const uint32_t* b12, int
 {
 	float bestCost = kInf;
 	int bestKey = 1 << 30, bestLeft = 0;
+	uint32_t v[3][kBinWords]; // all at once: the loads do not wait for each other
+#pragma unroll
+	for (int a = 0; a < 3; ++a) {
+#pragma unroll
+		for (int k = 0; k < kBinWords; ++k) {
+			v[a][k] = bins[(a * kBins + lane) * kBinWords + k];
+		}
+	}
+#pragma unroll
 	for (int a = 0; a < 3; ++a) {
 		const AxisFrame f = axisFrame(b12, a);
 		if (!f.valid) {
 			continue;
 		}
-		const uint32_t* bb = bins + (a * kBins + lane) * kBinWords;
-		uint32_t v[kBinWords];
-#pragma unroll
-		for (int k = 0; k < kBinWords; ++k) {
-			v[k] = bb[k];
-		}
 		// inclusive prefix (bins 0..lane) and suffix (bins lane..31)
 		uint32_t p[kBinWords], q[kBinWords];
 #pragma unroll
 		for (int k = 0; k < kBinWords; ++k) {
-			p[k] = v[k];
-			q[k] = v[k];
+			p[k] = v[a][k];
+			q[k] = v[a][k];
 		}
 #pragma unroll
 		for (int off = 1; off < 32; off <<= 1) {
@@ -222,319 +228,20 @@ __device__ SahSplit warpBestSplit(const uint32_t* bins, const uint32_t* b12, int
 	return s;
 }
 
-// Writes binary node `node` over sorted positions [lo, hi) split at lo + nLeft, allocates its
-// children's node indices and returns them (a leaf child is ~position).
-__device__ __forceinline__ void emitNode(int node, int lo, int hi, int nLeft, const uint32_t* b12, BinNode* bin, int32_t* rangeFirst,
-                                         int32_t* rangeLast, uint32_t* ctr, int32_t& left, int32_t& right)
-{
-	const int mid = lo + nLeft;
-	left = (mid - lo == 1) ? ~lo : (int32_t) atomicAdd(&ctr[kSahNodes], 1u);
-	right = (hi - mid == 1) ? ~mid : (int32_t) atomicAdd(&ctr[kSahNodes], 1u);
-	BinNode bn;
-	bn.lox = unordered(b12[0]);
-	bn.loy = unordered(b12[1]);
-	bn.loz = unordered(b12[2]);
-	bn.hix = unordered(b12[3]);
-	bn.hiy = unordered(b12[4]);
-	bn.hiz = unordered(b12[5]);
-	bn.left = left;
-	bn.right = right;
-	bin[node] = bn;
-	rangeFirst[node] = lo;
-	rangeLast[node] = hi - 1;
-}
-
 // ------------------------------------------------------------------ level loop (ranges > kBigTask)
 
-__global__ void kSahInit(const float4* __restrict__ lo, const float4* __restrict__ hi, int n, float4* __restrict__ cen,
-                         uint32_t* __restrict__ idsA, uint32_t* __restrict__ sorted, SahTask* levelTasks, SahTask* blockTasks, uint32_t* ctr)
+// One range of at most kBigTask primitives: its order, its task and the control words.
+__global__ void kSahInit(int n, uint32_t* sorted, SahTask* blockTasks, uint32_t* ctr)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < kSahWords) {
-		const bool big = n > kBigTask;
-		ctr[i] = i == kSahNodes ? 1u : (i == (big ? kSahNext : kSahBlocks) ? 1u : 0u);
-		if (i == 0) {
-			*(big ? levelTasks : blockTasks) = SahTask{0, n, 0, 0}; // the root
-		}
-	}
 	if (i < n) {
-		const float4 l = lo[i], h = hi[i];
-		cen[i] = make_float4(__fmul_rn(0.5f, __fadd_rn(l.x, h.x)), __fmul_rn(0.5f, __fadd_rn(l.y, h.y)), __fmul_rn(0.5f, __fadd_rn(l.z, h.z)),
-		                     0.0f);
-		idsA[i] = (uint32_t) i;
 		sorted[i] = (uint32_t) i;
 	}
-}
-
-// The level's task count (what the level before counted), the chunk prefix sums of its ranges and their
-// bounds cleared (one block). The kernels of a level read the count from the control words, so levels
-// follow each other without the host.
-__global__ void kSahLevelPrep(const SahTask* __restrict__ tasks, int32_t* chunkBase, uint32_t* bounds, uint32_t* ctr)
-{
-	__shared__ int32_t sWarp[32];
-	__shared__ int32_t sCarry;
-	const int nTasks = (int) ctr[kSahNext];
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		sCarry = 0;
-		ctr[kSahCur] = (uint32_t) nTasks;
-		ctr[kSahNext] = 0u;
+	if (i < kSahWords) {
+		ctr[i] = i == kSahNodes || i == kSahBlocks ? 1u : 0u; // the root
 	}
-	for (int i = threadIdx.x; i < nTasks * 12; i += blockDim.x) {
-		bounds[i] = isMinWord(i % 12) ? kEmptyLo : kEmptyHi;
-	}
-	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	for (int base = 0; base < nTasks; base += blockDim.x) {
-		const int t = base + (int) threadIdx.x;
-		const int v = t < nTasks ? (tasks[t].hi - tasks[t].lo + kChunk - 1) / kChunk : 0;
-		int incl = v;
-		for (int off = 1; off < 32; off <<= 1) {
-			const int u = __shfl_up_sync(0xffffffffu, incl, off);
-			if (lane >= off) {
-				incl += u;
-			}
-		}
-		if (lane == 31) {
-			sWarp[warp] = incl;
-		}
-		__syncthreads();
-		if (warp == 0) {
-			const int nw = blockDim.x / 32;
-			int w = lane < nw ? sWarp[lane] : 0;
-			for (int off = 1; off < 32; off <<= 1) {
-				const int u = __shfl_up_sync(0xffffffffu, w, off);
-				if (lane >= off) {
-					w += u;
-				}
-			}
-			if (lane < nw) {
-				sWarp[lane] = w; // inclusive over warps
-			}
-		}
-		__syncthreads();
-		const int warpBase = warp > 0 ? sWarp[warp - 1] : 0;
-		if (t < nTasks) {
-			chunkBase[t] = sCarry + warpBase + incl - v;
-		}
-		__syncthreads();
-		if (threadIdx.x == 0) {
-			sCarry += sWarp[blockDim.x / 32 - 1];
-		}
-		__syncthreads();
-	}
-	if (threadIdx.x == 0) {
-		chunkBase[nTasks] = sCarry;
-	}
-}
-
-// Range of chunk c: the task whose chunk prefix covers it.
-__device__ __forceinline__ bool chunkRange(const int32_t* chunkBase, const uint32_t* ctr, const SahTask* tasks, int c, int& t, int& start,
-                                           int& end, int& first)
-{
-	const int nTasks = (int) ctr[kSahCur];
-	if (nTasks == 0 || c >= chunkBase[nTasks]) {
-		return false;
-	}
-	int lo = 0, hi = nTasks; // chunkBase[lo] <= c < chunkBase[hi]
-	while (hi - lo > 1) {
-		const int mid = (lo + hi) >> 1;
-		if (chunkBase[mid] <= c) {
-			lo = mid;
-		} else {
-			hi = mid;
-		}
-	}
-	t = lo;
-	first = chunkBase[lo];
-	start = tasks[lo].lo + (c - first) * kChunk;
-	end = min(tasks[lo].hi, start + kChunk);
-	return true;
-}
-
-__device__ __forceinline__ void blockReduceBounds(Bounds12& b, uint32_t (*sRed)[12], uint32_t* out)
-{
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	b.warpReduce();
-	if (lane == 0) {
-#pragma unroll
-		for (int k = 0; k < 12; ++k) {
-			sRed[warp][k] = b.w[k];
-		}
-	}
-	__syncthreads();
-	if (threadIdx.x < 12) {
-		const int k = threadIdx.x;
-		uint32_t v = sRed[0][k];
-		for (int w = 1; w < kWarps; ++w) {
-			v = isMinWord(k) ? min(v, sRed[w][k]) : max(v, sRed[w][k]);
-		}
-		if (isMinWord(k)) {
-			atomicMin(&out[k], v);
-		} else {
-			atomicMax(&out[k], v);
-		}
-	}
-}
-
-__global__ void __launch_bounds__(kThreads) kSahBounds(const SahTask* __restrict__ tasks, const uint32_t* ctr, const int32_t* __restrict__ chunkBase,
-                                                       const uint32_t* __restrict__ ids, const float4* __restrict__ lo,
-                                                       const float4* __restrict__ hi, const float4* __restrict__ cen, uint32_t* bounds,
-                                                       uint32_t* bins)
-{
-	__shared__ uint32_t sRed[kWarps][12];
-	int t, start, end, first;
-	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
-		return;
-	}
-	if ((int) blockIdx.x == first) { // the range's first chunk clears its bins for the binning pass
-		uint32_t* tb = bins + (size_t) t * kTaskBinWords;
-		for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
-			const int w = k % kBinWords;
-			tb[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
-		}
-	}
-	Bounds12 b;
-	b.clear();
-	for (int i = start + (int) threadIdx.x; i < end; i += blockDim.x) {
-		const uint32_t id = ids[i];
-		b.add(lo[id], hi[id], cen[id]);
-	}
-	blockReduceBounds(b, sRed, bounds + (size_t) t * 12);
-}
-
-__global__ void __launch_bounds__(kThreads) kSahBins(const SahTask* __restrict__ tasks, const uint32_t* ctr, const int32_t* __restrict__ chunkBase,
-                                                     const uint32_t* __restrict__ ids, const float4* __restrict__ lo,
-                                                     const float4* __restrict__ hi, const float4* __restrict__ cen,
-                                                     const uint32_t* __restrict__ bounds, uint32_t* bins)
-{
-	__shared__ uint32_t sb[kTaskBinWords];
-	int t, start, end, first;
-	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
-		return;
-	}
-	for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
-		const int w = k % kBinWords;
-		sb[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
-	}
-	const uint32_t* b12 = bounds + (size_t) t * 12;
-	AxisFrame fr[3];
-#pragma unroll
-	for (int a = 0; a < 3; ++a) {
-		fr[a] = axisFrame(b12, a);
-	}
-	__syncthreads();
-	for (int i = start + (int) threadIdx.x; i < end; i += blockDim.x) {
-		const uint32_t id = ids[i];
-		const float4 l = lo[id], h = hi[id], c = cen[id];
-#pragma unroll
-		for (int a = 0; a < 3; ++a) {
-			if (!fr[a].valid) {
-				continue;
-			}
-			uint32_t* bb = sb + (a * kBins + binOf(comp3(c, a), fr[a].cmin, fr[a].scale)) * kBinWords;
-			atomicMin(&bb[0], ordered(l.x));
-			atomicMin(&bb[1], ordered(l.y));
-			atomicMin(&bb[2], ordered(l.z));
-			atomicMax(&bb[3], ordered(h.x));
-			atomicMax(&bb[4], ordered(h.y));
-			atomicMax(&bb[5], ordered(h.z));
-			atomicAdd(&bb[6], 1u);
-		}
-	}
-	__syncthreads();
-	uint32_t* tb = bins + (size_t) t * kTaskBinWords;
-	for (int k = threadIdx.x; k < 3 * kBins; k += blockDim.x) {
-		const uint32_t* bb = sb + k * kBinWords;
-		if (bb[6] == 0u) {
-			continue;
-		}
-		uint32_t* g = tb + k * kBinWords;
-		atomicMin(&g[0], bb[0]);
-		atomicMin(&g[1], bb[1]);
-		atomicMin(&g[2], bb[2]);
-		atomicMax(&g[3], bb[3]);
-		atomicMax(&g[4], bb[4]);
-		atomicMax(&g[5], bb[5]);
-		atomicAdd(&g[6], bb[6]);
-	}
-}
-
-// One warp per range: the split, the node, its children (next level, block phase or leaves).
-__global__ void kSahSplit(const SahTask* __restrict__ tasks, const uint32_t* __restrict__ bounds,
-                          const uint32_t* __restrict__ bins, SahSplit* splits, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
-                          SahTask* next, SahTask* blockTasks, uint32_t* ctr)
-{
-	const int w = (int) ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-	const int lane = threadIdx.x & 31;
-	if (w >= (int) ctr[kSahCur]) {
-		return;
-	}
-	const SahTask tk = tasks[w];
-	const uint32_t* b12 = bounds + (size_t) w * 12;
-	SahSplit s = warpBestSplit(bins + (size_t) w * kTaskBinWords, b12, lane);
-	if (s.axis < 0) {
-		s.nLeft = (tk.lo + tk.hi) / 2 - tk.lo;
-	}
-	if (lane == 0) {
-		splits[w] = s;
-		int32_t left, right;
-		emitNode(tk.node, tk.lo, tk.hi, s.nLeft, b12, bin, rangeFirst, rangeLast, ctr, left, right);
-		const int mid = tk.lo + s.nLeft;
-		const int cl[2] = {left, right};
-		const int r0[2] = {tk.lo, mid}, r1[2] = {mid, tk.hi};
-		for (int c = 0; c < 2; ++c) {
-			const int cnt = r1[c] - r0[c];
-			if (cnt < 2) {
-				continue;
-			}
-			const SahTask child{r0[c], r1[c], cl[c], 0};
-			if (cnt > kBigTask) {
-				next[atomicAdd(&ctr[kSahNext], 1u)] = child;
-			} else {
-				blockTasks[atomicAdd(&ctr[kSahBlocks], 1u)] = child;
-			}
-		}
-	}
-}
-
-__device__ __forceinline__ bool goesLeft(uint32_t id, int pos, const SahTask& tk, const SahSplit& s, const AxisFrame& f,
-                                         const float4* __restrict__ cen)
-{
-	if (s.axis < 0) {
-		return pos < tk.lo + s.nLeft;
-	}
-	return binOf(comp3(cen[id], s.axis), f.cmin, f.scale) < s.bin;
-}
-
-__global__ void __launch_bounds__(kThreads) kSahPartCount(const SahTask* __restrict__ tasks, const uint32_t* ctr,
-                                                          const int32_t* __restrict__ chunkBase, const uint32_t* __restrict__ ids,
-                                                          const float4* __restrict__ cen, const uint32_t* __restrict__ bounds,
-                                                          const SahSplit* __restrict__ splits, int32_t* chunkLeft)
-{
-	__shared__ int sW[kWarps];
-	int t, start, end, first;
-	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
-		return;
-	}
-	const SahTask tk = tasks[t];
-	const SahSplit s = splits[t];
-	const AxisFrame f = s.axis >= 0 ? axisFrame(bounds + (size_t) t * 12, s.axis) : AxisFrame{0.0f, 0.0f, false};
-	int cnt = 0;
-	for (int i = start + (int) threadIdx.x; i < end; i += blockDim.x) {
-		cnt += goesLeft(ids[i], i, tk, s, f, cen) ? 1 : 0;
-	}
-	cnt = __reduce_add_sync(0xffffffffu, cnt);
-	if ((threadIdx.x & 31) == 0) {
-		sW[threadIdx.x >> 5] = cnt;
-	}
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		int sum = 0;
-		for (int w = 0; w < kWarps; ++w) {
-			sum += sW[w];
-		}
-		chunkLeft[blockIdx.x] = sum;
+	if (i == 0) {
+		blockTasks[0] = SahTask{0, n, 0, 0};
 	}
 }
 
@@ -566,67 +273,430 @@ __device__ __forceinline__ int blockExclusiveScan(int v, int* sW, int& total)
 	return before + incl - v;
 }
 
-__global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __restrict__ tasks, uint32_t* ctr,
-                                                            const int32_t* __restrict__ chunkBase, const uint32_t* __restrict__ ids,
-                                                            const float4* __restrict__ cen, const uint32_t* __restrict__ bounds,
-                                                            const SahSplit* __restrict__ splits, const int32_t* __restrict__ chunkLeft,
-                                                            uint32_t* __restrict__ idsOut, uint32_t* __restrict__ sorted)
+// Where nodes go.
+struct NodeSink
 {
-	__shared__ int sW[kWarps];
-	int t, start, end, first;
-	if (!chunkRange(chunkBase, ctr, tasks, blockIdx.x, t, start, end, first)) {
-		return;
-	}
-	const SahTask tk = tasks[t];
-	const SahSplit s = splits[t];
-	const AxisFrame f = s.axis >= 0 ? axisFrame(bounds + (size_t) t * 12, s.axis) : AxisFrame{0.0f, 0.0f, false};
-	// left elements of the range's earlier chunks
-	int before = 0;
-	for (int c = first + (int) threadIdx.x; c < (int) blockIdx.x; c += blockDim.x) {
-		before += chunkLeft[c];
-	}
-	int dummy;
-	before = __reduce_add_sync(0xffffffffu, before);
-	if ((threadIdx.x & 31) == 0) {
-		sW[threadIdx.x >> 5] = before;
-	}
-	__syncthreads();
-	int leftBefore = 0;
-	for (int w = 0; w < kWarps; ++w) {
-		leftBefore += sW[w];
-	}
-	__syncthreads();
-	// this thread's run of kItems consecutive elements
-	const int p0 = start + (int) threadIdx.x * kItems;
-	uint32_t id[kItems];
-	bool fl[kItems];
-	int mine = 0;
-#pragma unroll
-	for (int k = 0; k < kItems; ++k) {
-		const int p = p0 + k;
-		fl[k] = false;
-		id[k] = 0;
-		if (p < end) {
-			id[k] = ids[p];
-			fl[k] = goesLeft(id[k], p, tk, s, f, cen);
-			mine += fl[k] ? 1 : 0;
+	BinNode* bin;
+	int32_t* rangeFirst;
+	int32_t* rangeLast;
+	uint32_t* ctr; // control words, or null (a one-block build: no other block, nobody reads the error word)
+	__device__ __forceinline__ void error() const
+	{
+		if (ctr != nullptr) {
+			atomicExch(&ctr[kSahError], 1u);
 		}
 	}
-	int rank = leftBefore + blockExclusiveScan(mine, sW, dummy);
+	__device__ __forceinline__ void write(int node, int lo, int hi, const uint32_t* b12, int32_t left, int32_t right) const
+	{
+		float4* p = reinterpret_cast<float4*>(bin + node);
+		p[0] = make_float4(unordered(b12[0]), unordered(b12[1]), unordered(b12[2]), __int_as_float(left));
+		p[1] = make_float4(unordered(b12[3]), unordered(b12[4]), unordered(b12[5]), __int_as_float(right));
+		rangeFirst[node] = lo;
+		rangeLast[node] = hi - 1;
+	}
+};
+
+// What a range's warp decides: the split, and the children's places among the next level's ranges (-1:
+// not one of them).
+struct LevelSplit
+{
+	SahSplit split;
+	int32_t child[2];
+};
+
+// Memory of the level loop; pairs are used in turn by the levels.
+struct SahLevels
+{
+	int n;
+	uint32_t *ids[2], *sorted;
+	SahTask *tasks[2], *blockTasks;
+	uint32_t *bounds[2], *bins;
+	int32_t *chunkBase[2], *chunkTask[2]; // first chunk of every range and the chunks; range of every chunk
+	int32_t* chunkLeft;                   // left elements of a chunk
+	LevelSplit* splits;
+	int maxBig;
+	BinNode* bin;
+	int32_t *rangeFirst, *rangeLast;
+	uint32_t* ctr;
+};
+
+// Adds a block's bounds to those of up to two ranges, null for none (every thread calls it; ends with a
+// barrier).
+template<int RANGES>
+__device__ __forceinline__ void blockAddBounds(Bounds12 (&b)[RANGES], uint32_t (*sRed)[kWarps][12], uint32_t* const (&out)[RANGES])
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-	for (int k = 0; k < kItems; ++k) {
-		const int p = p0 + k;
-		if (p < end) {
-			// left: lo + (left elements before p); right: lo + nLeft + (right elements before p)
-			const int dst = fl[k] ? tk.lo + rank : tk.lo + s.nLeft + (p - tk.lo - rank);
-			rank += fl[k] ? 1 : 0;
-			if (dst < tk.lo || dst >= tk.hi) {
-				atomicExch(&ctr[kSahError], 1u);
-				continue;
+	for (int r = 0; r < RANGES; ++r) {
+		if (out[r] == nullptr) {
+			continue;
+		}
+		b[r].warpReduce();
+		if (lane == 0) {
+#pragma unroll
+			for (int k = 0; k < 12; ++k) {
+				sRed[r][warp][k] = b[r].w[k];
 			}
-			idsOut[dst] = id[k];
-			sorted[dst] = id[k];
 		}
+	}
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r < RANGES; ++r) {
+		const int k = (int) threadIdx.x - 32 * r; // one warp each
+		if (out[r] != nullptr && k >= 0 && k < 12) {
+			uint32_t v = sRed[r][0][k];
+#pragma unroll
+			for (int w = 1; w < kWarps; ++w) {
+				v = isMinWord(k) ? min(v, sRed[r][w][k]) : max(v, sRed[r][w][k]);
+			}
+			if (isMinWord(k)) {
+				atomicMin(&out[r][k], v);
+			} else {
+				atomicMax(&out[r][k], v);
+			}
+		}
+	}
+	__syncthreads();
+}
+
+__device__ __forceinline__ float4 centroidOf(const float4& l, const float4& h)
+{
+	return make_float4(__fmul_rn(0.5f, __fadd_rn(l.x, h.x)), __fmul_rn(0.5f, __fadd_rn(l.y, h.y)), __fmul_rn(0.5f, __fadd_rn(l.z, h.z)), 0.0f);
+}
+
+__device__ __forceinline__ void addToBins(uint32_t* sb, const float4& l, const float4& h, const AxisFrame (&fr)[3])
+{
+	const float4 c = centroidOf(l, h);
+#pragma unroll
+	for (int a = 0; a < 3; ++a) {
+		if (!fr[a].valid) {
+			continue;
+		}
+		uint32_t* bb = sb + (a * kBins + binOf(comp3(c, a), fr[a].cmin, fr[a].scale)) * kBinWords;
+		atomicMin(&bb[0], ordered(l.x));
+		atomicMin(&bb[1], ordered(l.y));
+		atomicMin(&bb[2], ordered(l.z));
+		atomicMax(&bb[3], ordered(h.x));
+		atomicMax(&bb[4], ordered(h.y));
+		atomicMax(&bb[5], ordered(h.z));
+		atomicAdd(&bb[6], 1u);
+	}
+}
+
+__device__ __forceinline__ void clearBins(uint32_t* bins, int first, int step, int words = kTaskBinWords)
+{
+	for (int k = first; k < words; k += step) {
+		const int w = k % kBinWords;
+		bins[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
+	}
+}
+
+// A block's bins of a range added to the range's; the block's are empty afterwards.
+__device__ __forceinline__ void flushBins(uint32_t* sb, uint32_t* tb)
+{
+	for (int k = threadIdx.x; k < 3 * kBins; k += kThreads) {
+		uint32_t* bb = sb + k * kBinWords;
+		if (bb[6] == 0u) {
+			continue;
+		}
+		uint32_t* g = tb + k * kBinWords;
+		atomicMin(&g[0], bb[0]);
+		atomicMin(&g[1], bb[1]);
+		atomicMin(&g[2], bb[2]);
+		atomicMax(&g[3], bb[3]);
+		atomicMax(&g[4], bb[4]);
+		atomicMax(&g[5], bb[5]);
+		atomicAdd(&g[6], bb[6]);
+		clearBins(bb, 0, 1, kBinWords);
+	}
+}
+
+// All levels in one cooperative launch. A level has three phases with a grid barrier after each:
+//  1. one warp per range: the split from the range's bins, its node, its children;
+//  2. by chunks of kChunk elements: how many go left, and the children's bounds;
+//  3. by chunks: the elements to their places, and into their child's bins.
+// A block works through consecutive chunks and hands its bounds and bins on when the range changes.
+// What bounds a level of a mesh of 100,000 triangles is not its data (4 MB, in L2) but the phases after
+// each other: as six launches (chunk table, bounds, bins, split, count, scatter) a level took 27 us, and
+// the host had to guess how many levels to queue; here it takes 17 (split 3.2, count 3, scatter 6,
+// barriers 1 to 2 each), 182 us in all for 131,072 triangles against 245.
+__global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restrict__ lo, const float4* __restrict__ hi, SahLevels L)
+{
+	__shared__ uint32_t sBins[2][kTaskBinWords];
+	__shared__ uint32_t sRed[2][kWarps][12];
+	__shared__ int sW[kWarps];
+	cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int thread = (int) (blockIdx.x * kThreads + threadIdx.x), threads = (int) (gridDim.x * kThreads);
+	clearBins(sBins[0], (int) threadIdx.x, kThreads, 2 * kTaskBinWords);
+
+	// The root: its order, bounds and bins.
+	const int rootChunks = (L.n + kChunk - 1) / kChunk;
+	if (blockIdx.x == 0) {
+		if (threadIdx.x < kSahWords) {
+			L.ctr[threadIdx.x] = threadIdx.x == kSahNodes || threadIdx.x == kSahLevel ? 1u : 0u;
+		}
+		if (threadIdx.x < 12) {
+			L.bounds[0][threadIdx.x] = isMinWord((int) threadIdx.x) ? kEmptyLo : kEmptyHi;
+		}
+		if (threadIdx.x == 0) {
+			L.tasks[0][0] = SahTask{0, L.n, 0, 0};
+			L.chunkBase[0][0] = 0;
+			L.chunkBase[0][1] = rootChunks;
+		}
+	}
+	clearBins(L.bins, thread, threads, L.maxBig * kTaskBinWords);
+	Bounds12 b[1];
+	b[0].clear();
+	for (int i = thread; i < L.n; i += threads) {
+		if (i < rootChunks) {
+			L.chunkTask[0][i] = 0;
+		}
+		L.ids[0][i] = (uint32_t) i;
+		const float4 l = lo[i], h = hi[i];
+		b[0].add(l, h, centroidOf(l, h));
+	}
+	grid.sync();
+	blockAddBounds<1>(b, sRed, {L.bounds[0]});
+	grid.sync();
+	{
+		AxisFrame fr[3];
+#pragma unroll
+		for (int a = 0; a < 3; ++a) {
+			fr[a] = axisFrame(L.bounds[0], a);
+		}
+		for (int i = thread; i < L.n; i += threads) {
+			addToBins(sBins[0], lo[i], hi[i], fr);
+		}
+		__syncthreads();
+		flushBins(sBins[0], L.bins);
+	}
+	grid.sync();
+
+	for (int level = 0;; ++level) {
+		const int now = level & 1, then = now ^ 1;
+		SahTask* const tasks = L.tasks[now];
+		SahTask* const next = L.tasks[then];
+		uint32_t* const bounds = L.bounds[now];
+		uint32_t* const childBounds = L.bounds[then];
+		const uint32_t* const ids = L.ids[now];
+		const int32_t* const chunkBase = L.chunkBase[now];
+		// Counts of three levels in turn: this one's, the next one's, and one that nobody reads now.
+		uint32_t* const counts = L.ctr + kSahLevel;
+		const int nTasks = (int) *(volatile uint32_t*) &counts[level % 3];
+		if (nTasks == 0) {
+			break;
+		}
+		if (thread == 0) {
+			counts[(level + 2) % 3] = 0u;
+		}
+		for (int w = thread >> 5; w < nTasks; w += threads >> 5) {
+			const SahTask tk = tasks[w];
+			const uint32_t* b12 = bounds + (size_t) w * 12;
+			uint32_t* tb = L.bins + (size_t) w * kTaskBinWords;
+			LevelSplit s{warpBestSplit(tb, b12, lane), {-1, -1}};
+			if (s.split.axis < 0) {
+				s.split.nLeft = (tk.lo + tk.hi) / 2 - tk.lo;
+			}
+			__syncwarp();
+			clearBins(tb, lane, 32); // for the next level's range of this number
+			if (lane == 0) {
+				const int cut[3] = {tk.lo, tk.lo + s.split.nLeft, tk.hi};
+				uint32_t inner[2], big[2], block[2];
+#pragma unroll
+				for (int c = 0; c < 2; ++c) {
+					const int cnt = cut[c + 1] - cut[c];
+					inner[c] = cnt > 1 ? 1u : 0u;
+					big[c] = cnt > kBigTask ? 1u : 0u;
+					block[c] = inner[c] - big[c];
+				}
+				uint32_t node = atomicAdd(&L.ctr[kSahNodes], inner[0] + inner[1]);
+				uint32_t slot = atomicAdd(&counts[(level + 1) % 3], big[0] + big[1]);
+				uint32_t blockSlot = atomicAdd(&L.ctr[kSahBlocks], block[0] + block[1]);
+				int32_t child[2];
+#pragma unroll
+				for (int c = 0; c < 2; ++c) {
+					child[c] = inner[c] != 0u ? (int32_t) node : ~cut[c];
+					const SahTask range{cut[c], cut[c + 1], child[c], 0};
+					if (big[c] != 0u) {
+						s.child[c] = (int32_t) slot;
+						next[slot] = range;
+						uint32_t* cb = childBounds + (size_t) slot * 12;
+#pragma unroll
+						for (int k = 0; k < 12; ++k) {
+							cb[k] = isMinWord(k) ? kEmptyLo : kEmptyHi;
+						}
+					} else if (block[c] != 0u) {
+						L.blockTasks[blockSlot] = range;
+					}
+					node += inner[c];
+					slot += big[c];
+					blockSlot += block[c];
+				}
+				L.splits[w] = s;
+				NodeSink{L.bin, L.rangeFirst, L.rangeLast, L.ctr}.write(tk.node, tk.lo, tk.hi, b12, child[0], child[1]);
+			}
+			__syncwarp();
+		}
+		grid.sync();
+
+		const int nNext = (int) *(volatile uint32_t*) &counts[(level + 1) % 3];
+		const int nChunks = chunkBase[nTasks];
+		const int run = (nChunks + (int) gridDim.x - 1) / (int) gridDim.x;
+		const int c0 = min((int) blockIdx.x * run, nChunks), c1 = min(c0 + run, nChunks);
+		const int t0 = c0 < c1 ? L.chunkTask[now][c0] : 0;
+		{
+			Bounds12 side[2];
+			side[0].clear();
+			side[1].clear();
+			for (int c = c0, t = t0; c < c1; ++c) {
+				const SahTask tk = tasks[t];
+				const LevelSplit s = L.splits[t];
+				const AxisFrame f = s.split.axis >= 0 ? axisFrame(bounds + (size_t) t * 12, s.split.axis) : AxisFrame{0.0f, 0.0f, false};
+				const int start = tk.lo + (c - chunkBase[t]) * kChunk, end = min(tk.hi, start + kChunk);
+				int cnt = 0;
+#pragma unroll
+				for (int q = 0; q < kItems; ++q) {
+					const int i = start + q * kThreads + (int) threadIdx.x;
+					if (i < end) {
+						const uint32_t id = ids[i];
+						const float4 l = lo[id], h = hi[id], cen = centroidOf(l, h);
+						const bool left = s.split.axis < 0 ? i < tk.lo + s.split.nLeft
+						                                   : binOf(comp3(cen, s.split.axis), f.cmin, f.scale) < s.split.bin;
+						cnt += left ? 1 : 0;
+						if (left) {
+							side[0].add(l, h, cen);
+						} else {
+							side[1].add(l, h, cen);
+						}
+					}
+				}
+				cnt = __reduce_add_sync(0xffffffffu, cnt);
+				if (lane == 0) {
+					sW[warp] = cnt;
+				}
+				__syncthreads();
+				if (threadIdx.x == 0) {
+					int sum = 0;
+					for (int w = 0; w < kWarps; ++w) {
+						sum += sW[w];
+					}
+					L.chunkLeft[c] = sum;
+				}
+				__syncthreads();
+				if (c + 1 == c1 || c + 1 == chunkBase[t + 1]) { // the range ends here
+					uint32_t* const to[2] = {s.child[0] >= 0 ? childBounds + (size_t) s.child[0] * 12 : nullptr,
+					                         s.child[1] >= 0 ? childBounds + (size_t) s.child[1] * 12 : nullptr};
+					blockAddBounds<2>(side, sRed, to);
+					side[0].clear();
+					side[1].clear();
+					++t;
+				}
+			}
+		}
+		if (blockIdx.x == gridDim.x - 1) { // the next level's chunk table
+			int32_t* base = L.chunkBase[then];
+			int carry = 0;
+			for (int first = 0; first < nNext; first += kThreads) {
+				const int t = first + (int) threadIdx.x;
+				const int v = t < nNext ? (next[t].hi - next[t].lo + kChunk - 1) / kChunk : 0;
+				int total;
+				const int before = blockExclusiveScan(v, sW, total);
+				if (t < nNext) {
+					base[t] = carry + before;
+					for (int k = 0; k < v; ++k) {
+						L.chunkTask[then][carry + before + k] = t;
+					}
+				}
+				carry += total;
+			}
+			if (threadIdx.x == 0) {
+				base[nNext] = carry;
+			}
+		}
+		grid.sync();
+
+		AxisFrame fr[2][3];
+		for (int c = c0, t = t0; c < c1; ++c) {
+			const SahTask tk = tasks[t];
+			const LevelSplit s = L.splits[t];
+			const AxisFrame f = s.split.axis >= 0 ? axisFrame(bounds + (size_t) t * 12, s.split.axis) : AxisFrame{0.0f, 0.0f, false};
+			if (c == c0 || c == chunkBase[t]) {
+#pragma unroll
+				for (int q = 0; q < 2; ++q) {
+#pragma unroll
+					for (int a = 0; a < 3; ++a) {
+						fr[q][a] = s.child[q] >= 0 ? axisFrame(childBounds + (size_t) s.child[q] * 12, a) : AxisFrame{0.0f, 0.0f, false};
+					}
+				}
+			}
+			const int start = tk.lo + (c - chunkBase[t]) * kChunk, end = min(tk.hi, start + kChunk);
+			// left elements of the range's earlier chunks
+			int before = 0;
+			for (int k = chunkBase[t] + (int) threadIdx.x; k < c; k += kThreads) {
+				before += L.chunkLeft[k];
+			}
+			int leftBefore, total;
+			(void) blockExclusiveScan(before, sW, leftBefore);
+			// this thread's run of kItems consecutive elements
+			const int p0 = start + (int) threadIdx.x * kItems;
+			uint32_t id[kItems];
+			float4 l[kItems], h[kItems];
+			bool left[kItems];
+			int mine = 0;
+#pragma unroll
+			for (int q = 0; q < kItems; ++q) {
+				const int p = p0 + q;
+				left[q] = false;
+				if (p < end) {
+					id[q] = ids[p];
+					l[q] = lo[id[q]];
+					h[q] = hi[id[q]];
+					left[q] = s.split.axis < 0 ? p < tk.lo + s.split.nLeft
+					                           : binOf(comp3(centroidOf(l[q], h[q]), s.split.axis), f.cmin, f.scale) < s.split.bin;
+					mine += left[q] ? 1 : 0;
+				}
+			}
+			int rank = leftBefore + blockExclusiveScan(mine, sW, total);
+#pragma unroll
+			for (int q = 0; q < kItems; ++q) {
+				const int p = p0 + q;
+				if (p < end) {
+					// left: lo + (left elements before p); right: lo + nLeft + (right elements before p)
+					const int dst = left[q] ? tk.lo + rank : tk.lo + s.split.nLeft + (p - tk.lo - rank);
+					rank += left[q] ? 1 : 0;
+					if (dst < tk.lo || dst >= tk.hi) {
+						atomicExch(&L.ctr[kSahError], 1u);
+						continue;
+					}
+					if (s.child[left[q] ? 0 : 1] >= 0) {
+						L.ids[then][dst] = id[q];
+						if (left[q]) {
+							addToBins(sBins[0], l[q], h[q], fr[0]);
+						} else {
+							addToBins(sBins[1], l[q], h[q], fr[1]);
+						}
+					} else {
+						L.sorted[dst] = id[q];
+					}
+				}
+			}
+			if (c + 1 == c1 || c + 1 == chunkBase[t + 1]) { // the range ends here
+				__syncthreads();
+#pragma unroll
+				for (int q = 0; q < 2; ++q) {
+					if (s.child[q] >= 0) {
+						flushBins(sBins[q], L.bins + (size_t) s.child[q] * kTaskBinWords);
+					}
+				}
+				__syncthreads();
+				++t;
+			}
+		}
+		if (nNext == 0) {
+			break; // the same in every block
+		}
+		grid.sync();
 	}
 }
 
@@ -638,21 +708,22 @@ __global__ void __launch_bounds__(kThreads) kSahPartScatter(const SahTask* __res
 //  * ranges up to 32: one warp each, one element per lane, all subranges of a depth at once (smallBuild).
 // What bounds a block is the chain of splits below each other, so what matters is that splits which do
 // not depend on each other run together. With every range above 32 split by the whole block in turn and
-// every subrange of a small one split alone, the 131,072-triangle mesh took 885 us here, 94 instances 58.
-constexpr int kBlockThreads = 512;
-constexpr int kBlockGrid = 152; // one block per SM, by shared memory
-constexpr int kBlockWarps = kBlockThreads / 32;
+// every subrange of a small one split alone, the ranges of 131,072 triangles took 885 us, 94 instances 58;
+// side by side 255 (ranges of up to 2,048), 141 now; 94 instances 31.
 constexpr int kMidTask = 256;
 
+template<int CAPACITY, int THREADS>
 struct BlockShared
 {
-	float box[6][kBigTask];                        // by local element: lo xyz, hi xyz
-	uint32_t gid[kBigTask];                        // by local element: primitive
-	uint16_t ids[kBigTask], tmp[kBigTask];         // local elements in sorted order
+	static constexpr int kBlockThreads = THREADS, kBlockWarps = THREADS / 32;
+	static constexpr int kMaxMid = CAPACITY / (kSmallTask + 1) + 1, kMaxSmall = CAPACITY / 2, kMaxStack = CAPACITY / (kMidTask + 1) + 1;
+	float box[6][CAPACITY];                        // by local element: lo xyz, hi xyz
+	uint32_t gid[CAPACITY];                        // by local element: primitive
+	uint16_t ids[CAPACITY], tmp[CAPACITY];         // local elements in sorted order
 	uint32_t bins[kBlockWarps][kTaskBinWords];     // per warp; the first also for whole-block splits
-	int4 stack[16];                                // ranges above kMidTask: disjoint, at most kBigTask / 257
-	int4 mid[2][kBigTask / (kSmallTask + 1) + 1];  // ranges of 33..kMidTask of this depth and the next
-	int4 small[kBigTask / 2];                      // ranges of 2..32
+	int4 stack[kMaxStack];                         // ranges above kMidTask, disjoint
+	int4 mid[2][kMaxMid];                          // ranges of 33..kMidTask of this depth and the next
+	int4 small[kMaxSmall];                         // ranges of 2..32
 	uint32_t red[kBlockWarps][12];
 	uint32_t bounds[12];
 	int scan[kBlockWarps];
@@ -692,40 +763,10 @@ struct BlockShared
 	}
 };
 
-// Where a block's nodes go.
-struct NodeSink
-{
-	BinNode* bin;
-	int32_t* rangeFirst;
-	int32_t* rangeLast;
-	uint32_t* ctr; // control words, or null (a one-block build: no other block, nobody reads the error word)
-	__device__ __forceinline__ void error() const
-	{
-		if (ctr != nullptr) {
-			atomicExch(&ctr[kSahError], 1u);
-		}
-	}
-	__device__ __forceinline__ void write(int node, int lo, int hi, const uint32_t* b12, int32_t left, int32_t right) const
-	{
-		float4* p = reinterpret_cast<float4*>(bin + node);
-		p[0] = make_float4(unordered(b12[0]), unordered(b12[1]), unordered(b12[2]), __int_as_float(left));
-		p[1] = make_float4(unordered(b12[3]), unordered(b12[4]), unordered(b12[5]), __int_as_float(right));
-		rangeFirst[node] = lo;
-		rangeLast[node] = hi - 1;
-	}
-};
-
-__device__ __forceinline__ void clearBins(uint32_t* bins, int first, int step)
-{
-	for (int k = first; k < kTaskBinWords; k += step) {
-		const int w = k % kBinWords;
-		bins[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
-	}
-}
-
 // One thread: the node of range [a, b) split after nLeft elements, and its children queued by size.
 // Positions are the block's; `base` is the block's first sorted position.
-__device__ __forceinline__ void emitRange(BlockShared& S, int a, int b, int node, int nLeft, const uint32_t* b12, int base, int midList,
+template<class SHARED>
+__device__ __forceinline__ void emitRange(SHARED& S, int a, int b, int node, int nLeft, const uint32_t* b12, int base, int midList,
                                           const NodeSink& out)
 {
 	const int cut[3] = {a, a + nLeft, b};
@@ -740,21 +781,21 @@ __device__ __forceinline__ void emitRange(BlockShared& S, int a, int b, int node
 		const int n = cut[q + 1] - cut[q];
 		const int4 r = make_int4(cut[q], cut[q + 1], child[q], 0);
 		if (n > kMidTask) {
-			if (S.top < 16) { // whole-block splits only: no other thread pushes
+			if (S.top < S.kMaxStack) { // whole-block splits only: no other thread pushes
 				S.stack[S.top++] = r;
 			} else {
 				out.error();
 			}
 		} else if (n > kSmallTask) {
 			const int k = atomicAdd(&S.nMid[midList], 1);
-			if (k <= kBigTask / (kSmallTask + 1)) {
+			if (k < S.kMaxMid) {
 				S.mid[midList][k] = r;
 			} else {
 				out.error();
 			}
 		} else if (n >= 2) {
 			const int k = atomicAdd(&S.nSmall, 1);
-			if (k < kBigTask / 2) {
+			if (k < S.kMaxSmall) {
 				S.small[k] = r;
 			} else {
 				out.error();
@@ -764,7 +805,8 @@ __device__ __forceinline__ void emitRange(BlockShared& S, int a, int b, int node
 }
 
 // A range of 33..kMidTask elements split by one warp.
-__device__ void warpSplit(BlockShared& S, const int4 range, int base, int midList, const NodeSink& out)
+template<class SHARED>
+__device__ void warpSplit(SHARED& S, const int4 range, int base, int midList, const NodeSink& out)
 {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int a = range.x, b = range.y;
@@ -824,7 +866,8 @@ __device__ void warpSplit(BlockShared& S, const int4 range, int base, int midLis
 // of a split (the splits between two neighbouring elements' bins are the same split; the host takes the
 // first, after the left one's bin) and gathers both sides' boxes from its subrange, element by element,
 // along each axis; the best of the subrange's candidates, in the host's order, is its split.
-__device__ void smallBuild(BlockShared& S, const int4 range, int base, const NodeSink& out)
+template<class SHARED>
+__device__ void smallBuild(SHARED& S, const int4 range, int base, const NodeSink& out)
 {
 	constexpr uint32_t kAll = 0xffffffffu;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -849,7 +892,7 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 		if (longest == 0) {
 			break;
 		}
-		// Bounds of the subrange: every lane goes once around it.
+		// Bounds of the subrange: combined towards its last lane, which then tells the others.
 		uint32_t b12[12];
 #pragma unroll
 		for (int k = 0; k < 6; ++k) {
@@ -859,21 +902,19 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 		for (int k = 0; k < 3; ++k) {
 			b12[6 + k] = b12[9 + k] = ordered(c[k]);
 		}
-		int j = lane;
-		for (int k = 1; k < longest; ++k) {
-			j = j + 1 < y ? j + 1 : x;
-			const int src = active ? j : lane; // once around: further turns meet the same elements again
+		for (int off = 1; off < longest; off <<= 1) {
+			const bool mine = lane - off >= x;
 #pragma unroll
-			for (int q = 0; q < 6; ++q) {
-				const uint32_t v = __shfl_sync(kAll, w[q], src);
-				b12[q] = q < 3 ? min(b12[q], v) : max(b12[q], v);
+			for (int k = 0; k < 12; ++k) {
+				const uint32_t v = __shfl_up_sync(kAll, b12[k], off);
+				const uint32_t u = isMinWord(k) ? min(b12[k], v) : max(b12[k], v);
+				b12[k] = mine ? u : b12[k];
 			}
+		}
+		const int last = active ? y - 1 : lane;
 #pragma unroll
-			for (int q = 0; q < 3; ++q) {
-				const uint32_t v = ordered(__shfl_sync(kAll, c[q], src));
-				b12[6 + q] = min(b12[6 + q], v);
-				b12[9 + q] = max(b12[9 + q], v);
-			}
+		for (int k = 0; k < 12; ++k) {
+			b12[k] = __shfl_sync(kAll, b12[k], last);
 		}
 		uint32_t myBin[3], packed = 0;
 		bool valid[3];
@@ -895,7 +936,7 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 				R[ax][q] = q < 3 ? kEmptyLo : kEmptyHi;
 			}
 		}
-		j = lane;
+		int j = lane;
 		for (int k = 1; k < longest; ++k) {
 			j = j + 1 < y ? j + 1 : x;
 			const int src = active ? j : lane;
@@ -912,10 +953,11 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 				lc[ax] += l && counts ? 1 : 0;
 #pragma unroll
 				for (int q = 0; q < 6; ++q) {
-					const uint32_t empty = q < 3 ? kEmptyLo : kEmptyHi;
-					const uint32_t vl = l ? v[q] : empty, vr = l ? empty : v[q];
-					L[ax][q] = q < 3 ? min(L[ax][q], vl) : max(L[ax][q], vl);
-					R[ax][q] = q < 3 ? min(R[ax][q], vr) : max(R[ax][q], vr);
+					if (l) {
+						L[ax][q] = q < 3 ? min(L[ax][q], v[q]) : max(L[ax][q], v[q]);
+					} else {
+						R[ax][q] = q < 3 ? min(R[ax][q], v[q]) : max(R[ax][q], v[q]);
+					}
 				}
 			}
 		}
@@ -939,20 +981,16 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 			}
 		}
 		__syncwarp();
-		// The best of the subrange.
-		const float mineCost = bestCost;
-		const uint32_t mineKey = bestKey;
-		j = lane;
-		for (int k = 1; k < longest; ++k) {
-			j = j + 1 < y ? j + 1 : x;
-			const int src = active ? j : lane;
-			const float oc = __shfl_sync(kAll, mineCost, src);
-			const uint32_t ok = __shfl_sync(kAll, mineKey, src);
-			if (oc < bestCost || (oc == bestCost && ok < bestKey)) {
+		// The best of the subrange, as its bounds.
+		for (int off = 1; off < longest; off <<= 1) {
+			const float oc = __shfl_up_sync(kAll, bestCost, off);
+			const uint32_t ok = __shfl_up_sync(kAll, bestKey, off);
+			if (lane - off >= x && (oc < bestCost || (oc == bestCost && ok < bestKey))) {
 				bestCost = oc;
 				bestKey = ok;
 			}
 		}
+		bestKey = __shfl_sync(kAll, bestKey, last);
 		const bool middle = bestKey == 0xffffffffu;
 		const int nLeft = middle ? len / 2 : (int) (bestKey & 0xffu);
 		const uint32_t key = bestKey >> 8;
@@ -1011,8 +1049,9 @@ __device__ void smallBuild(BlockShared& S, const int4 range, int base, const Nod
 	__syncwarp();
 }
 
-// One range of at most kBigTask primitives, by the whole block; see kSahBlock.
-__device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, const SahTask* tasks, const InstanceRec* inst, float4* gLo,
+// One range of at most the capacity, by the whole block; see kSahBlock.
+template<class SHARED>
+__device__ __forceinline__ void buildRange(SHARED& S, const SahTask task, const SahTask* tasks, const InstanceRec* inst, float4* gLo,
                                            float4* gHi, uint32_t* sorted, const NodeSink& out)
 {
 	const int base = task.lo, cnt = task.hi - task.lo;
@@ -1079,12 +1118,12 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 				S.red[warp][k] = bd.w[k];
 			}
 		}
-		clearBins(S.bins[0], (int) threadIdx.x, kBlockThreads);
+		clearBins(S.bins[0], (int) threadIdx.x, S.kBlockThreads);
 		__syncthreads();
 		if (threadIdx.x < 12) {
 			const int k = threadIdx.x;
 			uint32_t v = S.red[0][k];
-			for (int w = 1; w < kBlockWarps; ++w) {
+			for (int w = 1; w < S.kBlockWarps; ++w) {
 				v = isMinWord(k) ? min(v, S.red[w][k]) : max(v, S.red[w][k]);
 			}
 			S.bounds[k] = v;
@@ -1112,7 +1151,7 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 		__syncthreads();
 		const SahSplit s = S.split;
 		// stable partition of [a, b): runs of consecutive elements per thread
-		const int per = (b - a + kBlockThreads - 1) / kBlockThreads;
+		const int per = (b - a + S.kBlockThreads - 1) / S.kBlockThreads;
 		const int p0 = a + (int) threadIdx.x * per;
 		const int p1 = min(b, p0 + per);
 		const AxisFrame f = s.axis >= 0 ? (s.axis == 0 ? fr[0] : (s.axis == 1 ? fr[1] : fr[2])) : AxisFrame{0.0f, 0.0f, false};
@@ -1121,7 +1160,7 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 			mine += S.left(S.ids[p], p, a, s, f) ? 1 : 0;
 		}
 		int total;
-		int rank = blockExclusiveScan<kBlockWarps>(mine, S.scan, total);
+		int rank = blockExclusiveScan<SHARED::kBlockWarps>(mine, S.scan, total);
 		for (int p = p0; p < p1; ++p) {
 			const uint16_t e = S.ids[p];
 			const bool gl = S.left(e, p, a, s, f);
@@ -1144,11 +1183,11 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 	}
 	// ranges of 33..kMidTask, depth by depth
 	for (int list = 0;; list ^= 1) {
-		const int m = min(S.nMid[list], kBigTask / (kSmallTask + 1) + 1);
+		const int m = min(S.nMid[list], S.kMaxMid);
 		if (m == 0) {
 			break;
 		}
-		for (int k = warp; k < m; k += kBlockWarps) {
+		for (int k = warp; k < m; k += S.kBlockWarps) {
 			warpSplit(S, S.mid[list][k], base, list ^ 1, out);
 		}
 		__syncthreads();
@@ -1158,7 +1197,7 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 		__syncthreads();
 	}
 	// ranges of up to 32 elements
-	for (int k = warp; k < min(S.nSmall, kBigTask / 2); k += kBlockWarps) {
+	for (int k = warp; k < min(S.nSmall, S.kMaxSmall); k += S.kBlockWarps) {
 		smallBuild(S, S.small[k], base, out);
 	}
 	__syncthreads();
@@ -1169,17 +1208,15 @@ __device__ __forceinline__ void buildRange(BlockShared& S, const SahTask task, c
 
 // tasks: ranges that the blocks take in turn, or null for a one-block build of primitives [0, n) in the given order. Boxes
 // come from gLo / gHi, or, for a TLAS, from the instance records, and are then stored there for the collapse.
-__global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __restrict__ tasks, int n, const InstanceRec* __restrict__ inst,
+template<class SHARED>
+__global__ void __launch_bounds__(SHARED::kBlockThreads) kSahBlock(const SahTask* __restrict__ tasks, int n, const InstanceRec* __restrict__ inst,
                                                            float4* gLo, float4* gHi, uint32_t* __restrict__ sorted, NodeSink out)
 {
 	extern __shared__ __align__(16) uint8_t smem[];
-	BlockShared& S = *reinterpret_cast<BlockShared*>(smem);
+	SHARED& S = *reinterpret_cast<SHARED*>(smem);
 	if (tasks == nullptr) {
 		buildRange(S, SahTask{0, n, 0, 0}, nullptr, inst, gLo, gHi, sorted, out);
 		return;
-	}
-	if (out.ctr[kSahNext] != 0u) {
-		return; // the levels are not done: nothing is taken yet
 	}
 	const uint32_t count = out.ctr[kSahBlocks];
 	for (;;) {
@@ -1196,6 +1233,21 @@ __global__ void __launch_bounds__(kBlockThreads) kSahBlock(const SahTask* __rest
 	}
 }
 
+// Ranges of a mesh, several blocks per SM; and the one block of a TLAS.
+using MeshShared = BlockShared<kBigTask, kMeshThreads>;
+using TlasShared = BlockShared<kSahSmallMax, 512>;
+
+// Blocks of a kernel that fit the device at once.
+template<class Kernel>
+int residentBlocks(Kernel kernel, int threads, size_t shared)
+{
+	int dev = 0, sms = 0, perSm = 0;
+	RGL_SAH_OK(cudaGetDevice(&dev));
+	RGL_SAH_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	RGL_SAH_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, shared));
+	return sms * perSm;
+}
+
 inline int blocksFor(int n, int b) { return (n + b - 1) / b; }
 
 } // namespace
@@ -1203,74 +1255,63 @@ inline int blocksFor(int n, int b) { return (n + b - 1) / b; }
 void prepareSahBlock()
 {
 	static const bool done = [] {
-		RGL_SAH_OK(cudaFuncSetAttribute(kSahBlock, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(BlockShared)));
+		RGL_SAH_OK(cudaFuncSetAttribute(kSahBlock<TlasShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(TlasShared)));
 		return true;
 	}();
 	(void) done;
 }
 
-SahTopology::SahTopology(const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
-                         uint32_t* sortedIds, cudaStream_t stream)
-    : lo_(lo), hi_(hi), n_(n), bin_(bin), rangeFirst_(rangeFirst), rangeLast_(rangeLast), sorted_(sortedIds), stream_(stream), scratch_(stream)
+const uint32_t* enqueueSahTopology(BuildScratch& scratch, const float4* lo, const float4* hi, int n, BinNode* bin, int32_t* rangeFirst,
+                                   int32_t* rangeLast, uint32_t* sortedIds, cudaStream_t stream)
 {
-	maxBig_ = n / (kBigTask + 1) + 1;       // disjoint ranges above kBigTask
-	const int maxBlock = n / 2 + 1;          // disjoint ranges of at least 2
-	const int maxChunks = n / kChunk + maxBig_ + 1;
-	scratch_.carve([&](BuildScratch::Carver& place) {
-		place(cen_, n);
-		place(idsCur_, n);
-		place(idsNext_, n);
-		place(cur_, maxBig_);
-		place(next_, maxBig_);
-		place(blockTasks_, maxBlock);
-		place(splits_, maxBig_);
-		place(bounds_, (size_t) maxBig_ * 12);
-		place(bins_, (size_t) maxBig_ * kTaskBinWords);
-		place(chunkBase_, maxBig_ + 1);
-		place(chunkLeft_, maxChunks);
-		place(ctr_, kSahWords);
-	});
-	kSahInit<<<blocksFor(n, 256), 256, 0, stream>>>(lo, hi, n, cen_, idsCur_, sortedIds, cur_, blockTasks_, ctr_);
-	countLaunch();
 	if (n < 2) {
-		ctr_ = nullptr;
-		return;
+		RGL_SAH_OK(cudaMemsetAsync(sortedIds, 0, sizeof(uint32_t), stream));
+		return nullptr;
 	}
-	// As many levels as an even tree takes and two more (a level with nothing left costs six empty
-	// launches, about 12 us; a look at what is left about 20).
-	while (n > kBigTask && (kBigTask << levels_) < n) {
-		++levels_;
+	SahLevels L{};
+	L.n = n;
+	L.maxBig = n / (kBigTask + 1) + 1; // disjoint ranges above kBigTask
+	const int maxChunks = n / kChunk + L.maxBig + 1;
+	scratch.carve([&](BuildScratch::Carver& place) {
+		place(L.ctr, kSahWords);
+		place(L.blockTasks, n / 2 + 1); // disjoint ranges of at least 2
+		if (n <= kBigTask) {
+			return;
+		}
+		for (int k = 0; k < 2; ++k) {
+			place(L.ids[k], n);
+			place(L.tasks[k], L.maxBig);
+			place(L.bounds[k], (size_t) L.maxBig * 12);
+			place(L.chunkBase[k], L.maxBig + 1);
+			place(L.chunkTask[k], maxChunks);
+		}
+		place(L.bins, (size_t) L.maxBig * kTaskBinWords);
+		place(L.chunkLeft, maxChunks);
+		place(L.splits, L.maxBig);
+	});
+	L.sorted = sortedIds;
+	L.bin = bin;
+	L.rangeFirst = rangeFirst;
+	L.rangeLast = rangeLast;
+	if (n <= kBigTask) {
+		kSahInit<<<blocksFor(n, 256), 256, 0, stream>>>(n, sortedIds, L.blockTasks, L.ctr);
+	} else {
+		static const int most = residentBlocks(kSahLevels, kThreads, 0); // the grid barrier needs all of them
+		void* args[] = {&lo, &hi, &L};
+		RGL_SAH_OK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&kSahLevels), dim3(std::min(most, maxChunks)),
+		                                       dim3(kThreads), args, 0, stream));
 	}
-	levels_ += levels_ > 0 ? 2 : 0;
-}
-
-void SahTopology::enqueue()
-{
-	if (ctr_ == nullptr) {
-		return;
-	}
-	const int grid = n_ / kChunk + maxBig_ + 1; // bound on a level's chunks; blocks past them return
-	for (int l = 0; l < levels_; ++l) {
-		kSahLevelPrep<<<1, 1024, 0, stream_>>>(cur_, chunkBase_, bounds_, ctr_);
-		kSahBounds<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, lo_, hi_, cen_, bounds_, bins_);
-		kSahBins<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, lo_, hi_, cen_, bounds_, bins_);
-		kSahSplit<<<blocksFor(maxBig_ * 32, 128), 128, 0, stream_>>>(cur_, bounds_, bins_, splits_, bin_, rangeFirst_, rangeLast_, next_,
-		                                                             blockTasks_, ctr_);
-		kSahPartCount<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, cen_, bounds_, splits_, chunkLeft_);
-		kSahPartScatter<<<grid, kThreads, 0, stream_>>>(cur_, ctr_, chunkBase_, idsCur_, cen_, bounds_, splits_, chunkLeft_, idsNext_, sorted_);
-		countLaunch(6);
-		std::swap(cur_, next_);
-		std::swap(idsCur_, idsNext_);
-	}
-	levels_ = 4; // of a tree that is deeper
-	// Blocks take ranges until none is left: their number is known on the device only.
-	prepareSahBlock();
-	kSahBlock<<<std::min(n_ / 2 + 1, kBlockGrid), kBlockThreads, sizeof(BlockShared), stream_>>>(
-	    blockTasks_, n_, nullptr, const_cast<float4*>(lo_), const_cast<float4*>(hi_), sorted_, NodeSink{bin_, rangeFirst_, rangeLast_, ctr_});
 	countLaunch();
+	// Blocks take ranges until none is left: their number is known on the device only.
+	static const int meshBlocks = [] {
+		RGL_SAH_OK(cudaFuncSetAttribute(kSahBlock<MeshShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(MeshShared)));
+		return residentBlocks(kSahBlock<MeshShared>, kMeshThreads, sizeof(MeshShared));
+	}();
+	kSahBlock<MeshShared><<<std::min(blocksFor(n, 32), meshBlocks), kMeshThreads, sizeof(MeshShared), stream>>>(
+	    L.blockTasks, n, nullptr, const_cast<float4*>(lo), const_cast<float4*>(hi), sortedIds, NodeSink{bin, rangeFirst, rangeLast, L.ctr});
+	countLaunch();
+	return L.ctr;
 }
-
-static_assert(kBigTask == kSahSmallMax, "one block builds ranges up to kSahSmallMax primitives");
 
 void enqueueSahTopologySmall(const InstanceRec* inst, float4* lo, float4* hi, int n, BinNode* bin, int32_t* rangeFirst, int32_t* rangeLast,
                              uint32_t* sortedIds, cudaStream_t s)
@@ -1278,7 +1319,7 @@ void enqueueSahTopologySmall(const InstanceRec* inst, float4* lo, float4* hi, in
 	if (n <= 0 || n > kSahSmallMax) {
 		throw std::runtime_error("SAH build: one-block topology takes 1.." + std::to_string(kSahSmallMax) + " primitives");
 	}
-	kSahBlock<<<1, kBlockThreads, sizeof(BlockShared), s>>>(nullptr, n, inst, lo, hi, sortedIds, NodeSink{bin, rangeFirst, rangeLast, nullptr});
+	kSahBlock<TlasShared><<<1, TlasShared::kBlockThreads, sizeof(TlasShared), s>>>(nullptr, n, inst, lo, hi, sortedIds, NodeSink{bin, rangeFirst, rangeLast, nullptr});
 	countLaunch();
 }
 

@@ -1,7 +1,7 @@
-"""Structure builds without the host in between, in kept device memory (csrc/build_memory.cpp, SahTopology).
+"""Structure builds without the host in between, in kept device memory (csrc/build_memory.cpp, kSahLevels).
 
-A mesh whose splits each take off one of ten clusters is deeper than the levels queued at first: the
-build goes on, and the tree is the host builder's. Meshes that come and go reuse storage that was freed;
+A mesh whose splits each take off one of ten clusters is deeper than an even tree, with a level per
+cluster: the tree is the host builder's. Meshes that come and go reuse storage that was freed;
 the scans must see the mesh that is there. Freed storage goes back to the device with rgl_cleanup.
 """
 import ctypes as C
@@ -27,7 +27,7 @@ def nested_clusters(clusters, per_cluster):
 
 
 @pytest.mark.parametrize("clusters,per_cluster", [(3, 700), (10, 2100), (12, 3000)])
-def test_trees_deeper_than_the_first_levels(rgl, clusters, per_cluster):
+def test_trees_deeper_than_an_even_one(rgl, clusters, per_cluster):
     v, idx, scale = nested_clusters(clusters, per_cluster)
     rng = np.random.default_rng(1)
     xy = (scale[::7, None] * rng.uniform(0.95, 1.05, (scale[::7].size, 2))).astype(np.float32)
