@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "common.hpp"
 #include "kernels.hpp"
@@ -240,6 +241,50 @@ __device__ __forceinline__ void copyElem(const uint8_t* src, uint8_t* dst, int s
 constexpr int kOpParamWords = (int) (sizeof(NoiseParams) / 4);
 static_assert(sizeof(NoiseParams) % 16 == 0 && sizeof(Mat34) <= sizeof(NoiseParams), "point-op parameter slot");
 
+// Loads and stores one field's element as words (sizes 4, 8 and 12) or as one 1- or 2-byte value; other
+// sizes go through copyElem.
+constexpr int kMaxElemWords = 3;
+__device__ __forceinline__ bool splitElem(int size) { return size <= 2 || size == 4 || size == 8 || size == 12; }
+__device__ __forceinline__ void loadElem(const uint8_t* s, int size, int i, uint32_t (&v)[kMaxElemWords])
+{
+	if (size == 1) {
+		v[0] = s[i];
+	} else if (size == 2) {
+		v[0] = reinterpret_cast<const uint16_t*>(s)[i];
+	} else {
+		const uint32_t* w = reinterpret_cast<const uint32_t*>(s) + (size_t) i * (size >> 2);
+		v[0] = w[0];
+		if (size >= 8) {
+			v[1] = w[1];
+		}
+		if (size == 12) {
+			v[2] = w[2];
+		}
+	}
+}
+__device__ __forceinline__ void storeElem(uint8_t* d, int size, uint32_t i, const uint32_t (&v)[kMaxElemWords])
+{
+	if (size == 1) {
+		d[i] = (uint8_t) v[0];
+	} else if (size == 2) {
+		reinterpret_cast<uint16_t*>(d)[i] = (uint16_t) v[0];
+	} else {
+		uint32_t* w = reinterpret_cast<uint32_t*>(d) + (size_t) i * (size >> 2);
+		w[0] = v[0];
+		if (size >= 8) {
+			w[1] = v[1];
+		}
+		if (size == 12) {
+			w[2] = v[2];
+		}
+	}
+}
+
+// What bounds it at scan sizes is the latency of one tile's phases, one after another: ticket 0.5 us,
+// flags 0.4, scan and list 0.4, look-back 1, fields and operations the rest. Four points per thread: with
+// two or one the phases of a tile are shorter, but more tiles look back further and ask for parameters
+// (524,288 points with three operations 22.8 / 28.2 / 33.0 us, 131,072 without 7.0 / 7.3 / 9.2, 32,768 6.5 /
+// 6.5 / 5.9).
 __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ flags, int cap, const int32_t* dInCount,
                                                    const __grid_constant__ FieldCopies fc, const __grid_constant__ PointOps ops,
                                                    int32_t* dOutCount, uint32_t* scratch,
@@ -257,13 +302,17 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 		tileShared = (int) atomicAdd(scratch, 1u);
 		lbFail = 0;
 	}
-	// The absorbed operations' parameters straight from the pinned blocks the nodes staged them in: at most
-	// 576 bytes a block, about 1 us of latency that other blocks cover. As copy nodes between the traversal
-	// and this kernel they held it up by 16 us (three operations).
-	for (int k = 0; k < ops.count; ++k) {
-		const int words = ops.op[k].kind == kOpTransform ? (int) (sizeof(Mat34) / 4) : kOpParamWords;
-		for (int w = tid; w < words; w += kBlock) {
-			opParams[k][w] = __ldcv(static_cast<const uint32_t*>(ops.op[k].params) + w);
+	// The absorbed operations' parameters straight from the pinned blocks the nodes staged them in, at most
+	// 576 bytes a block. They take 3 to 10 us to arrive when every block asks at once, so they are asked for
+	// here, into registers, and waited for before the operations only. (As copy nodes between the traversal
+	// and this kernel they held it up by 16 us, three operations.)
+	static_assert(kOpParamWords <= kBlock, "a word per thread");
+	uint32_t staged[kMaxPointOps];
+#pragma unroll
+	for (int k = 0; k < kMaxPointOps; ++k) {
+		staged[k] = 0u;
+		if (k < ops.count && tid < (ops.op[k].kind == kOpTransform ? (int) (sizeof(Mat34) / 4) : kOpParamWords)) {
+			staged[k] = __ldcv(static_cast<const uint32_t*>(ops.op[k].params) + tid);
 		}
 	}
 	__syncthreads();
@@ -391,39 +440,50 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 	}
 	__syncthreads();
 	const uint32_t kept = tileKept;
-	// Kept points c = tid + j * kBlock (at most kCompactItems per thread). Each field's source values of
-	// all the thread's points are loaded before the first store: the compiler cannot move a load past a
-	// store to a pointer that may alias it, so a point-at-a-time loop would serialise the loads.
+	// Kept points c = tid + j * kBlock (at most kCompactItems per thread). The source values of all the thread's
+	// points, of two fields at a time, are loaded before the first store: the compiler cannot move a
+	// load past a store to a pointer that may alias it, so one field after another (0.8 us each) or a point
+	// at a time would wait for every load in turn.
 	int src[kCompactItems];
 #pragma unroll
 	for (int j = 0; j < kCompactItems; ++j) {
 		const uint32_t c = (uint32_t) (tid + j * kBlock);
 		src[j] = c < kept ? tile * kCompactTile + keptLocal[c] : -1;
 	}
-	for (int f = 0; f < fc.count; ++f) {
-		if (f == ops.xyzField || f == ops.distField) {
-			continue;
-		}
-		const int sz = fc.f[f].size;
-		const uint8_t* s = static_cast<const uint8_t*>(fc.f[f].src);
-		uint8_t* d = static_cast<uint8_t*>(fc.f[f].dst);
-		if (sz == 4) {
-			uint32_t v[kCompactItems];
+	constexpr int kFields = 2; // fields in flight
+	for (int f0 = 0; f0 < fc.count; f0 += kFields) {
+		uint32_t v[kFields][kCompactItems][kMaxElemWords];
 #pragma unroll
-			for (int j = 0; j < kCompactItems; ++j) {
-				v[j] = src[j] >= 0 ? reinterpret_cast<const uint32_t*>(s)[src[j]] : 0u;
+		for (int q = 0; q < kFields; ++q) {
+			const int f = f0 + q;
+			if (f >= fc.count || f == ops.xyzField || f == ops.distField || !splitElem(fc.f[f].size)) {
+				continue;
 			}
 #pragma unroll
 			for (int j = 0; j < kCompactItems; ++j) {
 				if (src[j] >= 0) {
-					reinterpret_cast<uint32_t*>(d)[tileBase + tid + j * kBlock] = v[j];
+					loadElem(static_cast<const uint8_t*>(fc.f[f].src), fc.f[f].size, src[j], v[q][j]);
 				}
 			}
-		} else {
+		}
+#pragma unroll
+		for (int q = 0; q < kFields; ++q) {
+			const int f = f0 + q;
+			if (f >= fc.count || f == ops.xyzField || f == ops.distField) {
+				continue;
+			}
+			const int sz = fc.f[f].size;
+			uint8_t* d = static_cast<uint8_t*>(fc.f[f].dst);
 #pragma unroll
 			for (int j = 0; j < kCompactItems; ++j) {
-				if (src[j] >= 0) {
-					copyElem(s + (size_t) src[j] * sz, d + (size_t) (tileBase + tid + j * kBlock) * sz, sz);
+				if (src[j] < 0) {
+					continue;
+				}
+				const uint32_t pos = tileBase + (uint32_t) (tid + j * kBlock);
+				if (splitElem(sz)) {
+					storeElem(d, sz, pos, v[q][j]);
+				} else {
+					copyElem(static_cast<const uint8_t*>(fc.f[f].src) + (size_t) src[j] * sz, d + (size_t) pos * sz, sz);
 				}
 			}
 		}
@@ -437,6 +497,13 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 			p[j] = (src[j] >= 0 && ops.srcXyz) ? loadXyz(ops.srcXyz, src[j]) : v3(0.0f, 0.0f, 0.0f);
 			dd[j] = (src[j] >= 0 && ops.srcDist) ? ops.srcDist[src[j]] : 0.0f;
 		}
+#pragma unroll
+		for (int o = 0; o < kMaxPointOps; ++o) {
+			if (o < ops.count && tid < kOpParamWords) {
+				opParams[o][tid] = staged[o];
+			}
+		}
+		__syncthreads();
 #pragma unroll
 		for (int j = 0; j < kCompactItems; ++j) {
 			if (src[j] < 0) {
@@ -484,11 +551,16 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 
 struct WordMap
 {
-	int8_t field[64];  // field index of output word k, -1 = padding
-	int8_t word[64];   // word index inside that field
+	int8_t field[64];    // field of output word k, -1 = padding, kMixedWord = four bytes of their own
+	uint8_t word[64];    // word index inside that field
+	int8_t byteField[256]; // of mixed words: field of every output byte, -1 = padding,
+	uint8_t byteOf[256];   // and byte index inside it
 };
+constexpr int8_t kMixedWord = -2;
 
-// Word-aligned layouts: one thread per output 32-bit word, coalesced stores.
+// One thread per output 32-bit word, coalesced stores. A word inside one field of whole words is one
+// load, a word of smaller fields one load per byte (131,072 points of 32 bytes with three fields of 1 and
+// 2 bytes: 18 us with one thread per point and a store per byte).
 // The point of word w is w / pointWords; `magic` = ceil(2^32 / pointWords) turns that into one
 // multiply-high, exact for w < 2^26 (pointWords <= 64), and is 0 for larger launches.
 __global__ void kFormatWords(const __grid_constant__ FieldCopies fc, const __grid_constant__ WordMap wm, int pointWords, uint32_t magic,
@@ -506,11 +578,19 @@ __global__ void kFormatWords(const __grid_constant__ FieldCopies fc, const __gri
 	if (f >= 0) {
 		const int fw = fc.f[f].size >> 2;
 		v = static_cast<const uint32_t*>(fc.f[f].src)[(size_t) i * fw + wm.word[k]];
+	} else if (f == kMixedWord) {
+#pragma unroll
+		for (int b = 0; b < 4; ++b) {
+			const int bf = wm.byteField[4 * k + b];
+			if (bf >= 0) {
+				v |= (uint32_t) static_cast<const uint8_t*>(fc.f[bf].src)[(size_t) i * fc.f[bf].size + wm.byteOf[4 * k + b]] << (8 * b);
+			}
+		}
 	}
 	out[w] = v;
 }
 
-// Any layout: one thread per point, byte copies (padding bytes zeroed).
+// Points of no whole number of words: one thread per point, byte copies (padding bytes zeroed).
 __global__ void kFormatBytes(const __grid_constant__ FieldCopies fc, int pointSize, int cap, const int32_t* dCount, uint8_t* __restrict__ out)
 {
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -549,7 +629,7 @@ __global__ void kAosToSoa(const uint8_t* __restrict__ in, int pointSize, int n, 
 // Point clouds concatenated: blockIdx.y is the input, blockIdx.x a tile of its points. Every block
 // finds its input's offset by summing the counts before it (inputs are few); the copy moves whole
 // 4-byte words when the element size allows (all but 1- and 2-byte fields).
-constexpr int kMergeTile = 2048;
+constexpr int kMergeTile = 512; // four inputs of 32,768 points: 14.5 us with 64 blocks of 2,048 and one load in flight
 
 struct MergeTableView
 {
@@ -576,8 +656,19 @@ __device__ __forceinline__ void copyRange(const void* src, void* dst, long srcFi
 {
 	const W* s = static_cast<const W*>(src) + srcFirst;
 	W* d = static_cast<W*>(dst) + dstFirst;
-	for (long k = threadIdx.x; k < n; k += blockDim.x) {
-		d[k] = s[k];
+	constexpr int kInFlight = 4; // loads before the first store, which may alias
+	for (long k = threadIdx.x; k < n; k += kInFlight * kBlock) {
+		W v[kInFlight];
+#pragma unroll
+		for (int u = 0; u < kInFlight; ++u) {
+			v[u] = k + u * kBlock < n ? s[k + u * kBlock] : W(0);
+		}
+#pragma unroll
+		for (int u = 0; u < kInFlight; ++u) {
+			if (k + u * kBlock < n) {
+				d[k + u * kBlock] = v[u];
+			}
+		}
 	}
 }
 
@@ -749,7 +840,7 @@ void launchCompact(const int32_t* flags, int cap, const int32_t* dInCount, const
 		}
 		return;
 	}
-	int tiles = (cap + kCompactTile - 1) / kCompactTile;
+	const int tiles = (cap + kCompactTile - 1) / kCompactTile;
 	kCompact<<<tiles, kBlock, 0, s>>>(flags, cap, dInCount, fields, po, dOutCount, static_cast<uint32_t*>(scratch), dError, hostCount);
 	countLaunch();
 }
@@ -759,24 +850,22 @@ void launchFormat(const FieldCopies& fields, int pointSize, int cap, const int32
 	if (cap <= 0 || pointSize <= 0) {
 		return;
 	}
-	bool words = (pointSize % 4 == 0) && pointSize / 4 <= 64;
-	for (int f = 0; f < fields.count && words; ++f) {
-		words = (fields.f[f].size % 4 == 0) && (fields.f[f].offset % 4 == 0);
-	}
-	if (words) {
+	if (pointSize % 4 == 0 && pointSize / 4 <= 64) {
 		WordMap wm;
-		for (int k = 0; k < 64; ++k) {
-			wm.field[k] = -1;
-			wm.word[k] = 0;
-		}
+		std::memset(wm.byteField, -1, sizeof(wm.byteField));
+		std::memset(wm.byteOf, 0, sizeof(wm.byteOf));
 		for (int f = 0; f < fields.count; ++f) {
-			if (fields.f[f].src == nullptr) {
-				continue;
+			for (int b = 0; b < fields.f[f].size && fields.f[f].src != nullptr; ++b) {
+				wm.byteField[fields.f[f].offset + b] = (int8_t) f;
+				wm.byteOf[fields.f[f].offset + b] = (uint8_t) b;
 			}
-			for (int k = 0; k < fields.f[f].size / 4; ++k) {
-				wm.field[fields.f[f].offset / 4 + k] = (int8_t) f;
-				wm.word[fields.f[f].offset / 4 + k] = (int8_t) k;
-			}
+		}
+		for (int k = 0; k < 64; ++k) {
+			const int8_t* bf = wm.byteField + 4 * k;
+			const bool one = bf[0] == bf[1] && bf[0] == bf[2] && bf[0] == bf[3];
+			const bool whole = one && (bf[0] < 0 || (fields.f[bf[0]].size % 4 == 0 && wm.byteOf[4 * k] % 4 == 0));
+			wm.field[k] = whole ? bf[0] : kMixedWord;
+			wm.word[k] = (uint8_t) (wm.byteOf[4 * k] / 4);
 		}
 		int pw = pointSize / 4;
 		long total = (long) cap * pw;
