@@ -183,15 +183,18 @@ struct BuildStages
 // The whole collapse of a binary tree over n primitives in one cooperative launch, depth by depth with
 // a grid barrier between (one launch per depth, sixteen between host checks of the queue, before). A
 // depth adds to its own counter; the counter after next is cleared meanwhile, when nobody reads it.
-// `st` is zero at the start. A SAH topology that is not complete is not collapsed: the report says so. levelStarts (optional) receives the first node of every depth and the node
-// count, up to levelCap entries. 131,072 triangles: 516 us for sixteen launches before, see
-// collapse.cuh for what a depth cost and why.
+// `st` is zero at the start. A SAH topology that is not complete is not collapsed: the report says so.
+// levelStarts (optional) receives the first node of every depth and the node count, up to levelCap
+// entries. 131,072 triangles: sixteen launches 516 us, one 100 us, with the leaf records written at the
+// end, eight blocks per SM instead of four and the choices below 90 us (8 us a depth, see collapse.cuh
+// for what bounds it; the barriers 1.4 each).
 constexpr int kCollapseThreads = 128;
 __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, CollapseState* st,
                                                               int32_t* levelStarts, int32_t* nLevels, int levelCap, BuildStages stages)
 {
 	cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-	const uint32_t warp = (blockIdx.x * kCollapseThreads + threadIdx.x) >> 5, warps = gridDim.x * (kCollapseThreads / 32);
+	// Neighbouring nodes go to different SMs.
+	const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (kCollapseThreads / 32);
 	const uint32_t group = (threadIdx.x & 31u) >> 3;
 	const bool first = blockIdx.x == 0 && threadIdx.x == 0;
 	uint32_t start = 0, end = 1, leaves = 0;
@@ -242,6 +245,11 @@ __global__ void __launch_bounds__(kCollapseThreads) kCollapse(CollapseInputs in,
 			break; // not a proper tree; the host sees the counts
 		}
 	}
+	if (in.vertices != nullptr && end <= (uint32_t) n && leaves == (uint32_t) n) { // every record has its position
+		for (uint32_t i = blockIdx.x * kCollapseThreads + threadIdx.x; i < leaves; i += gridDim.x * kCollapseThreads) {
+			collapsedev::writeTriangle(in, out.tris, i);
+		}
+	}
 	if (first) {
 		report->nodes = end;
 		report->leaves = leaves;
@@ -287,11 +295,10 @@ void launchCollapse(CollapseInputs in, collapsedev::CollapseTarget out, int n, C
 		RGL_CUDA_OK(cudaGetDevice(&dev));
 		RGL_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 		RGL_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kCollapse, kCollapseThreads, 0));
-		return sms * std::min(perSm, 4);
+		return sms * std::min(perSm, 8);
 	}();
-	// The widest depths hold about n / 6 nodes, 16 at a time per block; a small tree takes fewer blocks,
-	// whose barrier is cheaper.
-	int grid = std::max(1, std::min(most, n / 256));
+	// The widest depths hold about n / 5 nodes, 16 at a time per block; a small tree takes fewer blocks.
+	int grid = std::max(1, std::min(most, n / 80));
 	void* args[] = {&in, &out, &n, &state, &levels.starts, &levels.count, &levels.capacity, &stages};
 	RGL_CUDA_OK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&kCollapse), dim3(grid), dim3(kCollapseThreads), args, 0, s));
 	countLaunch();

@@ -2,12 +2,14 @@
 // lane per child, four nodes per warp. The host function is its specification: same children, same
 // slots, same bytes; only the numbers of the nodes and of the leaf records follow the atomics.
 //
-// What bounds it is the chain of dependent loads from a node to its children's children: up to seven
-// rounds of opening the largest child, each one load latency. One thread per node, with the eight
-// children in local arrays, walked everything else serially as well (areas, slots, 48 plane
-// quantisations in double precision) and took 33-36 us per depth; here every lane holds one child in
-// registers and the choices are shuffles. Wide nodes are numbered depth by depth, so the queue entry
-// of a node sits at its own index and a depth is a range of indices: no queue counter.
+// What bounds it is latency, of instructions as much as of loads: a node takes about 8 us from its task to
+// its record, up to seven rounds of opening the largest child one after another, then slots, quantisation
+// and packing. One thread per node, with the eight children in local arrays, took 33-36 us per depth; here
+// every lane holds one child in registers and the choices are shuffles. The children of a child that may
+// be opened are prefetched while the choice is made, the slots are given out from one list that all eight
+// lanes hold, and a mesh's leaf records are written once all depths are done. Wide nodes are numbered depth
+// by depth, so the queue entry of a node sits at its own index and a depth is a range of indices: no queue
+// counter.
 #pragma once
 
 #include "bvh_core.hpp"
@@ -26,6 +28,11 @@ constexpr int32_t kNoChild = 0x7fffffff;
 // Per-depth counters: wide nodes allocated for the next depth (low word) and leaf records written by
 // this one (high word), so one 64-bit atomic serves both.
 using DepthCounter = unsigned long long;
+
+__device__ __forceinline__ void prefetchL1(const void* p)
+{
+	asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
+}
 
 struct CollapseTarget
 {
@@ -74,26 +81,42 @@ __device__ __forceinline__ void collapseGroups(bool valid, uint32_t wideIdx, Col
 		load();
 	}
 	float area = has ? halfArea(b) : -1.0f;
-	bool open = has && c >= 0 && cnt > in.leafMax; // an inner child that may be opened
+	// An inner child that may be opened has a key: its area's bits (areas are not negative, their bits are
+	// ordered; a NaN is never opened).
+	auto openKey = [&]() { return has && c >= 0 && cnt > in.leafMax && area >= 0.0f ? __float_as_uint(area + 0.0f) + 1u : 0u; };
+	uint32_t open = openKey();
+	// Its children are likely to be held next: asked for while the choice is made.
+	auto prefetch = [&]() {
+		if (TRIANGLES && open != 0u) {
+#pragma unroll
+			for (int q = 0; q < 2; ++q) {
+				const int32_t k = q == 0 ? left : right;
+				if (k >= 0) {
+					prefetchL1(in.bin + k);
+					prefetchL1(in.rangeFirst + k);
+					prefetchL1(in.rangeLast + k);
+				} else {
+					prefetchL1(in.sortedIds + ~k);
+				}
+			}
+		}
+	};
+	prefetch();
 
 	// Open the largest inner child until eight children are held or none is left (ties: the lowest).
 	int n = valid ? (task.right == kNoChild ? 1 : 2) : kWideArity;
 	for (;;) {
-		float bestA = open ? area : -1.0f;
-		int bestK = sub;
+		uint32_t best = open;
 #pragma unroll
 		for (int d = 1; d < 8; d <<= 1) {
-			const float oa = __shfl_xor_sync(kAll, bestA, d);
-			const int ok = __shfl_xor_sync(kAll, bestK, d);
-			if (oa > bestA || (oa == bestA && ok < bestK) || !(bestA >= 0.0f)) {
-				bestA = oa;
-				bestK = ok;
-			}
+			best = max(best, __shfl_xor_sync(kAll, best, d));
 		}
-		const bool go = n < kWideArity && bestA >= 0.0f;
+		const bool go = n < kWideArity && best != 0u;
+		const uint32_t holders = __ballot_sync(kAll, go && open == best) >> (8 * group) & 0xffu;
 		if (__ballot_sync(kAll, go) == 0u) {
 			break;
 		}
+		const int bestK = holders != 0u ? (int) lowestBit(holders) : 0;
 		const int32_t l = __shfl_sync(kAll, left, bestK, 8), r = __shfl_sync(kAll, right, bestK, 8);
 		const bool mine = go && (sub == bestK || sub == n);
 		if (mine) {
@@ -101,7 +124,8 @@ __device__ __forceinline__ void collapseGroups(bool valid, uint32_t wideIdx, Col
 			has = true;
 			load();
 			area = halfArea(b);
-			open = c >= 0 && cnt > in.leafMax;
+			open = openKey();
+			prefetch();
 		}
 		n += go ? 1 : 0;
 	}
@@ -128,21 +152,26 @@ __device__ __forceinline__ void collapseGroups(bool valid, uint32_t wideIdx, Col
 	const float ncx = 0.5f * (nb.lox + nb.hix), ncy = 0.5f * (nb.loy + nb.hiy), ncz = 0.5f * (nb.loz + nb.hiz);
 	const uint32_t oct = ((0.5f * (b.lox + b.hix) >= ncx) ? 1u : 0u) | ((0.5f * (b.loy + b.hiy) >= ncy) ? 2u : 0u) |
 	                     ((0.5f * (b.loz + b.hiz) >= ncz) ? 4u : 0u);
+	// Octants and lanes by rank, one word each for the whole group: every lane then walks the same list.
+	uint32_t octs = has ? oct << (3 * rank) : 0u, lanes = has ? (uint32_t) sub << (3 * rank) : 0u;
+#pragma unroll
+	for (int d = 1; d < 8; d <<= 1) {
+		octs |= __shfl_xor_sync(kAll, octs, d);
+		lanes |= __shfl_xor_sync(kAll, lanes, d);
+	}
+	const int children = __popc(__ballot_sync(kAll, has) >> (8 * group) & 0xffu);
 	uint32_t freeSlots = 0xffu;
 	int from = -1; // the lane whose child takes this lane's slot
 #pragma unroll
 	for (int r = 0; r < kWideArity; ++r) {
-		const uint32_t who = (__ballot_sync(kAll, has && rank == r) >> (8 * group)) & 0xffu;
-		const int src = who != 0u ? (int) lowestBit(who) : 0;
-		const uint32_t o = __shfl_sync(kAll, oct, src, 8);
-		const uint32_t near12 = octantPermute(0x6816u, o); // slots at distance 1 (low byte) and 2 of octant o
-		const uint32_t d0 = freeSlots & (1u << o), d1 = freeSlots & near12 & 0xffu, d2 = freeSlots & (near12 >> 8);
+		const uint32_t o = (octs >> (3 * r)) & 7u;
+		// slots at distance 1 and 2 of octant o: byte o of the eight
+		const uint32_t near1 = __byte_perm(0x86492916u, 0x68949261u, o), near2 = __byte_perm(0x61929468u, 0x16294986u, o);
+		const uint32_t d0 = freeSlots & (1u << o), d1 = freeSlots & near1, d2 = freeSlots & near2;
 		const uint32_t pick = d0 != 0u ? d0 : (d1 != 0u ? d1 : (d2 != 0u ? d2 : freeSlots));
-		const int s = pick != 0u ? (int) lowestBit(pick) : 0;
-		if (who != 0u) {
-			freeSlots &= ~(1u << s);
-			from = sub == s ? src : from;
-		}
+		const uint32_t bit = r < children ? pick & (0u - pick) : 0u;
+		freeSlots ^= bit;
+		from = bit == (1u << sub) ? (int) ((lanes >> (3 * r)) & 7u) : from;
 	}
 
 	// From here on a lane is a slot.
@@ -233,22 +262,30 @@ __device__ __forceinline__ void collapseGroups(bool valid, uint32_t wideIdx, Col
 		out.queue[childBase + (uint32_t) __popc(imask & ((1u << sub) - 1u))] = CollapseTask{left, right};
 	}
 	for (int m = 0; m < leafCnt; ++m) {
-		const int32_t id = in.sortedIds[first + m];
 		float4* rec = reinterpret_cast<float4*>(out.tris + triBase + (uint32_t) (triOff + m));
 		if (TRIANGLES) {
-			const int32_t* ix = in.indices + 3 * (size_t) id;
-			const float* va = in.vertices + 3 * (size_t) ix[0];
-			const float* vb = in.vertices + 3 * (size_t) ix[1];
-			const float* vc = in.vertices + 3 * (size_t) ix[2];
-			rec[0] = make_float4(va[0], va[1], va[2], __int_as_float(id));
-			rec[1] = make_float4(vb[0], vb[1], vb[2], 0.0f);
-			rec[2] = make_float4(vc[0], vc[1], vc[2], 0.0f);
+			rec[0].w = __int_as_float(first + m); // the sorted position: writeTriangle turns it into the record
 		} else { // TLAS leaf: the instance index only
-			rec[0] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(id));
+			rec[0] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(in.sortedIds[first + m]));
 			rec[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 			rec[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 		}
 	}
+}
+
+// Leaf record i of a mesh, once every depth is done: all records at once, so the chain from position to
+// triangle to indices to vertices is walked once, not once per depth.
+__device__ __forceinline__ void writeTriangle(const CollapseInputs& in, TriRecord* tris, uint32_t i)
+{
+	float4* rec = reinterpret_cast<float4*>(tris + i);
+	const int32_t id = in.sortedIds[__float_as_int(rec[0].w)];
+	const int32_t* ix = in.indices + 3 * (size_t) id;
+	const float* va = in.vertices + 3 * (size_t) ix[0];
+	const float* vb = in.vertices + 3 * (size_t) ix[1];
+	const float* vc = in.vertices + 3 * (size_t) ix[2];
+	rec[0] = make_float4(va[0], va[1], va[2], __int_as_float(id));
+	rec[1] = make_float4(vb[0], vb[1], vb[2], 0.0f);
+	rec[2] = make_float4(vc[0], vc[1], vc[2], 0.0f);
 }
 
 // The root's task.

@@ -55,7 +55,7 @@ constexpr int kBins = 32;
 constexpr int kBinWords = 7;                    // lo xyz, hi xyz (ordered bits), count
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 // Larger ranges split in the level loop, the others are built by a block each. 131,072 triangles, 2,048 /
-// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us (two blocks per SM from 1,024 down).
+// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us (one block of 512 threads per SM, by registers).
 constexpr int kBigTask = 1024;
 constexpr int kMeshThreads = 512;
 constexpr int kChunk = 512;                     // elements per block in the level loop: 256 blocks for 131,072 triangles
@@ -709,7 +709,8 @@ __global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restri
 // What bounds a block is the chain of splits below each other, so what matters is that splits which do
 // not depend on each other run together. With every range above 32 split by the whole block in turn and
 // every subrange of a small one split alone, the ranges of 131,072 triangles took 885 us, 94 instances 58;
-// side by side 255 (ranges of up to 2,048), 141 now; 94 instances 31.
+// side by side 255 (ranges of up to 2,048), with ranges of up to 1,024 and segmented scans in the smallest
+// 136; 94 instances 31.
 constexpr int kMidTask = 256;
 
 template<int CAPACITY, int THREADS>
@@ -727,7 +728,7 @@ struct BlockShared
 	uint32_t red[kBlockWarps][12];
 	uint32_t bounds[12];
 	int scan[kBlockWarps];
-	uint8_t perm[kBlockWarps][32];
+	uint8_t perm[kBlockWarps][3][32];
 	int top, nMid[2], nSmall;
 	uint32_t nextNode, taken;
 	int4 cur;
@@ -862,10 +863,9 @@ __device__ void warpSplit(SHARED& S, const int4 range, int base, int midList, co
 }
 
 // A range of 2..32 elements built to its leaves by one warp: lane j holds the element at position j, and
-// all subranges of a depth are split together. Every lane takes its own element's bin as the last one left
-// of a split (the splits between two neighbouring elements' bins are the same split; the host takes the
-// first, after the left one's bin) and gathers both sides' boxes from its subrange, element by element,
-// along each axis; the best of the subrange's candidates, in the host's order, is its split.
+// all subranges of a depth are split together, per axis by a sort of the subrange's elements by bin and a
+// segmented scan of their boxes from either end; the best of the candidates, in the host's order, is its
+// split.
 template<class SHARED>
 __device__ void smallBuild(SHARED& S, const int4 range, int base, const NodeSink& out)
 {
@@ -916,67 +916,77 @@ __device__ void smallBuild(SHARED& S, const int4 range, int base, const NodeSink
 		for (int k = 0; k < 12; ++k) {
 			b12[k] = __shfl_sync(kAll, b12[k], last);
 		}
-		uint32_t myBin[3], packed = 0;
+		// The subrange's elements in order of their bins, one order per axis: a bin's place is the number of
+		// smaller ones, counted bit by bit with ballots.
+		const uint32_t below = (1u << lane) - 1u;
+		const uint32_t segment = active ? ((y < 32 ? 1u << y : 0u) - 1u) & ~((1u << x) - 1u) : 1u << lane;
+		uint32_t myBin[3];
 		bool valid[3];
 #pragma unroll
 		for (int ax = 0; ax < 3; ++ax) {
 			const AxisFrame f = axisFrame(b12, ax);
 			valid[ax] = f.valid;
 			myBin[ax] = f.valid ? (uint32_t) binOf(c[ax], f.cmin, f.scale) : 0u;
-			packed |= myBin[ax] << (8 * ax);
+			uint32_t less = 0, equal = segment;
+#pragma unroll
+			for (int bit = 4; bit >= 0; --bit) {
+				const bool one = ((myBin[ax] >> bit) & 1u) != 0u;
+				const uint32_t ones = __ballot_sync(kAll, one);
+				less |= one ? equal & ~ones : 0u;
+				equal &= one ? ones : ~ones;
+			}
+			S.perm[warp][ax][(active ? x : lane) + __popc(less) + __popc(equal & below)] = (uint8_t) lane;
 		}
-		// Both sides of this lane's candidate on each axis.
-		uint32_t L[3][6], R[3][6];
-		int lc[3] = {1, 1, 1};
+		__syncwarp();
+		// Boxes of everything up to a place and from it on; a split after a place is a candidate when the next
+		// element is in another bin.
+		uint32_t L[3][6], R[3][6], bin[3];
 #pragma unroll
 		for (int ax = 0; ax < 3; ++ax) {
+			const int src = S.perm[warp][ax][lane];
+			bin[ax] = __shfl_sync(kAll, myBin[ax], src);
 #pragma unroll
 			for (int q = 0; q < 6; ++q) {
-				L[ax][q] = w[q];
-				R[ax][q] = q < 3 ? kEmptyLo : kEmptyHi;
+				L[ax][q] = R[ax][q] = __shfl_sync(kAll, w[q], src);
 			}
 		}
-		int j = lane;
-		for (int k = 1; k < longest; ++k) {
-			j = j + 1 < y ? j + 1 : x;
-			const int src = active ? j : lane;
-			const bool counts = k < len;
-			const uint32_t theirs = __shfl_sync(kAll, packed, src);
-			uint32_t v[6];
-#pragma unroll
-			for (int q = 0; q < 6; ++q) {
-				v[q] = __shfl_sync(kAll, w[q], src);
-			}
+		for (int off = 1; off < longest; off <<= 1) {
+			const bool up = lane - off >= x, down = lane + off < y;
 #pragma unroll
 			for (int ax = 0; ax < 3; ++ax) {
-				const bool l = ((theirs >> (8 * ax)) & 0xffu) <= myBin[ax];
-				lc[ax] += l && counts ? 1 : 0;
 #pragma unroll
 				for (int q = 0; q < 6; ++q) {
-					if (l) {
-						L[ax][q] = q < 3 ? min(L[ax][q], v[q]) : max(L[ax][q], v[q]);
-					} else {
-						R[ax][q] = q < 3 ? min(R[ax][q], v[q]) : max(R[ax][q], v[q]);
+					const uint32_t l = __shfl_up_sync(kAll, L[ax][q], off), r = __shfl_down_sync(kAll, R[ax][q], off);
+					if (up) {
+						L[ax][q] = q < 3 ? min(L[ax][q], l) : max(L[ax][q], l);
+					}
+					if (down) {
+						R[ax][q] = q < 3 ? min(R[ax][q], r) : max(R[ax][q], r);
 					}
 				}
 			}
 		}
-		// The lane's best candidate as (cost bits, axis and bin, left count): costs are not negative, so their
-		// bits are ordered, and among equal costs the first (axis, bin) is the smaller word.
+		// The lane's best candidate as (cost, axis and bin, left count); among equal costs the first (axis, bin)
+		// is the smaller word.
 		float bestCost = kInf;
 		uint32_t bestKey = 0xffffffffu;
+		const int lc = lane + 1 - x, rc = y - lane - 1;
 #pragma unroll
 		for (int ax = 0; ax < 3; ++ax) {
-			const int rc = len - lc[ax];
-			if (active && valid[ax] && rc > 0) {
+			uint32_t r[6];
+#pragma unroll
+			for (int q = 0; q < 6; ++q) {
+				r[q] = __shfl_down_sync(kAll, R[ax][q], 1);
+			}
+			const uint32_t nextBin = __shfl_down_sync(kAll, bin[ax], 1);
+			if (active && valid[ax] && rc > 0 && nextBin != bin[ax]) {
 				const float ha = halfAreaOf(unordered(L[ax][0]), unordered(L[ax][1]), unordered(L[ax][2]), unordered(L[ax][3]), unordered(L[ax][4]),
 				                            unordered(L[ax][5]));
-				const float hb = halfAreaOf(unordered(R[ax][0]), unordered(R[ax][1]), unordered(R[ax][2]), unordered(R[ax][3]), unordered(R[ax][4]),
-				                            unordered(R[ax][5]));
-				const float cost = __fadd_rn(__fmul_rn(ha, (float) lc[ax]), __fmul_rn(hb, (float) rc));
+				const float hb = halfAreaOf(unordered(r[0]), unordered(r[1]), unordered(r[2]), unordered(r[3]), unordered(r[4]), unordered(r[5]));
+				const float cost = __fadd_rn(__fmul_rn(ha, (float) lc), __fmul_rn(hb, (float) rc));
 				if (cost < bestCost) {
 					bestCost = cost;
-					bestKey = ((uint32_t) (ax * kBins) + myBin[ax] + 1u) << 8 | (uint32_t) lc[ax];
+					bestKey = ((uint32_t) (ax * kBins) + bin[ax] + 1u) << 8 | (uint32_t) lc;
 				}
 			}
 		}
@@ -998,14 +1008,14 @@ __device__ void smallBuild(SHARED& S, const int4 range, int base, const NodeSink
 		const uint32_t mine = axis == 0u ? myBin[0] : (axis == 1u ? myBin[1] : myBin[2]);
 		const bool goLeft = active && (middle ? lane < x + nLeft : mine < cut);
 		// stable partition within the subrange
-		const uint32_t below = (1u << lane) - 1u, fromX = ~((1u << x) - 1u);
+		const uint32_t fromX = ~((1u << x) - 1u);
 		const int leftRank = __popc(__ballot_sync(kAll, goLeft) & below & fromX);
 		int dst = !active ? lane : (goLeft ? x + leftRank : x + nLeft + (lane - x - leftRank));
 		if (dst < 0 || dst >= 32) {
 			out.error();
 			dst = lane;
 		}
-		S.perm[warp][dst] = (uint8_t) lane;
+		S.perm[warp][0][dst] = (uint8_t) lane;
 		// Nodes: each subrange's first lane writes it and takes numbers for its inner children.
 		const bool leads = active && lane == x;
 		int32_t child[2] = {~(base + a + x), ~(base + a + x + nLeft)};
@@ -1026,7 +1036,7 @@ __device__ void smallBuild(SHARED& S, const int4 range, int base, const NodeSink
 		}
 		__syncwarp();
 		const int32_t cl = __shfl_sync(kAll, child[0], x), cr = __shfl_sync(kAll, child[1], x);
-		const int src = S.perm[warp][lane];
+		const int src = S.perm[warp][0][lane];
 		__syncwarp();
 		e = __shfl_sync(kAll, e, src);
 #pragma unroll
