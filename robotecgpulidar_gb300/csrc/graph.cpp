@@ -603,15 +603,17 @@ void RaytraceNode::ensureOrder(const rgl::BatchJob& b, cudaStream_t s)
 	const float hi[3] = {scene->worldUpper()[0], scene->worldUpper()[1], scene->worldUpper()[2]};
 	auto* keys = static_cast<uint32_t*>(orderKeys.ensure(sizeof(uint32_t) * n));
 	auto* vals = static_cast<uint32_t*>(orderVals.ensure(sizeof(uint32_t) * n));
-	auto* err = static_cast<int32_t*>(orderError.ensure(sizeof(int32_t)));
-	RGL_CHECK_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
+	auto* err = static_cast<int32_t*>(orderError.ensure(2 * sizeof(int32_t))); // sort error, direction cells
+	RGL_CHECK_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(int32_t), s));
 	rgl::launchBeamKeys(b.p.rays, b.hasRayTransform ? &b.rayTransform : nullptr, n, 0, schedule.order, lo, hi, keys, vals, s);
 	rgl::sortPairs(keys, vals, n, kKeyBits, orderScratch.ensure(rgl::sortPairsScratchBytes(n, kKeyBits)), err, s);
-	int32_t failed = 0;
-	RGL_CHECK_CUDA(cudaMemcpyAsync(&failed, err, sizeof(failed), cudaMemcpyDeviceToHost, s));
+	rgl::launchCountCells(keys, n, err + 1, s);
+	int32_t result[2] = {0, 0};
+	RGL_CHECK_CUDA(cudaMemcpyAsync(result, err, sizeof(result), cudaMemcpyDeviceToHost, s));
 	RGL_CHECK_CUDA(cudaStreamSynchronize(s));
 	// A sort whose look-back gave up leaves no permutation: cast in the given order instead.
-	orderValid = failed == 0;
+	orderValid = result[0] == 0;
+	orderCells = result[1];
 	if (!orderValid) {
 		rgl::logMessage(rgl::LogLevel::Warn, "RaytraceNode: beam ordering sort did not complete; casting beams in the given order");
 	}
@@ -630,7 +632,7 @@ void RaytraceNode::stageJob(cudaStream_t s)
 	(void) job.device();
 	rgl::TaskRange& tr = job.host().tasks;
 	tr.base[0] = 0;
-	tr.base[1] = rgl::setJobTasks(b, schedule.packing, b.p.nRays);
+	tr.base[1] = rgl::setJobTasks(b, schedule.packing, b.p.nRays, b.order != nullptr ? orderCells : 0);
 	shading = rgl::needsShadingKernel(p);
 	if (counter.get() == nullptr) {
 		RGL_CHECK_CUDA(cudaMemset(counter.ensure(rgl::kTraceCounterBytes), 0, rgl::kTraceCounterBytes));

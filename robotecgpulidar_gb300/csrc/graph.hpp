@@ -373,6 +373,7 @@ private:
 	void ensureOrder(const rgl::BatchJob& b, cudaStream_t s);
 	rgl::DeviceBuffer orderKeys{false}, orderVals{false}, orderScratch{false}, orderError{false};
 	int32_t orderCount = -1, orderKind = rgl::kOrderNatural;
+	int32_t orderCells = 0; // direction cells that the ordered beams fill
 	const void* orderRays = nullptr;
 	bool orderValid = false;
 };

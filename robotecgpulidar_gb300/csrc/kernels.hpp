@@ -158,8 +158,14 @@ static_assert(kPoolSamples >= kMaxBeamSamples, "a beam's samples fit the pool");
 // / 37 / 32 us, 32,768 beams 39 / 37 / 36 / 101 us, 76,920 beams 112 / 97 / 99 / 365 us, 131,072 beams 92
 // / 89 / 98 / 474 us. Pooled samples want about eight tasks per warp (58 samples, 65,536 beams: 1221 /
 // 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per task): fewer leave a long tail.
+// `cells`: direction cells that the beams fill (launchCountCells on their sorted keys, 0: not known). The
+// beams of a cell, less than 0.4 degrees apart in azimuth, take nearly the same walk, so a warp takes them
+// together however small the launch: a ring of 3,000 / 12,000 / 30,000 beams took 27 / 29 / 29 us in
+// tasks of 1 / 3 / 7 beams, 21 us in tasks of 2 / 10 / 16 and more.
 constexpr int kResidentWarps = 16; // per SM, at 128 registers
-int setJobTasks(BatchJob& job, int packing, int64_t launchBeams);
+int setJobTasks(BatchJob& job, int packing, int64_t launchBeams, int cells = 0);
+// Adds the number of distinct keys among n sorted ones to *cells (device).
+void launchCountCells(const uint32_t* sortedKeys, int n, int32_t* cells, cudaStream_t stream);
 // Resolves and caches the launch configuration (occupancy, shared-memory opt-in) of a schedule;
 // call it outside stream capture before the first captured launch of that schedule.
 void prepareTraceBatch(int nJobs, int maxSamples, bool shading, const BatchSchedule& s);

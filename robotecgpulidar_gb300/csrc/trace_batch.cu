@@ -115,6 +115,16 @@ __global__ void kBeamKeys(const Mat34* __restrict__ rays, Mat34 tf, int hasTf, i
 	values[i] = (uint32_t) i;
 }
 
+// Distinct keys among n sorted ones, added to *cells.
+__global__ void kCountCells(const uint32_t* __restrict__ keys, int n, int32_t* cells)
+{
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t firsts = __ballot_sync(0xffffffffu, i < n && (i == 0 || keys[i] != keys[i - 1]));
+	if ((threadIdx.x & 31) == 0 && firsts != 0u) {
+		atomicAdd(cells, (int32_t) __popc(firsts));
+	}
+}
+
 template<int MODE, bool SHADING>
 const void* batchKernel(int regs)
 {
@@ -172,13 +182,16 @@ int smCount()
 
 } // namespace
 
-int setJobTasks(BatchJob& job, int packing, int64_t launchBeams)
+int setJobTasks(BatchJob& job, int packing, int64_t launchBeams, int cells)
 {
 	const int S = job.p.nSamples;
 	int beams = 32;
 	if (packing != kPackSerial) {
 		const int64_t resident = (int64_t) smCount() * kResidentWarps;
-		const int64_t want = S <= kLaneGroupSamples ? (launchBeams + 2 * resident - 1) / (2 * resident) : launchBeams / (8 * resident);
+		int64_t want = S <= kLaneGroupSamples ? (launchBeams + 2 * resident - 1) / (2 * resident) : launchBeams / (8 * resident);
+		if (S <= kLaneGroupSamples && cells > 0) {
+			want = std::max<int64_t>(want, job.p.nRays / cells);
+		}
 		const int most = S <= kLaneGroupSamples ? 32 / S : std::min(32, kPoolSamples / S);
 		beams = (int) std::max<int64_t>(1, std::min<int64_t>(want, most));
 	}
@@ -257,6 +270,14 @@ void launchTraceBatch(const BatchJob* dJobs, const int32_t* dTaskBase, int nJobs
 	cfg.numAttrs = overlapPrevious ? 1 : 0;
 	RGL_BATCH_CUDA_OK(cudaLaunchKernelExC(&cfg, ls.fn, args));
 	countLaunch();
+}
+
+void launchCountCells(const uint32_t* sortedKeys, int n, int32_t* cells, cudaStream_t stream)
+{
+	if (n > 0) {
+		kCountCells<<<(n + 255) / 256, 256, 0, stream>>>(sortedKeys, n, cells);
+		countLaunch();
+	}
 }
 
 void launchBeamKeys(const Mat34* rays, const Mat34* transform, int n, uint32_t jobIndex, int order, const float* worldLo, const float* worldHi, uint32_t* keys,
