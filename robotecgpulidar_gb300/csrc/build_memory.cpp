@@ -12,8 +12,8 @@ namespace {
 
 // A pool keeps this much unused memory over a synchronisation. With the default pool, which returns
 // everything at every synchronisation, each build mapped its memory anew: an allocation, its release and
-// the synchronisation after it cost 86 us against 2 us from a pool that keeps it. The bound holds a build
-// of 4 million triangles (about 120 bytes each).
+// the synchronisation after it cost 86 us against 2 us from a pool that keeps it. The bound holds the
+// temporaries of a build of 3 million triangles (about 160 bytes each).
 constexpr uint64_t kKeepBytes = 512ull << 20;
 
 // Made at the first use and never destroyed: storage of static objects is freed during exit. The
