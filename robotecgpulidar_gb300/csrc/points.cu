@@ -235,11 +235,14 @@ __device__ __forceinline__ void copyElem(const uint8_t* src, uint8_t* dst, int s
 }
 
 // One pass: per-tile flag counts, decoupled look-back for the tile offset, scatter of every field.
-// scratch: [0] tile ticket, [1..tiles] tile status words, [tiles + 1] finished tiles; zero before the
-// first launch, and the last tile to finish zeroes it again for the next one.
+// scratch: tile ticket, finished tiles, whether the operations' parameters are there, the parameters, then
+// one status word per tile; zero but for the parameters before the first launch, and the last tile to finish
+// makes it so again for the next one.
+enum { kScratchTicket = 0, kScratchFinished = 1, kScratchReady = 2, kScratchParams = 4 };
 // Parameters of the absorbed point operations, copied into shared memory once per block.
 constexpr int kOpParamWords = (int) (sizeof(NoiseParams) / 4);
 static_assert(sizeof(NoiseParams) % 16 == 0 && sizeof(Mat34) <= sizeof(NoiseParams), "point-op parameter slot");
+constexpr int kScratchStatus = kScratchParams + kMaxPointOps * kOpParamWords;
 
 // Loads and stores one field's element as words (sizes 4, 8 and 12) or as one 1- or 2-byte value; other
 // sizes go through copyElem.
@@ -282,9 +285,8 @@ __device__ __forceinline__ void storeElem(uint8_t* d, int size, uint32_t i, cons
 
 // What bounds it at scan sizes is the latency of one tile's phases, one after another: ticket 0.5 us,
 // flags 0.4, scan and list 0.4, look-back 1, fields and operations the rest. Four points per thread: with
-// two or one the phases of a tile are shorter, but more tiles look back further and ask for parameters
-// (524,288 points with three operations 22.8 / 28.2 / 33.0 us, 131,072 without 7.0 / 7.3 / 9.2, 32,768 6.5 /
-// 6.5 / 5.9).
+// two the phases of a tile are shorter, but twice the tiles look back further (524,288 points with three
+// operations 18.3 / 21.3 us, 131,072 without 7.0 / 7.8, 32,768 6.5 / 6.2).
 __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ flags, int cap, const int32_t* dInCount,
                                                    const __grid_constant__ FieldCopies fc, const __grid_constant__ PointOps ops,
                                                    int32_t* dOutCount, uint32_t* scratch,
@@ -299,24 +301,25 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 	__shared__ uint32_t lbBallot[kBlock / 32], lbSum[kBlock / 32];
 	__shared__ int lbFail;
 	if (tid == 0) {
-		tileShared = (int) atomicAdd(scratch, 1u);
+		tileShared = (int) atomicAdd(&scratch[kScratchTicket], 1u);
 		lbFail = 0;
-	}
-	// The absorbed operations' parameters straight from the pinned blocks the nodes staged them in, at most
-	// 576 bytes a block. They take 3 to 10 us to arrive when every block asks at once, so they are asked for
-	// here, into registers, and waited for before the operations only. (As copy nodes between the traversal
-	// and this kernel they held it up by 16 us, three operations.)
-	static_assert(kOpParamWords <= kBlock, "a word per thread");
-	uint32_t staged[kMaxPointOps];
-#pragma unroll
-	for (int k = 0; k < kMaxPointOps; ++k) {
-		staged[k] = 0u;
-		if (k < ops.count && tid < (ops.op[k].kind == kOpTransform ? (int) (sizeof(Mat34) / 4) : kOpParamWords)) {
-			staged[k] = __ldcv(static_cast<const uint32_t*>(ops.op[k].params) + tid);
-		}
 	}
 	__syncthreads();
 	const int tile = tileShared;
+	// The absorbed operations' parameters come straight from the pinned blocks the nodes staged them in, at
+	// most 576 bytes. The first tile fetches them while it counts and leaves them in the scratch for the
+	// others: with every block asking at once they took 3 to 10 us to arrive. (As copy nodes between the
+	// traversal and this kernel they held it up by 16 us, three operations.)
+	static_assert(kOpParamWords <= kBlock, "a word per thread");
+	uint32_t staged[kMaxPointOps] = {};
+	if (tile == 0) {
+#pragma unroll
+		for (int k = 0; k < kMaxPointOps; ++k) {
+			if (k < ops.count && tid < (ops.op[k].kind == kOpTransform ? (int) (sizeof(Mat34) / 4) : kOpParamWords)) {
+				staged[k] = __ldcv(static_cast<const uint32_t*>(ops.op[k].params) + tid);
+			}
+		}
+	}
 	const int n = dInCount ? *dInCount : cap;
 	const int first = tile * kCompactTile + tid * kCompactItems;
 	int keep[kCompactItems];
@@ -359,8 +362,21 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 			warpSums[w] = run;
 			run += v;
 		}
-		atomicExch(&scratch[1 + tile], (tile == 0 ? kFlagInc : kFlagAgg) | run);
+		atomicExch(&scratch[kScratchStatus + tile], (tile == 0 ? kFlagInc : kFlagAgg) | run);
 		tileKept = run;
+	}
+	if (tile == 0 && ops.count > 0) {
+#pragma unroll
+		for (int k = 0; k < kMaxPointOps; ++k) {
+			if (k < ops.count && tid < kOpParamWords) {
+				__stcg(scratch + kScratchParams + k * kOpParamWords + tid, staged[k]);
+			}
+		}
+		__threadfence();
+		__syncthreads();
+		if (tid == 0) {
+			atomicExch(&scratch[kScratchReady], 1u);
+		}
 	}
 	// Decoupled look-back by the whole block: each step reads the status words of the kBlock
 	// predecessors before the window's end (one per thread, spinning until it is published) and sums
@@ -371,7 +387,7 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 		const int idx = k - tid;
 		uint32_t st = kFlagInc; // before tile 0: an inclusive prefix of 0
 		if (idx >= 0) {
-			const volatile uint32_t* p = scratch + 1 + idx;
+			const volatile uint32_t* p = scratch + kScratchStatus + idx;
 			int spins = 0;
 			st = *p;
 			while ((st & ~kValueMask) == 0u && ++spins < kSpinLimit) {
@@ -417,7 +433,7 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 		}
 		const uint32_t run = tileKept;
 		if (tile > 0) {
-			atomicExch(&scratch[1 + tile], kFlagInc | (prefix + run));
+			atomicExch(&scratch[kScratchStatus + tile], kFlagInc | (prefix + run));
 		}
 		tileBase = prefix;
 		const int tiles = (cap + kCompactTile - 1) / kCompactTile;
@@ -497,13 +513,26 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 			p[j] = (src[j] >= 0 && ops.srcXyz) ? loadXyz(ops.srcXyz, src[j]) : v3(0.0f, 0.0f, 0.0f);
 			dd[j] = (src[j] >= 0 && ops.srcDist) ? ops.srcDist[src[j]] : 0.0f;
 		}
-#pragma unroll
-		for (int o = 0; o < kMaxPointOps; ++o) {
-			if (o < ops.count && tid < kOpParamWords) {
-				opParams[o][tid] = staged[o];
+		if (ops.count > 0) {
+			if (tid == 0) {
+				const volatile uint32_t* ready = scratch + kScratchReady;
+				int spins = 0;
+				while (*ready == 0u && ++spins < kSpinLimit) {
+				}
+				if (*ready == 0u) {
+					*(volatile int32_t*) errorFlag = 1; // never expected: the first tile is running
+				}
+				__threadfence();
 			}
+			__syncthreads();
+#pragma unroll
+			for (int o = 0; o < kMaxPointOps; ++o) {
+				if (o < ops.count && tid < kOpParamWords) {
+					opParams[o][tid] = __ldcg(scratch + kScratchParams + o * kOpParamWords + tid);
+				}
+			}
+			__syncthreads();
 		}
-		__syncthreads();
 #pragma unroll
 		for (int j = 0; j < kCompactItems; ++j) {
 			if (src[j] < 0) {
@@ -537,12 +566,15 @@ __global__ void __launch_bounds__(kBlock) kCompact(const int32_t* __restrict__ f
 	const int tiles = (cap + kCompactTile - 1) / kCompactTile;
 	if (tid == 0) {
 		__threadfence();
-		lastTile = atomicAdd(&scratch[1 + tiles], 1u) == (uint32_t) (tiles - 1);
+		lastTile = atomicAdd(&scratch[kScratchFinished], 1u) == (uint32_t) (tiles - 1);
 	}
 	__syncthreads();
 	if (lastTile) {
-		for (int k = tid; k < tiles + 2; k += kBlock) {
-			scratch[k] = 0u;
+		for (int k = tid; k < tiles; k += kBlock) {
+			scratch[kScratchStatus + k] = 0u;
+		}
+		if (tid < kScratchParams) {
+			scratch[tid] = 0u;
 		}
 	}
 }
@@ -821,7 +853,7 @@ void launchNoiseDistance(const float* inXyz, const float* inDist, float* outXyz,
 	}
 }
 
-size_t compactScratchBytes(int cap) { return sizeof(uint32_t) * (size_t) (2 + (cap + kCompactTile - 1) / kCompactTile); }
+size_t compactScratchBytes(int cap) { return sizeof(uint32_t) * (size_t) (kScratchStatus + (cap + kCompactTile - 1) / kCompactTile); }
 
 void launchCompact(const int32_t* flags, int cap, const int32_t* dInCount, const FieldCopies& fields, const PointOps* ops,
                    int32_t* dOutCount, void* scratch, int32_t* dError, cudaStream_t s, int32_t* hostCount)
