@@ -20,7 +20,9 @@ uint64_t launchCount();
 
 // ---- sort.cu
 size_t sortPairsScratchBytes(int n, int keyBits);
+size_t sortPairsZeroBytes(int n, int keyBits); // leading bytes of the scratch that a sort starts from as zero
 void sortPairs(uint32_t* keys, uint32_t* values, int n, int keyBits, void* scratch, int32_t* errorFlag, cudaStream_t stream);
+void sortCountedPairs(uint32_t* keys, uint32_t* values, int n, int keyBits, void* scratch, int32_t* errorFlag, cudaStream_t stream);
 
 // ---- bvh.cu
 struct BlasBuild

@@ -174,12 +174,14 @@ __global__ void __launch_bounds__(kThreads) kOnesweep(const uint32_t* __restrict
 
 } // namespace
 
-size_t sortPairsScratchBytes(int n, int keyBits)
+// Scratch: digit counts of every pass, tile tickets, tile status words (all zero at the start), then the
+// other half of the ping-pong.
+size_t sortPairsZeroBytes(int n, int keyBits)
 {
-	int passes = (keyBits + 7) / 8;
-	int tiles = (n + kTile - 1) / kTile;
-	return sizeof(uint32_t) * (size_t) (passes * 256 + passes + (size_t) passes * tiles * 256 + 2 * (size_t) n);
+	const int passes = (keyBits + 7) / 8, tiles = (n + kTile - 1) / kTile;
+	return sizeof(uint32_t) * (size_t) (passes * 256 + passes + (size_t) passes * tiles * 256);
 }
+size_t sortPairsScratchBytes(int n, int keyBits) { return sortPairsZeroBytes(n, keyBits) + sizeof(uint32_t) * 2 * (size_t) n; }
 
 // Sorts keys/values in place (ascending, stable). `scratch` must hold sortPairsScratchBytes(n, keyBits).
 void sortPairs(uint32_t* keys, uint32_t* values, int n, int keyBits, void* scratch, int32_t* errorFlag, cudaStream_t stream)
@@ -187,19 +189,28 @@ void sortPairs(uint32_t* keys, uint32_t* values, int n, int keyBits, void* scrat
 	if (n <= 1) {
 		return;
 	}
-	int passes = (keyBits + 7) / 8;
-	int tiles = (n + kTile - 1) / kTile;
+	const int passes = (keyBits + 7) / 8;
+	cudaMemsetAsync(scratch, 0, sortPairsZeroBytes(n, keyBits), stream);
+	int hb = (n + 1023) / 1024;
+	hb = hb > 1024 ? 1024 : hb;
+	kHistogram<<<hb, 256, 0, stream>>>(keys, n, passes, static_cast<uint32_t*>(scratch));
+	countLaunch();
+	sortCountedPairs(keys, values, n, keyBits, scratch, errorFlag, stream);
+}
+
+// The passes alone: the caller has zeroed the first sortPairsZeroBytes of the scratch and counted the keys'
+// digits into its first words, 256 a pass, the lowest digit first.
+void sortCountedPairs(uint32_t* keys, uint32_t* values, int n, int keyBits, void* scratch, int32_t* errorFlag, cudaStream_t stream)
+{
+	if (n <= 1) {
+		return;
+	}
+	const int passes = (keyBits + 7) / 8, tiles = (n + kTile - 1) / kTile;
 	uint32_t* hist = static_cast<uint32_t*>(scratch);
 	uint32_t* tickets = hist + passes * 256;
 	uint32_t* status = tickets + passes;
 	uint32_t* k2 = status + (size_t) passes * tiles * 256;
 	uint32_t* v2 = k2 + n;
-	size_t zeroBytes = sizeof(uint32_t) * (size_t) (passes * 256 + passes + (size_t) passes * tiles * 256);
-	cudaMemsetAsync(hist, 0, zeroBytes, stream);
-	int hb = (n + 1023) / 1024;
-	hb = hb > 1024 ? 1024 : hb;
-	kHistogram<<<hb, 256, 0, stream>>>(keys, n, passes, hist);
-	countLaunch();
 	uint32_t *ki = keys, *vi = values, *ko = k2, *vo = v2;
 	for (int p = 0; p < passes; ++p) {
 		kOnesweep<<<tiles, kThreads, 0, stream>>>(ki, vi, ko, vo, n, 8 * p, hist + p * 256, status + (size_t) p * tiles * 256,
