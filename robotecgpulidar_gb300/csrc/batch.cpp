@@ -20,34 +20,6 @@ bool sameSchedule(const rgl::BatchSchedule& a, const rgl::BatchSchedule& b)
 	return a.block == b.block && a.packing == b.packing && a.order == b.order && a.chunk == b.chunk && a.regs == b.regs;
 }
 
-// Gives every kernel node of a captured frame except the traversal launches the greatest priority:
-// a wave's later nodes, ready when its traversal completes, then take the SM slots that free up
-// before the blocks of the next traversal launch waiting for them.
-cudaError_t prioritizeNodeKernels(cudaGraph_t graph, int priority)
-{
-	size_t n = 0;
-	cudaError_t e = cudaGraphGetNodes(graph, nullptr, &n);
-	std::vector<cudaGraphNode_t> nodes(n);
-	if (e == cudaSuccess && n > 0) {
-		e = cudaGraphGetNodes(graph, nodes.data(), &n);
-	}
-	for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
-		cudaGraphNodeType type;
-		e = cudaGraphNodeGetType(nodes[i], &type);
-		if (e != cudaSuccess || type != cudaGraphNodeTypeKernel) {
-			continue;
-		}
-		cudaKernelNodeParams params = {};
-		e = cudaGraphKernelNodeGetParams(nodes[i], &params);
-		if (e != cudaSuccess || rgl::isTraceBatchKernel(params.func)) {
-			continue;
-		}
-		cudaLaunchAttributeValue v = {};
-		v.priority = priority;
-		e = cudaGraphKernelNodeSetAttribute(nodes[i], cudaLaunchAttributePriority, &v);
-	}
-	return e;
-}
 } // namespace
 
 BatchRun::BatchRun(std::vector<Node::Ptr> a) : anchors(std::move(a)), dKeys(false), dOrder(false), dSortScratch(false), dError(false)
@@ -537,7 +509,7 @@ void BatchRun::run()
 					}
 				}
 				if (inst == cudaSuccess) {
-					inst = prioritizeNodeKernels(graph, priorityHigh);
+					inst = rgl::prioritizeNodeKernels(graph, priorityHigh);
 				}
 				if (inst == cudaSuccess) {
 					inst = cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);

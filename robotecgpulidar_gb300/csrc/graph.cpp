@@ -1549,7 +1549,18 @@ void GraphRunCtx::run()
 			}
 			cudaGraph_t graph = nullptr;
 			RGL_CHECK_CUDA(cudaStreamEndCapture(stream_, &graph));
-			const cudaError_t inst = cudaGraphInstantiate(&exec, graph, 0);
+			// What follows a traversal goes before the traversals of other graphs that wait for SMs: in a loop
+			// that runs 64 graphs and then reads them, every compaction otherwise came after the last
+			// traversal, and no read overlapped one (9.3 ms a frame, so 6.4).
+			static const int high = [] {
+				int least = 0, greatest = 0;
+				RGL_CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+				return greatest;
+			}();
+			cudaError_t inst = rgl::prioritizeNodeKernels(graph, high);
+			if (inst == cudaSuccess) {
+				inst = cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+			}
 			cudaGraphDestroy(graph);
 			RGL_CHECK_CUDA(inst);
 			execKernels = rgl::launchCount() - launches0;

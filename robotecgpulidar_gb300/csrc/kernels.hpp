@@ -158,8 +158,10 @@ static_assert(kPoolSamples >= kMaxBeamSamples, "a beam's samples fit the pool");
 // that does not fill the chip twice over takes fewer beams per task, because a warp ends with its
 // slowest ray and fewer rays diverge less: with 32 beams, 16, 8 and 1 per task, 3,600 beams took 35 / 33
 // / 37 / 32 us, 32,768 beams 39 / 37 / 36 / 101 us, 76,920 beams 112 / 97 / 99 / 365 us, 131,072 beams 92
-// / 89 / 98 / 474 us. Pooled samples want about eight tasks per warp (58 samples, 65,536 beams: 1221 /
-// 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per task): fewer leave a long tail.
+// / 89 / 98 / 474 us. (With L2 flushed before every run one round of tasks is worth more: 32,768 beams
+// of the plain scene in tasks of 7 / 14 / 32 took 57 / 45 / 48 us.) Pooled samples want about eight tasks
+// per warp (58 samples, 65,536 beams: 1221 / 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per
+// task): fewer leave a long tail.
 // `cells`: direction cells that the beams fill (launchCountCells on their sorted keys, 0: not known). The
 // beams of a cell, less than 0.4 degrees apart in azimuth, take nearly the same walk, so a warp takes them
 // together however small the launch: a ring of 3,000 / 12,000 / 30,000 beams took 27 / 29 / 29 us in
@@ -176,6 +178,10 @@ void prepareTraceBatch(int nJobs, int maxSamples, bool shading, const BatchSched
 cudaError_t addParamGatherNode(cudaGraph_t graph, const ParamCopy* dTable, int n);
 // Whether `fn` (a kernel node's function) is one of the persistent traversal kernels.
 bool isTraceBatchKernel(const void* fn);
+// Gives every kernel node of a captured frame except the traversal launches the greatest priority:
+// a wave's later nodes, ready when its traversal completes, then take the SM slots that free up
+// before the blocks of the next traversal launch waiting for them.
+cudaError_t prioritizeNodeKernels(cudaGraph_t graph, int priority);
 // The traversal's counter block: task ticket and finished blocks, zeroed once when allocated; every
 // launch leaves it zero again.
 constexpr size_t kTraceCounterBytes = 2 * sizeof(uint32_t);

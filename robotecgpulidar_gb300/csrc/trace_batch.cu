@@ -20,6 +20,7 @@
 #include <stdexcept>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include "trace_batch_kernel.cuh"
 
@@ -240,6 +241,32 @@ bool isTraceBatchKernel(const void* fn)
 		}
 	}
 	return false;
+}
+
+cudaError_t prioritizeNodeKernels(cudaGraph_t graph, int priority)
+{
+	size_t n = 0;
+	cudaError_t e = cudaGraphGetNodes(graph, nullptr, &n);
+	std::vector<cudaGraphNode_t> nodes(n);
+	if (e == cudaSuccess && n > 0) {
+		e = cudaGraphGetNodes(graph, nodes.data(), &n);
+	}
+	for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+		cudaGraphNodeType type;
+		e = cudaGraphNodeGetType(nodes[i], &type);
+		if (e != cudaSuccess || type != cudaGraphNodeTypeKernel) {
+			continue;
+		}
+		cudaKernelNodeParams params = {};
+		e = cudaGraphKernelNodeGetParams(nodes[i], &params);
+		if (e != cudaSuccess || isTraceBatchKernel(params.func)) {
+			continue;
+		}
+		cudaLaunchAttributeValue v = {};
+		v.priority = priority;
+		e = cudaGraphKernelNodeSetAttribute(nodes[i], cudaLaunchAttributePriority, &v);
+	}
+	return e;
 }
 
 void prepareTraceBatch(int nJobs, int maxSamples, bool shading, const BatchSchedule& s)
