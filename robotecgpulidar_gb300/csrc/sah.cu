@@ -52,10 +52,10 @@ namespace {
 	} while (0)
 
 constexpr int kBins = 32;
-constexpr int kBinWords = 7;                    // lo xyz, hi xyz (ordered bits), count
+constexpr int kBinWords = 7;                    // lo xyz (ordered bits, complemented), hi xyz (ordered bits), count: empty is 0
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 // Larger ranges split in the level loop, the others are built by a block each. 131,072 triangles, 2,048 /
-// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us (one block of 512 threads per SM, by registers).
+// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us, before the bins were filled out of step (one block of 512 threads per SM, by registers).
 constexpr int kBigTask = 1024;
 constexpr int kMeshThreads = 512;
 constexpr int kChunk = 512;                     // elements per block in the level loop: 256 blocks for 131,072 triangles
@@ -141,6 +141,48 @@ __device__ __forceinline__ AxisFrame axisFrame(const uint32_t* b12, int a)
 	return f;
 }
 
+// Adds an element to its bin of every axis. Neighbouring elements of a mesh share bins, and 32 lanes adding
+// to one word take turns; so every lane goes through the axes and words from a place of its own: a value is
+// turned by the lane's number, as the word it goes to (131,072 triangles of a terrain: levels 183 us in step,
+// 167 so, block ranges 141 and 122; 94 instances 32 and 27).
+__device__ __forceinline__ void addToBins(uint32_t* bins, const float4& l, const float4& h, const float4& c, const AxisFrame (&fr)[3])
+{
+	const uint32_t lane = threadIdx.x & 31u, turn = lane % 6u, third = lane % 3u;
+	uint32_t v[6] = {~ordered(l.x), ~ordered(l.y), ~ordered(l.z), ordered(h.x), ordered(h.y), ordered(h.z)};
+#pragma unroll
+	for (int by = 1; by < 6; by <<= 1) {
+		uint32_t t[6];
+#pragma unroll
+		for (int j = 0; j < 6; ++j) {
+			t[j] = (turn & (uint32_t) by) != 0u ? v[(j + by) % 6] : v[j];
+		}
+#pragma unroll
+		for (int j = 0; j < 6; ++j) {
+			v[j] = t[j];
+		}
+	}
+	int at[3];
+#pragma unroll
+	for (int a = 0; a < 3; ++a) {
+		at[a] = fr[a].valid ? (a * kBins + binOf(comp3(c, a), fr[a].cmin, fr[a].scale)) * kBinWords : -1;
+	}
+	const int first = third == 0u ? at[0] : (third == 1u ? at[1] : at[2]), second = third == 0u ? at[1] : (third == 1u ? at[2] : at[0]),
+	          last = third == 0u ? at[2] : (third == 1u ? at[0] : at[1]);
+	const int order[3] = {first, second, last};
+#pragma unroll
+	for (int a = 0; a < 3; ++a) {
+		if (order[a] < 0) {
+			continue;
+		}
+		uint32_t* bin = bins + order[a];
+#pragma unroll
+		for (uint32_t j = 0; j < 6; ++j) {
+			atomicMax(bin + (turn + j < 6u ? turn + j : turn + j - 6u), v[j]);
+		}
+		atomicAdd(bin + 6, 1u);
+	}
+}
+
 // Best split of a range from its bins (3 x 32 x 7 words, any address space) and bounds, by one warp:
 // the candidate between bins b-1 and b of axis a costs halfArea(left) * nLeft + halfArea(right) * nRight;
 // candidates with an empty side are skipped; the lowest cost wins, the first in (axis, b) order among
@@ -154,7 +196,8 @@ __device__ SahSplit warpBestSplit(const uint32_t* bins, const uint32_t* b12, int
 	for (int a = 0; a < 3; ++a) {
 #pragma unroll
 		for (int k = 0; k < kBinWords; ++k) {
-			v[a][k] = bins[(a * kBins + lane) * kBinWords + k];
+			const uint32_t word = bins[(a * kBins + lane) * kBinWords + k];
+			v[a][k] = k < 3 ? ~word : word;
 		}
 	}
 #pragma unroll
@@ -364,30 +407,10 @@ __device__ __forceinline__ float4 centroidOf(const float4& l, const float4& h)
 	return make_float4(__fmul_rn(0.5f, __fadd_rn(l.x, h.x)), __fmul_rn(0.5f, __fadd_rn(l.y, h.y)), __fmul_rn(0.5f, __fadd_rn(l.z, h.z)), 0.0f);
 }
 
-__device__ __forceinline__ void addToBins(uint32_t* sb, const float4& l, const float4& h, const AxisFrame (&fr)[3])
-{
-	const float4 c = centroidOf(l, h);
-#pragma unroll
-	for (int a = 0; a < 3; ++a) {
-		if (!fr[a].valid) {
-			continue;
-		}
-		uint32_t* bb = sb + (a * kBins + binOf(comp3(c, a), fr[a].cmin, fr[a].scale)) * kBinWords;
-		atomicMin(&bb[0], ordered(l.x));
-		atomicMin(&bb[1], ordered(l.y));
-		atomicMin(&bb[2], ordered(l.z));
-		atomicMax(&bb[3], ordered(h.x));
-		atomicMax(&bb[4], ordered(h.y));
-		atomicMax(&bb[5], ordered(h.z));
-		atomicAdd(&bb[6], 1u);
-	}
-}
-
 __device__ __forceinline__ void clearBins(uint32_t* bins, int first, int step, int words = kTaskBinWords)
 {
 	for (int k = first; k < words; k += step) {
-		const int w = k % kBinWords;
-		bins[k] = w < 3 ? kEmptyLo : (w < 6 ? kEmptyHi : 0u);
+		bins[k] = 0u;
 	}
 }
 
@@ -400,12 +423,10 @@ __device__ __forceinline__ void flushBins(uint32_t* sb, uint32_t* tb)
 			continue;
 		}
 		uint32_t* g = tb + k * kBinWords;
-		atomicMin(&g[0], bb[0]);
-		atomicMin(&g[1], bb[1]);
-		atomicMin(&g[2], bb[2]);
-		atomicMax(&g[3], bb[3]);
-		atomicMax(&g[4], bb[4]);
-		atomicMax(&g[5], bb[5]);
+#pragma unroll
+		for (int w = 0; w < 6; ++w) {
+			atomicMax(&g[w], bb[w]);
+		}
 		atomicAdd(&g[6], bb[6]);
 		clearBins(bb, 0, 1, kBinWords);
 	}
@@ -419,7 +440,7 @@ __device__ __forceinline__ void flushBins(uint32_t* sb, uint32_t* tb)
 // What bounds a level of a mesh of 100,000 triangles is not its data (4 MB, in L2) but the phases after
 // each other: as six launches (chunk table, bounds, bins, split, count, scatter) a level took 27 us, and
 // the host had to guess how many levels to queue; here it takes 17 (split 3.2, count 3, scatter 6,
-// barriers 1 to 2 each), 182 us in all for 131,072 triangles against 245.
+// barriers 1 to 2 each) and less since, 167 us in all for 131,072 triangles against 245.
 __global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restrict__ lo, const float4* __restrict__ hi, SahLevels L)
 {
 	__shared__ uint32_t sBins[2][kTaskBinWords];
@@ -466,7 +487,8 @@ __global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restri
 			fr[a] = axisFrame(L.bounds[0], a);
 		}
 		for (int i = thread; i < L.n; i += threads) {
-			addToBins(sBins[0], lo[i], hi[i], fr);
+			const float4 l = lo[i], h = hi[i];
+			addToBins(sBins[0], l, h, centroidOf(l, h), fr);
 		}
 		__syncthreads();
 		flushBins(sBins[0], L.bins);
@@ -672,9 +694,9 @@ __global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restri
 					if (s.child[left[q] ? 0 : 1] >= 0) {
 						L.ids[then][dst] = id[q];
 						if (left[q]) {
-							addToBins(sBins[0], l[q], h[q], fr[0]);
+							addToBins(sBins[0], l[q], h[q], centroidOf(l[q], h[q]), fr[0]);
 						} else {
-							addToBins(sBins[1], l[q], h[q], fr[1]);
+							addToBins(sBins[1], l[q], h[q], centroidOf(l[q], h[q]), fr[1]);
 						}
 					} else {
 						L.sorted[dst] = id[q];
@@ -710,7 +732,7 @@ __global__ void __launch_bounds__(kThreads, 2) kSahLevels(const float4* __restri
 // not depend on each other run together. With every range above 32 split by the whole block in turn and
 // every subrange of a small one split alone, the ranges of 131,072 triangles took 885 us, 94 instances 58;
 // side by side 255 (ranges of up to 2,048), with ranges of up to 1,024 and segmented scans in the smallest
-// 136; 94 instances 31.
+// 141, with bins filled out of step 122; 94 instances 27.
 constexpr int kMidTask = 256;
 
 template<int CAPACITY, int THREADS>
@@ -743,20 +765,8 @@ struct BlockShared
 	__device__ __forceinline__ float centroid(int e, int a) const { return __fmul_rn(0.5f, __fadd_rn(box[a][e], box[3 + a][e])); }
 	__device__ __forceinline__ void bin(uint32_t* to, int e, const AxisFrame (&fr)[3]) const
 	{
-#pragma unroll
-		for (int a = 0; a < 3; ++a) {
-			if (!fr[a].valid) {
-				continue;
-			}
-			uint32_t* bb = to + (a * kBins + binOf(centroid(e, a), fr[a].cmin, fr[a].scale)) * kBinWords;
-			atomicMin(&bb[0], ordered(box[0][e]));
-			atomicMin(&bb[1], ordered(box[1][e]));
-			atomicMin(&bb[2], ordered(box[2][e]));
-			atomicMax(&bb[3], ordered(box[3][e]));
-			atomicMax(&bb[4], ordered(box[4][e]));
-			atomicMax(&bb[5], ordered(box[5][e]));
-			atomicAdd(&bb[6], 1u);
-		}
+		const float4 l = make_float4(box[0][e], box[1][e], box[2][e], 0.0f), h = make_float4(box[3][e], box[4][e], box[5][e], 0.0f);
+		addToBins(to, l, h, make_float4(centroid(e, 0), centroid(e, 1), centroid(e, 2), 0.0f), fr);
 	}
 	__device__ __forceinline__ bool left(int e, int pos, int first, const SahSplit& s, const AxisFrame& f) const
 	{
