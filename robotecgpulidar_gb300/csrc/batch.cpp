@@ -46,6 +46,7 @@ BatchRun::~BatchRun()
 	if (running) {
 		cudaEventSynchronize(frameStop);
 	}
+	reads.finish();
 	for (auto& m : members) {
 		for (cudaEvent_t e : waveDone) {
 			m.ctx->forgetBatchEvent(e);
@@ -445,11 +446,11 @@ void BatchRun::run()
 	}
 
 	std::vector<uint64_t> sceneVersions;
-	for (Scene* sc : scenes) {
-		sc->prepareBatched(stream);
-		sceneVersions.push_back(sc->structureVersion());
-	}
 	try {
+		for (Scene* sc : scenes) {
+			sc->prepareBatched(stream);
+			sceneVersions.push_back(sc->structureVersion());
+		}
 		for (auto& m : members) {
 			m.ctx->prepareForBatch(stream);
 		}
@@ -532,8 +533,11 @@ void BatchRun::run()
 			RGL_CHECK_CUDA(cudaGraphLaunch(exec, stream));
 		}
 		RGL_CHECK_CUDA(cudaEventRecord(frameStop, stream));
+		reads.enqueued(frameStop);
 	}
 	catch (...) {
+		cudaEventRecord(frameStop, stream); // behind whatever got enqueued
+		reads.enqueued(frameStop);
 		for (Scene* sc : scenes) {
 			sc->markPosesDirty(); // the refit of this frame may not have been enqueued
 		}

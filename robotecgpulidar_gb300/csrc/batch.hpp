@@ -107,6 +107,8 @@ private:
 	std::vector<uint8_t> uploaded; // bytes of the job table and task bases last uploaded
 	rgl::DeviceBuffer dParamTable{false}; // the captured frame's parameter copies (read by its gather node)
 
+	rgl::StorageReader reads;
+
 	// Captured frame.
 	cudaGraphExec_t exec = nullptr;
 	std::vector<int> execWaveFirst;

@@ -1,5 +1,6 @@
 #include "build_memory.hpp"
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -49,6 +50,26 @@ cudaMemPool_t scratchPool()
 	return pool;
 }
 
+// Allocations of the first form: a stream of their own, so that they neither wait for nor disturb the legacy
+// stream.
+cudaStream_t storageStream()
+{
+	static cudaStream_t stream = [] {
+		cudaStream_t s = nullptr;
+		RGL_CHECK_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+		return s;
+	}();
+	return stream;
+}
+
+// Held while their events are waited for, so that no owner destroys one meanwhile.
+std::mutex readerMutex;
+std::vector<StorageReader*>& readers()
+{
+	static auto* all = new std::vector<StorageReader*>(); // never destroyed, as the pools
+	return *all;
+}
+
 // Report blocks not in use; as many exist as builds ever ran at the same time.
 std::mutex reportMutex;
 std::vector<BuildReport*>& freeReports()
@@ -71,14 +92,52 @@ void* allocate(cudaMemPool_t pool, size_t bytes, cudaStream_t s)
 
 } // namespace
 
+StorageReader::StorageReader()
+{
+	std::lock_guard<std::mutex> g(readerMutex);
+	readers().push_back(this);
+}
+
+StorageReader::~StorageReader()
+{
+	std::lock_guard<std::mutex> g(readerMutex);
+	readers().erase(std::find(readers().begin(), readers().end(), this));
+}
+
+void StorageReader::finish()
+{
+	std::lock_guard<std::mutex> g(readerMutex);
+	wait();
+}
+
+void StorageReader::wait()
+{
+	if (cudaEvent_t e = last_.exchange(nullptr)) {
+		cudaEventSynchronize(e);
+	}
+}
+
+void* allocateStorage(size_t bytes)
+{
+	void* p = allocate(storagePool(), bytes, storageStream());
+	RGL_CHECK_CUDA(cudaStreamSynchronize(storageStream()));
+	return p;
+}
+
 void* allocateStorage(size_t bytes, cudaStream_t s) { return allocate(storagePool(), bytes, s); }
 
 void freeStorage(void* p)
 {
-	if (p != nullptr) {
-		cudaDeviceSynchronize(); // a freed block is handed out again at once, on any stream
-		cudaFree(p);
+	if (p == nullptr) {
+		return;
 	}
+	{
+		std::lock_guard<std::mutex> g(readerMutex);
+		for (StorageReader* r : readers()) {
+			r->wait();
+		}
+	}
+	cudaFree(p); // of a pool's block: waits for nothing
 }
 
 uintptr_t BuildScratch::allocate(size_t bytes)
@@ -90,7 +149,10 @@ uintptr_t BuildScratch::allocate(size_t bytes)
 BuildScratch::~BuildScratch()
 {
 	if (base_ != nullptr) {
-		cudaFreeAsync(base_, stream_);
+		// Freed for good, so that trimBuildMemory finds it free: one that is queued on a stream counts as in
+		// use until the host has waited for it. A build has waited for its stream already.
+		cudaStreamSynchronize(stream_);
+		cudaFree(base_);
 	}
 }
 
@@ -127,7 +189,6 @@ bool trimBuildMemory()
 	if (!poolsMade) {
 		return false;
 	}
-	cudaDeviceSynchronize(); // frees still queued on streams count as in use
 	cudaMemPoolTrimTo(storagePool(), 0);
 	cudaMemPoolTrimTo(scratchPool(), 0);
 	std::lock_guard<std::mutex> g(reportMutex);

@@ -4,19 +4,43 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
 namespace rgl {
 
 // Scene storage (mesh vertices, indices, BLAS nodes), from a pool that keeps up to kKeepBytes for the
-// next mesh. The memory is usable on every stream once `s` has reached the call's point; freeing waits
-// for the device first, as cudaFree of a plain allocation does.
+// next mesh. The first form is usable on every stream at once, the second once `s` has reached the call's
+// point. A freed block is handed out again at once, on any stream, so freeing first waits for all
+// StorageReaders.
+void* allocateStorage(size_t bytes);
 void* allocateStorage(size_t bytes, cudaStream_t s);
 void freeStorage(void* p);
 
-// Temporaries of one build on one stream: one stream-ordered allocation, given back in the stream's
-// order when the object goes.
+// Device work that may read scene storage (a graph's runs, a batch's frames, a server slot's batches). Its
+// owner names an event behind the work it has just enqueued; freeStorage waits for the events named last.
+// It does not wait for the device as a whole, which is not allowed while any stream of the process is being
+// captured, by this library on another thread or by another one, and would end that capture.
+class StorageReader
+{
+public:
+	StorageReader();
+	StorageReader(const StorageReader&) = delete;
+	StorageReader& operator=(const StorageReader&) = delete;
+	~StorageReader();
+	// `behind` is recorded (not in a capture) after everything enqueued so far; it is the owner's.
+	void enqueued(cudaEvent_t behind) { last_.store(behind); }
+	// Waits for that event, which the owner is about to destroy.
+	void finish();
+
+private:
+	friend void freeStorage(void* p);
+	void wait();
+	std::atomic<cudaEvent_t> last_{nullptr};
+};
+
+// Temporaries of one build on one stream: one allocation, given back when the object goes, after the stream.
 class BuildScratch
 {
 public:

@@ -201,8 +201,7 @@ void* DeviceBuffer::ensure(size_t bytes)
 		}
 		RGL_CHECK_CUDA(e);
 	} else {
-		p = allocateStorage(want, nullptr);
-		RGL_CHECK_CUDA(cudaStreamSynchronize(nullptr)); // usable on every stream
+		p = allocateStorage(want);
 	}
 	if (ptr_) {
 		tracked_ ? (void) cudaFree(ptr_) : freeStorage(ptr_);

@@ -1330,6 +1330,7 @@ GraphRunCtx::~GraphRunCtx()
 {
 	releaseGraph();
 	releaseBranches();
+	reads.finish();
 	cudaEventDestroy(done);
 	cudaEventDestroy(runStart);
 	cudaEventDestroy(runStop);
@@ -1510,6 +1511,21 @@ void GraphRunCtx::run()
 	}
 	running = true;
 	batchedLast = false;
+	try {
+		enqueueRun(version);
+	}
+	catch (...) {
+		cudaEventRecord(done, stream_); // behind whatever got enqueued
+		reads.enqueued(done);
+		throw;
+	}
+	RGL_CHECK_CUDA(cudaEventRecord(done, stream_));
+	reads.enqueued(done);
+}
+
+// The prepare phase and the device work of a run (see run()).
+void GraphRunCtx::enqueueRun(uint64_t version)
+{
 	for (auto& n : order) {
 		n->prepareImpl(stream_);
 	}
@@ -1574,7 +1590,6 @@ void GraphRunCtx::run()
 		}
 		RGL_CHECK_CUDA(cudaGraphLaunch(exec, stream_));
 	}
-	RGL_CHECK_CUDA(cudaEventRecord(done, stream_));
 }
 
 // As run() but without the nodes' validation when no API call that may change a graph came since

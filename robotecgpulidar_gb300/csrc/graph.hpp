@@ -662,6 +662,7 @@ private:
 	};
 	void planBranches();
 	void enqueueNodes();
+	void enqueueRun(uint64_t version);
 	std::vector<Placement> placements; // by position in `order`; empty: everything on stream_
 	std::vector<cudaStream_t> branches;
 	std::vector<cudaEvent_t> branchEvents; // one per branch (join), then the fork's
@@ -669,6 +670,7 @@ private:
 	std::vector<Node::Ptr> order;
 	cudaStream_t stream_ = nullptr;
 	cudaEvent_t done = nullptr, runStart = nullptr, runStop = nullptr;
+	rgl::StorageReader reads;
 	cudaEvent_t batchDone = nullptr; // completion of the graph's part of the last batched frame
 	uint64_t validatedEpoch = 0;     // graphEditEpoch() of the last successful batch validation
 	bool validated = false;

@@ -108,6 +108,7 @@ Server::~Server()
 	}
 	cudaFreeHost(arena.host);
 	for (auto& s : slots) {
+		s->reads.finish();
 		cudaEventDestroy(s->done);
 		cudaEventDestroy(s->counted);
 		cudaEventDestroy(s->t0);
@@ -540,6 +541,7 @@ void Server::launch(Slot& slot, const rgl::BatchSchedule& sched, Slot* after)
 	// the other slot's result copies on the copy engine, and this batch's successor waits for it.
 	rgl::launchPublishWords(dResults, slot.hResultsDev, 2 * n, slot.stream);
 	RGL_CHECK_CUDA(cudaEventRecord(slot.counted, slot.stream));
+	slot.reads.enqueued(slot.counted);
 	RGL_CHECK_CUDA(cudaEventRecord(slot.tCounted, slot.stream));
 	slot.phase = Phase::Tracing;
 	RGL_CHECK_CUDA(cudaLaunchHostFunc(slot.stream, &Server::batchDone, this));
@@ -565,6 +567,7 @@ void Server::copyOut(Slot& slot)
 	}
 	RGL_CHECK_CUDA(cudaEventRecord(slot.t1, slot.stream));
 	RGL_CHECK_CUDA(cudaEventRecord(slot.done, slot.stream));
+	slot.reads.enqueued(slot.done);
 	slot.phase = Phase::Copying;
 	RGL_CHECK_CUDA(cudaLaunchHostFunc(slot.stream, &Server::batchDone, this));
 }
@@ -649,6 +652,7 @@ void Server::loop()
 						hCounts[s->reqs.size() + j] = 2;
 					}
 					cudaEventRecord(s->done, s->stream);
+					s->reads.enqueued(s->done);
 					s->phase = Phase::Copying;
 				}
 				lk.lock();
@@ -727,6 +731,8 @@ void Server::loop()
 				}
 				lk.lock();
 				if (!ok) {
+					cudaEventRecord(freeSlot->done, freeSlot->stream); // behind whatever got enqueued
+					freeSlot->reads.enqueued(freeSlot->done);
 					// The batch never reached the device: fail its requests.
 					const auto now = Clock::now();
 					for (auto* r : batch) {

@@ -144,6 +144,7 @@ private:
 		rgl::DeviceBuffer staged{false}; // compacted results: per request one block, xyz | distance | entity id
 		rgl::PinnedBuffer hTables, hResults;
 		int32_t* hResultsDev = nullptr; // device address of hResults (written by a kernel, not a copy)
+		rgl::StorageReader reads;
 		Phase phase = Phase::Tracing;
 		bool busy = false;
 	};
