@@ -513,7 +513,7 @@ void BatchRun::run()
 					inst = rgl::prioritizeNodeKernels(graph, priorityHigh);
 				}
 				if (inst == cudaSuccess) {
-					inst = cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+					inst = rgl::trimAndRetry([&] { return cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority); });
 				}
 				cudaGraphDestroy(graph);
 				RGL_CHECK_CUDA(inst);

@@ -1,11 +1,11 @@
 #include "build_memory.hpp"
 
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 #include <vector>
 
 #include "common.hpp"
+#include "kernels.hpp"
 
 namespace rgl {
 
@@ -17,13 +17,15 @@ namespace {
 // temporaries of a build of 3 million triangles (about 160 bytes each).
 constexpr uint64_t kKeepBytes = 512ull << 20;
 
-// Made at the first use and never destroyed: storage of static objects is freed during exit. The
-// allocator serialises threads and orders streams itself.
-std::atomic<bool> poolsMade{false};
+// Two pools: scene storage stays in use and would count against what the temporaries may keep. Made at the
+// first use and never destroyed: storage of static objects is freed during exit. The allocator serialises
+// threads and orders streams itself.
+enum Pool { kStorage, kScratch, kPools };
+std::mutex poolMutex;
+cudaMemPool_t pools[kPools] = {};
 
 cudaMemPool_t makePool()
 {
-	poolsMade = true;
 	int device = 0;
 	RGL_CHECK_CUDA(cudaGetDevice(&device));
 	cudaMemPoolProps props{};
@@ -38,16 +40,13 @@ cudaMemPool_t makePool()
 	return pool;
 }
 
-// Two pools: scene storage stays in use and would count against what the temporaries may keep.
-cudaMemPool_t storagePool()
+cudaMemPool_t poolOf(Pool which)
 {
-	static cudaMemPool_t pool = makePool();
-	return pool;
-}
-cudaMemPool_t scratchPool()
-{
-	static cudaMemPool_t pool = makePool();
-	return pool;
+	std::lock_guard<std::mutex> g(poolMutex);
+	if (pools[which] == nullptr) {
+		pools[which] = makePool();
+	}
+	return pools[which];
 }
 
 // Allocations of the first form: a stream of their own, so that they neither wait for nor disturb the legacy
@@ -78,16 +77,37 @@ std::vector<BuildReport*>& freeReports()
 	return *reports;
 }
 
-void* allocate(cudaMemPool_t pool, size_t bytes, cudaStream_t s)
+void* allocate(Pool which, size_t bytes, cudaStream_t s)
 {
+	const cudaMemPool_t pool = poolOf(which);
 	void* p = nullptr;
-	cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
-	if (e == cudaErrorMemoryAllocation && trimBuildMemory()) {
-		cudaGetLastError();
-		e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
-	}
-	RGL_CHECK_CUDA(e);
+	RGL_CHECK_CUDA(trimAndRetry([&] { return cudaMallocFromPoolAsync(&p, bytes, pool, s); }));
 	return p;
+}
+
+// A plain allocation of `count` elements.
+template<class T>
+void allocateArray(T*& p, size_t count)
+{
+	RGL_CHECK_CUDA(trimAndRetry([&] { return cudaMalloc(reinterpret_cast<void**>(&p), sizeof(T) * count); }));
+}
+
+template<class T>
+void freeArray(T*& p)
+{
+	cudaFree(p);
+	p = nullptr;
+}
+
+void freeTlasScratch(TlasBuild& t)
+{
+	t.smallCapacity = 0;
+	freeArray(t.lo);
+	freeArray(t.hi);
+	freeArray(t.bin);
+	freeArray(t.rangeFirst);
+	freeArray(t.rangeLast);
+	freeArray(t.sortedIds);
 }
 
 } // namespace
@@ -119,12 +139,12 @@ void StorageReader::wait()
 
 void* allocateStorage(size_t bytes)
 {
-	void* p = allocate(storagePool(), bytes, storageStream());
+	void* p = allocate(kStorage, bytes, storageStream());
 	RGL_CHECK_CUDA(cudaStreamSynchronize(storageStream()));
 	return p;
 }
 
-void* allocateStorage(size_t bytes, cudaStream_t s) { return allocate(storagePool(), bytes, s); }
+void* allocateStorage(size_t bytes, cudaStream_t s) { return allocate(kStorage, bytes, s); }
 
 void freeStorage(void* p)
 {
@@ -142,7 +162,7 @@ void freeStorage(void* p)
 
 uintptr_t BuildScratch::allocate(size_t bytes)
 {
-	base_ = rgl::allocate(scratchPool(), bytes, stream_);
+	base_ = rgl::allocate(kScratch, bytes, stream_);
 	return reinterpret_cast<uintptr_t>(base_);
 }
 
@@ -186,17 +206,63 @@ HostReport::~HostReport()
 
 bool trimBuildMemory()
 {
-	if (!poolsMade) {
-		return false;
+	bool made = false;
+	{
+		std::lock_guard<std::mutex> g(poolMutex);
+		for (cudaMemPool_t p : pools) {
+			if (p != nullptr) {
+				cudaMemPoolTrimTo(p, 0);
+				made = true;
+			}
+		}
 	}
-	cudaMemPoolTrimTo(storagePool(), 0);
-	cudaMemPoolTrimTo(scratchPool(), 0);
 	std::lock_guard<std::mutex> g(reportMutex);
 	for (BuildReport* r : freeReports()) {
 		cudaFreeHost(r);
 	}
 	freeReports().clear();
-	return true;
+	return made;
+}
+
+// The capacities are set once all arrays are there: after an allocation that failed, the next build of that
+// size starts over instead of using the ones that are missing.
+void allocateTlas(TlasBuild& t, int n)
+{
+	if (n > t.capacity) {
+		freeTlas(t);
+		allocateArray(t.nodes, (size_t) n);
+		allocateArray(t.leaves, (size_t) n);
+		allocateArray(t.enter, (size_t) n);
+		allocateArray(t.boxes, 6 * (size_t) n);
+		allocateArray(t.levelStarts, (size_t) n + 2);
+		allocateArray(t.nLevels, 1);
+		t.levelCapacity = n + 2;
+		t.capacity = n;
+	}
+	// The one-block rebuild's scratch has a size of its own: a scene that shrinks from above
+	// kSahSmallMax instances keeps its node storage but has no scratch yet.
+	if (n <= kSahSmallMax && n > t.smallCapacity) {
+		freeTlasScratch(t);
+		allocateArray(t.lo, (size_t) n);
+		allocateArray(t.hi, (size_t) n);
+		allocateArray(t.bin, (size_t) n);
+		allocateArray(t.rangeFirst, (size_t) n);
+		allocateArray(t.rangeLast, (size_t) n);
+		allocateArray(t.sortedIds, (size_t) n);
+		t.smallCapacity = n;
+	}
+}
+
+void freeTlas(TlasBuild& t)
+{
+	freeTlasScratch(t);
+	freeArray(t.nodes);
+	freeArray(t.leaves);
+	freeArray(t.enter);
+	freeArray(t.boxes);
+	freeArray(t.levelStarts);
+	freeArray(t.nLevels);
+	t = TlasBuild{};
 }
 
 } // namespace rgl

@@ -110,4 +110,17 @@ private:
 // Returns what the pools and the report list keep beyond what is in use; false when nothing was ever kept.
 bool trimBuildMemory();
 
+// Every device allocation of the library that may be large goes through this: memory may be out only
+// because of what the pools keep, so the allocation runs once more without it.
+template<class Allocate>
+cudaError_t trimAndRetry(Allocate&& allocate)
+{
+	cudaError_t e = allocate();
+	if (e == cudaErrorMemoryAllocation && trimBuildMemory()) {
+		cudaGetLastError();
+		e = allocate();
+	}
+	return e;
+}
+
 } // namespace rgl

@@ -759,48 +759,16 @@ __global__ void kEnterRecords(const TriRecord* __restrict__ leaves, const Instan
 // refit kernel.
 namespace {
 
-void freeSmallScratch(TlasBuild& t)
+// Shared memory of the one-block kernels, set outside any capture and for the largest scene: the limit is the
+// kernel's, so a small scene must not lower it under a large one.
+void prepareSmallTlas()
 {
-	void* ptrs[] = {t.lo, t.hi, t.bin, t.rangeFirst, t.rangeLast, t.sortedIds};
-	for (void* p : ptrs) {
-		cudaFree(p);
-	}
-	t.lo = t.hi = nullptr;
-	t.bin = nullptr;
-	t.rangeFirst = t.rangeLast = nullptr;
-	t.sortedIds = nullptr;
-	t.smallCapacity = 0;
-}
-
-void allocTlas(TlasBuild& t, int n)
-{
-	if (n > t.capacity) {
-		freeTlas(t);
-		t.capacity = n;
-		RGL_CUDA_OK(cudaMalloc(&t.nodes, sizeof(WideNode) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.leaves, sizeof(TriRecord) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.enter, sizeof(EnterRec) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.boxes, sizeof(Box) * (size_t) n));
-		t.levelCapacity = n + 2;
-		RGL_CUDA_OK(cudaMalloc(&t.levelStarts, sizeof(int32_t) * (size_t) t.levelCapacity));
-		RGL_CUDA_OK(cudaMalloc(&t.nLevels, sizeof(int32_t)));
-	}
-	// The one-block rebuild's scratch has a size of its own: a scene that shrinks from above
-	// kSahSmallMax instances keeps its node storage but has no scratch yet.
-	if (n <= kSahSmallMax && n > t.smallCapacity) {
-		freeSmallScratch(t);
-		RGL_CUDA_OK(cudaMalloc(&t.lo, sizeof(float4) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.hi, sizeof(float4) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.bin, sizeof(BinNode) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.rangeFirst, sizeof(int32_t) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.rangeLast, sizeof(int32_t) * (size_t) n));
-		RGL_CUDA_OK(cudaMalloc(&t.sortedIds, sizeof(uint32_t) * (size_t) n));
+	static const bool done = [] {
 		prepareSahBlock();
-		// Shared memory of the one-block collapse, set outside any capture and for the largest scene: the limit
-		// is the kernel's, so a small scene must not lower it under a large one.
 		RGL_CUDA_OK(cudaFuncSetAttribute(kCollapseSmall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smallCollapseLayout(kSahSmallMax).bytes));
-		t.smallCapacity = n;
-	}
+		return true;
+	}();
+	(void) done;
 }
 
 // The rebuild of up to kSahSmallMax instances from their device records: two launches, no host
@@ -820,7 +788,7 @@ void rebuildTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBuild& t, cudaStream_t s)
 {
 	if (n > 0) {
-		allocTlas(t, n);
+		allocateTlas(t, n);
 	}
 	t.nInstances = n;
 	t.nodeCount = 0;
@@ -828,6 +796,7 @@ void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBu
 		return;
 	}
 	if (n <= kSahSmallMax) {
+		prepareSmallTlas();
 		rebuildTlas(dInst, t, s);
 		return;
 	}
@@ -873,16 +842,6 @@ void refitTlas(const InstanceRec* dInst, TlasBuild& t, cudaStream_t s)
 	kRefitTlas<<<1, 256, 0, s>>>(t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), dInst, t.levelStarts, t.nLevels);
 	kEnterRecords<<<blocks(t.nInstances, 128), 128, 0, s>>>(t.leaves, dInst, t.nInstances, t.enter);
 	countLaunch(2);
-}
-
-void freeTlas(TlasBuild& t)
-{
-	freeSmallScratch(t);
-	void* ptrs[] = {t.nodes, t.leaves, t.enter, t.boxes, t.levelStarts, t.nLevels};
-	for (void* p : ptrs) {
-		cudaFree(p);
-	}
-	t = TlasBuild{};
 }
 
 } // namespace rgl

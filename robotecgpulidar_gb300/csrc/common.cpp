@@ -194,12 +194,7 @@ void* DeviceBuffer::ensure(size_t bytes)
 	size_t want = bytes < 256 ? 256 : bytes;
 	void* p = nullptr;
 	if (tracked_) {
-		cudaError_t e = cudaMalloc(&p, want);
-		if (e == cudaErrorMemoryAllocation && trimBuildMemory()) {
-			cudaGetLastError();
-			e = cudaMalloc(&p, want);
-		}
-		RGL_CHECK_CUDA(e);
+		RGL_CHECK_CUDA(trimAndRetry([&] { return cudaMalloc(&p, want); }));
 	} else {
 		p = allocateStorage(want);
 	}

@@ -1575,7 +1575,7 @@ void GraphRunCtx::enqueueRun(uint64_t version)
 			}();
 			cudaError_t inst = rgl::prioritizeNodeKernels(graph, high);
 			if (inst == cudaSuccess) {
-				inst = cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+				inst = rgl::trimAndRetry([&] { return cudaGraphInstantiateWithFlags(&exec, graph, cudaGraphInstantiateFlagUseNodePriority); });
 			}
 			cudaGraphDestroy(graph);
 			RGL_CHECK_CUDA(inst);

@@ -95,6 +95,8 @@ void buildTlas(const InstanceRec* hInstances, const InstanceRec* dInstances, int
 void updateTlas(const InstanceRec* dInstances, TlasBuild& t, cudaStream_t stream);
 // Refits the TLAS after instance boxes changed (same instance set): one single-block launch.
 void refitTlas(const InstanceRec* dInstances, TlasBuild& t, cudaStream_t stream);
+// Arrays for n instances, and for their one-block rebuild when n is within its limit (build_memory.cpp).
+void allocateTlas(TlasBuild& t, int n);
 void freeTlas(TlasBuild& t);
 
 // ---- animate.cu: mesh animation of entities

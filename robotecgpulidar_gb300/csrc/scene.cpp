@@ -74,7 +74,7 @@ void Mesh::setTexCoords(const rgl_vec2f* uvs, int32_t count)
 Texture::Texture(const void* texels, int32_t w, int32_t h) : width(w), height(h)
 {
 	const cudaChannelFormatDesc channel = cudaCreateChannelDesc<unsigned char>();
-	RGL_CHECK_CUDA(cudaMallocArray(&array, &channel, (size_t) w, (size_t) h));
+	RGL_CHECK_CUDA(rgl::trimAndRetry([&] { return cudaMallocArray(&array, &channel, (size_t) w, (size_t) h); }));
 	const size_t pitch = (size_t) w;
 	cudaError_t e = cudaMemcpy2DToArray(array, 0, 0, texels, pitch, pitch, (size_t) h, cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) {
