@@ -118,22 +118,17 @@ RGL_HD bool intersectTriangle(Vec3 a, Vec3 b, Vec3 c, Vec3 o, const Watertight& 
 	return true;
 }
 
-// Inverse of a direction component for the slab tests only, which are conservative and need no exact
-// inverse: the device's approximate reciprocal (relative error up to 2^-23) is one instruction where a
-// correctly rounded division is a sequence with a slow path, three times per frame change.
+// Inverse of a direction component, correctly rounded on the host and on the device, whose traversals the
+// completeness tests take for the same arithmetic. (The device's approximate reciprocal, wrong in the last
+// bit, made a scan of 524,288 points over 1M triangles 243 us where it is 250, and one of 58 samples a
+// beam 686 where it is 713; a caller has no say in that bit, so it stays exact.)
 RGL_HD float safeInv(float d)
 {
 	const float tiny = 1e-30f;
 	if (absf_(d) < tiny) {
 		d = d < 0.0f ? -tiny : tiny;
 	}
-#if defined(__CUDA_ARCH__)
-	float r;
-	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-	return r;
-#else
 	return 1.0f / d;
-#endif
 }
 
 RGL_HD float exp2Byte(uint8_t e)
@@ -175,8 +170,8 @@ RGL_HD int popc8(uint32_t x)
 // fma(1 + q 2^-15, S, D -+ e) with S = 2^15 A, A = s * inv (one grid step in t, exact: s is a power of
 // two), C = (p - o) * inv and D = C - S (see the node loop). Against the exact distance of the ray
 // with direction 1/inv it errs by at most
-//  * relative: inv (up to 2u), the FMA and the |t| share of the C terms, 7u|t| (u = 2^-24); entry and
-//    exit together 14u, covered by entry <= exit * (1 + 2e-6) (34u);
+//  * relative: inv, the FMA and the |t| share of the C terms, 6u|t| (u = 2^-24); entry and exit
+//    together 12u, covered by entry <= exit * (1 + 2e-6) (34u);
 //  * absolute: C rounds twice and D and D -+ e once each, 4u|C| + 2^-8 |A| with |C| <= |t| + 255 |A|,
 //    i.e. (2^-8 + 1020u) |A| < 0.0041 |A| beyond the relative part; near planes are moved earlier and
 //    far planes later by e = 0.01 |A| (kPlaneSlack).
