@@ -7,6 +7,7 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "beam_tasks.hpp"
 #include "build_memory.hpp"
 #include "device_types.hpp"
 
@@ -147,28 +148,9 @@ inline bool needsShadingKernel(const TraceParams& p)
 	return p.needIntensity != 0 || p.out.normal != nullptr || p.out.incidentAngle != nullptr || p.out.absVelocity != nullptr ||
 	       p.out.relVelocity != nullptr || p.out.radialSpeed != nullptr || p.distortion != 0;
 }
-// Lane groups take patterns of up to this many samples. Beyond, lanes idle (17 samples leave 15 of 32) and
-// the selection, done by one lane per beam, weighs more: 58 samples on two rounds of 32 lanes took
-// 2276 us for 65,536 beams over 1M triangles, pooled 1195 us; 5 samples took 302 us for 262,144 beams
-// in groups, pooled 327 us (the pool and the poses read again for six beams a task).
-constexpr int kLaneGroupSamples = 8;
-// Samples that a warp keeps in shared memory between tracing a task's beams and selecting their returns.
-constexpr int kPoolSamples = 352; // 6 beams of 58: two blocks of 256 threads with shading keep 98 KB each
 static_assert(kPoolSamples >= kMaxBeamSamples, "a beam's samples fit the pool");
-// Cuts a job's beams into tasks (one warp's work each) for a packing: sets the job's beamsPerTask and
-// sampleMagic and returns the number of tasks. launchBeams: beams of all jobs of the launch. A launch
-// that does not fill the chip twice over takes fewer beams per task, because a warp ends with its
-// slowest ray and fewer rays diverge less: with 32 beams, 16, 8 and 1 per task, 3,600 beams took 35 / 33
-// / 37 / 32 us, 32,768 beams 39 / 37 / 36 / 101 us, 76,920 beams 112 / 97 / 99 / 365 us, 131,072 beams 92
-// / 89 / 98 / 474 us. (With L2 flushed before every run one round of tasks is worth more: 32,768 beams
-// of the plain scene in tasks of 7 / 14 / 32 took 57 / 45 / 48 us.) Pooled samples want about eight tasks
-// per warp (58 samples, 65,536 beams: 1221 / 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per
-// task): fewer leave a long tail.
-// `cells`: direction cells that the beams fill (launchCountCells on their sorted keys, 0: not known). The
-// beams of a cell, less than 0.4 degrees apart in azimuth, take nearly the same walk, so a warp takes them
-// together however small the launch: a ring of 3,000 / 12,000 / 30,000 beams took 27 / 29 / 29 us in
-// tasks of 1 / 3 / 7 beams, 21 us in tasks of 2 / 10 / 16 and more.
-constexpr int kResidentWarps = 16; // per SM, at 128 registers
+// Cuts a job's beams into tasks (one warp's work each, beam_tasks.hpp) for a packing: sets the job's
+// beamsPerTask and sampleMagic and returns the number of tasks. launchBeams: beams of all jobs of the launch.
 int setJobTasks(BatchJob& job, int packing, int64_t launchBeams, int cells = 0);
 // Adds the number of distinct keys among n sorted ones to *cells (device).
 void launchCountCells(const uint32_t* sortedKeys, int n, int32_t* cells, cudaStream_t stream);

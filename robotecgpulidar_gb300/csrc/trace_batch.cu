@@ -185,19 +185,10 @@ int smCount()
 
 int setJobTasks(BatchJob& job, int packing, int64_t launchBeams, int cells)
 {
-	const int S = job.p.nSamples;
-	int beams = 32;
-	if (packing != kPackSerial) {
-		const int64_t resident = (int64_t) smCount() * kResidentWarps;
-		int64_t want = S <= kLaneGroupSamples ? (launchBeams + 2 * resident - 1) / (2 * resident) : launchBeams / (8 * resident);
-		if (S <= kLaneGroupSamples && cells > 0) {
-			want = std::max<int64_t>(want, job.p.nRays / cells);
-		}
-		const int most = S <= kLaneGroupSamples ? 32 / S : std::min(32, kPoolSamples / S);
-		beams = (int) std::max<int64_t>(1, std::min<int64_t>(want, most));
-	}
+	const int64_t resident = (int64_t) smCount() * kResidentWarps;
+	const int beams = packing == kPackSerial ? 32 : beamsPerTask(job.p.nSamples, job.p.nRays, launchBeams, resident, cells);
 	job.beamsPerTask = beams;
-	job.sampleMagic = (uint32_t) ((65536 + S - 1) / S);
+	job.sampleMagic = sampleFactor(job.p.nSamples);
 	return (job.p.nRays + beams - 1) / beams;
 }
 
