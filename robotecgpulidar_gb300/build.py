@@ -35,7 +35,7 @@ def _cuda_home() -> str:
 def _headers():
     out = []
     for d in (CSRC, os.path.join(INCLUDE, "rgl", "api"), os.path.join(INCLUDE, "rgl", "api", "extensions")):
-        out += [os.path.join(d, f) for f in os.listdir(d) if f.endswith((".hpp", ".h"))]
+        out += [os.path.join(d, f) for f in os.listdir(d) if f.endswith((".hpp", ".h", ".cuh"))]
     return out
 
 
