@@ -24,11 +24,12 @@ constexpr int kResidentWarps = 16; // per SM, at 128 registers
 // A launch that does not fill the chip twice over takes fewer beams per task, because a warp ends with its
 // slowest ray and fewer rays diverge less: with 32 beams, 16, 8 and 1 per task, 3,600 beams took 35 / 33
 // / 37 / 32 us, 32,768 beams 39 / 37 / 36 / 101 us, 76,920 beams 112 / 97 / 99 / 365 us, 131,072 beams 92
-// / 89 / 98 / 474 us. It depends on the pose, and not on what L2 holds: 32,768 beams of the plain scene in
-// tasks of 7 / 14 / 32 took 33 / 35 / 42 us from poses about the scene, 37 / 40 / 45 with L2 written over
-// before every run, but 58 / 48 / 49 from its centre. Pooled samples want about eight tasks per warp (58
-// samples, 65,536 beams: 1221 / 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams per task): fewer
-// leave a long tail.
+// / 89 / 98 / 474 us. What L2 holds does not matter, a pose may: 32,768 beams in tasks of 4 / 7 / 14 / 32 took
+// 49 / 46 / 48 / 54 us over twelve poses in the plain scene and 94 / 100 / 119 / 143 in a hilly one (37 / 40 /
+// 45 against 33 / 35 / 42 in tasks of 7 / 14 / 32 with L2 written over before every run), but 58 / 48 / 49 in
+// tasks of 7 / 14 / 32 from the plain scene's centre, facing along an axis. Pooled samples want about eight
+// tasks per warp (58 samples, 65,536 beams: 1221 / 1001 / 916 / 928 / 1010 us with 1 / 2 / 3 / 4 / 6 beams
+// per task): fewer leave a long tail.
 // `cells`: direction cells that the beams fill (launchCountCells on their sorted keys, 0: not known). The
 // beams of a cell, less than 0.4 degrees apart in azimuth, take nearly the same walk, so a warp takes them
 // together however small the launch: a ring of 3,000 / 12,000 / 30,000 beams took 27 / 29 / 29 us in

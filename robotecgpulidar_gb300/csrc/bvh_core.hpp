@@ -2,7 +2,8 @@
 // are thin wrappers; the test-suite's CPU harness runs the same functions serially).
 //
 // Build = Morton codes (30 bit) -> radix sort -> LBVH (Karras, "Maximizing Parallelism in the
-// Construction of BVHs, Octrees, and k-d Trees", HPG 2012) -> bottom-up bounds -> top-down collapse
+// Construction of BVHs, Octrees, and k-d Trees", HPG 2012) -> node boxes (on the device from a pyramid of
+// aligned groups of sorted primitives, bvh.cu; in the CPU harness bottom-up) -> top-down collapse
 // into 8-wide nodes (children chosen by repeatedly opening the child of largest surface area) with
 // 8-bit child boxes rounded outward and verified in float.  It replaces OptiX's GAS/IAS builds at
 // reference src/scene/GASBuilder.hpp:31-100 and src/scene/Scene.cpp:131-190.

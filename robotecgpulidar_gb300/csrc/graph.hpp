@@ -258,7 +258,7 @@ struct PointwisePointsNode : PointsNodeSingleInput
 		PointsNodeSingleInput::validateImpl();
 		absorbed = false;
 	}
-	// Stages this node's parameters on `s` and appends its operation.
+	// Appends this node's operation, with its parameters where they are staged in pinned memory.
 	virtual void appendPointOp(rgl::PointOps& ops) = 0;
 	std::shared_ptr<PointsNode> source() const { return input; }
 	bool absorbed = false;

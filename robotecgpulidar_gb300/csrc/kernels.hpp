@@ -94,7 +94,8 @@ void buildTlas(const InstanceRec* hInstances, const InstanceRec* dInstances, int
 // topology. A refit only is cheaper but degrades as entities move across the scene: after a few
 // frames of random re-poses the old topology's boxes cover most of the scene.
 void updateTlas(const InstanceRec* dInstances, TlasBuild& t, cudaStream_t stream);
-// Refits the TLAS after instance boxes changed (same instance set): one single-block launch.
+// Refits the TLAS after instance boxes changed (same instance set): a single-block launch, then one that
+// writes the enter records.
 void refitTlas(const InstanceRec* dInstances, TlasBuild& t, cudaStream_t stream);
 // Arrays for n instances, and for their one-block rebuild when n is within its limit (build_memory.cpp).
 void allocateTlas(TlasBuild& t, int n);

@@ -55,7 +55,7 @@ constexpr int kBins = 32;
 constexpr int kBinWords = 7;                    // lo xyz (ordered bits, complemented), hi xyz (ordered bits), count: empty is 0
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 // Larger ranges split in the level loop, the others are built by a block each. 131,072 triangles, 2,048 /
-// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us, before the bins were filled out of step (one block of 512 threads per SM, by registers).
+// 1,024 / 512: levels 166 / 194 / 222 us, blocks 231 / 143 / 120 us, before the bins were filled out of step.
 constexpr int kBigTask = 1024;
 constexpr int kMeshThreads = 512;
 constexpr int kChunk = 512;                     // elements per block in the level loop: 256 blocks for 131,072 triangles
@@ -1253,7 +1253,8 @@ __global__ void __launch_bounds__(SHARED::kBlockThreads) kSahBlock(const SahTask
 	}
 }
 
-// Ranges of a mesh, several blocks per SM; and the one block of a TLAS.
+// Ranges of a mesh, one block per SM (88 KB of shared memory would let two in, 115 registers for each of 512
+// threads do not); and the one block of a TLAS.
 using MeshShared = BlockShared<kBigTask, kMeshThreads>;
 using TlasShared = BlockShared<kSahSmallMax, 512>;
 

@@ -9,12 +9,11 @@
 //
 // Each job names its own scene, so one launch may cover sensors of several resident scenes.
 //
-// Scheduling: the beams of sensor j form tasks (up to 32 beams and kPoolSamples samples with pooled
-// samples, 32 beams with one lane per beam). A persistent grid of
-// (SM count x resident blocks) blocks fetches `chunk` tasks at a time from one global counter; a
-// warp maps a task to its sensor by binary search over the task prefix sums staged in shared memory.
+// Scheduling: the beams of sensor j form tasks (beams of up to 32 samples together with lane groups, up to 32
+// beams and kPoolSamples samples with pooled samples, 32 beams with one lane per beam; beam_tasks.hpp). A
+// persistent grid of (SM count x resident blocks) blocks fetches `chunk` tasks at a time from one global
+// counter; a warp maps a task to its sensor by binary search over the task prefix sums staged in shared memory.
 // Sensors of uneven size therefore share the GPU without a tail per sensor.
-#include <algorithm>
 #include <map>
 #include <mutex>
 #include <stdexcept>
