@@ -170,8 +170,10 @@ BuildScratch::~BuildScratch()
 {
 	if (base_ != nullptr) {
 		// Freed for good, so that trimBuildMemory finds it free: one that is queued on a stream counts as in
-		// use until the host has waited for it. A build has waited for its stream already.
-		cudaStreamSynchronize(stream_);
+		// use until the host has waited for it.
+		if (!waited_) {
+			cudaStreamSynchronize(stream_);
+		}
 		cudaFree(base_);
 	}
 }

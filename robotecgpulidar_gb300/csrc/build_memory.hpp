@@ -76,10 +76,14 @@ public:
 		layout(place);
 	}
 
+	// The host has waited for the stream since the last use of the arrays.
+	void waited() { waited_ = true; }
+
 private:
 	uintptr_t allocate(size_t bytes);
 	cudaStream_t stream_;
 	void* base_ = nullptr;
+	bool waited_ = false;
 };
 
 // What a device build tells the host: written by the build's last kernel straight into mapped pinned

@@ -469,6 +469,8 @@ WideBuildResult buildWide(const float4* lo, const float4* hi, const uint32_t* cb
 	const volatile BuildReport& r = *report.host();
 	launchCollapse(ci, collapsedev::CollapseTarget{outNodes, outLeaves, outBoxes, queue}, n, state, levels, stages, s);
 	RGL_CUDA_OK(cudaStreamSynchronize(s));
+	scratch.waited();
+	sahScratch.waited();
 	if (r.done == 0) {
 		throw std::runtime_error("BVH build: the collapse did not report");
 	}
@@ -526,6 +528,7 @@ void buildBlas(const float* dVertices, int nVertices, const int32_t* dIndices, i
 	kTriBounds<<<blocks(T, 256), 256, 0, s>>>(dVertices, dIndices, T, lo, hi, cb);
 	countLaunch();
 	const WideBuildResult r = buildWide(lo, hi, cb, T, dVertices, dIndices, kLeafMaxTris, out.nodes, out.tris, nullptr, s);
+	scratch.waited();
 	out.nodeCount = r.nodeCount;
 	out.bounds[0] = r.bounds.lox;
 	out.bounds[1] = r.bounds.loy;
@@ -817,6 +820,7 @@ void buildTlas(const InstanceRec* hInst, const InstanceRec* dInst, int n, TlasBu
 	RGL_CUDA_OK(cudaMemcpyAsync(hi, hHi.data(), sizeof(float4) * (size_t) n, cudaMemcpyHostToDevice, s));
 	const WideBuildResult r = buildWide(lo, hi, nullptr, n, nullptr, nullptr, 1, t.nodes, t.leaves, reinterpret_cast<Box*>(t.boxes), s,
 	                                    LevelRecord{t.levelStarts, t.nLevels, t.levelCapacity});
+	scratch.waited();
 	t.nodeCount = r.nodeCount;
 	kEnterRecords<<<blocks(n, 128), 128, 0, s>>>(t.leaves, dInst, n, t.enter);
 	countLaunch();
